@@ -67,13 +67,24 @@ PT_HD inline void load_node(const DeviceScene &s, int32_t node, BvhNode &n) {
 #endif
 }
 
-// Tests leaf `slot`; updates the running answer.  Returns true when a hit was accepted.  `any`
-// selects any-hit (the first hit is the answer) or closest-hit (ties by key) at run time; the
-// template below fixes it at compile time.
+// The smallest float above x (x finite): nextafterf(x, +inf) in a few integer operations.
+PT_HD inline float next_up(float x) {
+#ifdef __CUDA_ARCH__
+    const int32_t b = __float_as_int(x);
+    return x == 0.0f ? __int_as_float(1) : __int_as_float(b + (b < 0 ? -1 : 1));
+#else
+    return std::nextafter(x, INFINITY);
+#endif
+}
+
+// Tests leaf `slot`; updates the running answer: hit.slot < 0 until a hit is accepted, then `limit`
+// is the float above the closest distance (an accepted t is below tmax, so nextafterf(t, tmax) is
+// next_up(t)).  The limit changes only here, so it is kept instead of being recomputed before each
+// test, and the tie key is formed only when two distances are equal (2^25 rays on the 1M-triangle
+// scene: 7.00 -> 6.39 ms; 2^22 incoherent ones: 2.02 -> 1.85).  Returns true when a hit was accepted.  `any` selects any-hit (the first hit is the answer) or closest-hit (ties by key) at run
+// time; the template below fixes it at compile time.
 PT_HD __forceinline__ bool test_leaf_rt(const DeviceScene &s, int32_t slot, const pt_ray &r, float dl, float tmin,
-                                        float tmax, int tie, bool any, bool &found, float &closest, long long &best_key,
-                                        HitInfo &hit, uint32_t &prims) {
-    float limit = found ? nextafterf(closest, tmax) : tmax;
+                                        float &limit, int tie, bool any, HitInfo &hit, uint32_t &prims) {
     float t, u = 0, v = 0;
     bool ok;
     prims++;
@@ -87,23 +98,17 @@ PT_HD __forceinline__ bool test_leaf_rt(const DeviceScene &s, int32_t slot, cons
         ok = sphere_hit(sp, r, tmin, limit, t);
     }
     if (!ok) return false;
-    if (!any && found && !(t < closest)) {
-        long long key = tie_key(s, slot, tie);
-        if (!(key < best_key)) return false;
-        best_key = key;
-    } else if (!any) {
-        best_key = tie_key(s, slot, tie);
+    if (!any) {
+        if (hit.slot >= 0 && !(t < hit.t) && !(tie_key(s, slot, tie) < tie_key(s, hit.slot, tie))) return false;
+        limit = next_up(t);
     }
-    found = true;
-    closest = t;
     hit.t = t; hit.u = u; hit.v = v; hit.slot = slot;
     return true;
 }
 template <bool kAny>
 PT_HD __forceinline__ bool test_leaf(const DeviceScene &s, int32_t slot, const pt_ray &r, float dl, float tmin,
-                                     float tmax, int tie, bool &found, float &closest, long long &best_key,
-                                     HitInfo &hit, uint32_t &prims) {
-    return test_leaf_rt(s, slot, r, dl, tmin, tmax, tie, kAny, found, closest, best_key, hit, prims);
+                                     float &limit, int tie, HitInfo &hit, uint32_t &prims) {
+    return test_leaf_rt(s, slot, r, dl, tmin, limit, tie, kAny, hit, prims);
 }
 
 // Closest hit (any = false) or any hit (any = true) over (tmin, tmax), from node `root` of the
@@ -114,16 +119,13 @@ PT_HD inline bool traverse_rt(const DeviceScene &s, const pt_ray &r, float tmin,
     if (s.empty || s.node_count == 0 || root < 0) return false;
     RayBox rb = ray_box(r);
     float dl = length(mk(r.direction));
-    bool found = false;
-    float closest = tmax;
-    long long best_key = 0;
+    float limit = tmax;
     int32_t stack[kStackCapacity];
     int sp = 0;
     int32_t node = root;
     for (;;) {
         BvhNode n;
         load_node(s, node, n);
-        float limit = found ? nextafterf(closest, tmax) : tmax;
         float e0, e1;
         bool h0 = n.child0 != kEmptyChild &&
                   box_hit(rb, n.c0lox, n.c0hix, n.c0loy, n.c0hiy, n.c0loz, n.c0hiz, tmin, limit, e0);
@@ -139,12 +141,12 @@ PT_HD inline bool traverse_rt(const DeviceScene &s, const pt_ray &r, float tmin,
         int ninner = 0;
         if (hf) {
             if (first < 0) {
-                if (test_leaf_rt(s, ~first, r, dl, tmin, tmax, tie, any, found, closest, best_key, hit, prims) && any) return true;
+                if (test_leaf_rt(s, ~first, r, dl, tmin, limit, tie, any, hit, prims) && any) return true;
             } else inner[ninner++] = first;
         }
         if (hs) {
             if (second < 0) {
-                if (test_leaf_rt(s, ~second, r, dl, tmin, tmax, tie, any, found, closest, best_key, hit, prims) && any) return true;
+                if (test_leaf_rt(s, ~second, r, dl, tmin, limit, tie, any, hit, prims) && any) return true;
             } else inner[ninner++] = second;
         }
         if (ninner == 2) {
@@ -158,7 +160,7 @@ PT_HD inline bool traverse_rt(const DeviceScene &s, const pt_ray &r, float tmin,
             node = stack[--sp];
         }
     }
-    return found;
+    return hit.slot >= 0;
 }
 template <bool kAny>
 PT_HD inline bool traverse(const DeviceScene &s, const pt_ray &r, float tmin, float tmax, int tie,
@@ -178,14 +180,12 @@ PT_HD inline bool traverse_reference(const DeviceScene &s, const pt_ray &r, floa
     if (s.empty || s.node_count == 0) return false;
     RayBox rb = ray_box(r);
     float dl = length(mk(r.direction));
-    bool found = false;
-    float closest = tmax;
-    long long best_key = 0;
+    float limit = tmax;
     if (s.root_leaf) {
         BvhNode n;
         load_node(s, 0, n);
-        test_leaf<false>(s, ~n.child0, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims);
-        return found;
+        test_leaf<false>(s, ~n.child0, r, dl, tmin, limit, tie, hit, prims);
+        return hit.slot >= 0;
     }
     // the root branch: its own box first
     {
@@ -213,7 +213,6 @@ PT_HD inline bool traverse_reference(const DeviceScene &s, const pt_ray &r, floa
         int32_t child = side ? p.child1 : p.child0;
         if (child >= 0) {
             boxes++;
-            float limit = found ? nextafterf(closest, tmax) : tmax;
             float e;
             bool h = side ? box_hit(rb, p.c1lox, p.c1hix, p.c1loy, p.c1hiy, p.c1loz, p.c1hiz, tmin, limit, e)
                           : box_hit(rb, p.c0lox, p.c0hix, p.c0loy, p.c0hiy, p.c0loz, p.c0hiz, tmin, limit, e);
@@ -225,10 +224,10 @@ PT_HD inline bool traverse_reference(const DeviceScene &s, const pt_ray &r, floa
             if (n.child1 != kEmptyChild) stack[sp++] = (child << 1) | 1;
             stack[sp++] = (child << 1) | 0;
         } else {
-            test_leaf<false>(s, ~child, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims);
+            test_leaf<false>(s, ~child, r, dl, tmin, limit, tie, hit, prims);
         }
     }
-    return found;
+    return hit.slot >= 0;
 }
 
 // trace_world(…, brute = true) (src/renderer/transport.h:48-60): every leaf, in flat
@@ -239,14 +238,12 @@ PT_HD inline bool traverse_brute(const DeviceScene &s, const int32_t *order, int
     hit.slot = -1; hit.t = 0; hit.u = 0; hit.v = 0;
     if (s.empty) return false;
     float dl = length(mk(r.direction));
-    bool found = false;
-    float closest = tmax;
-    long long best_key = 0;
+    float limit = tmax;
     for (int32_t i = 0; i < leaves; i++) {
-        if (test_leaf<kAny>(s, order[i], r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny)
+        if (test_leaf<kAny>(s, order[i], r, dl, tmin, limit, tie, hit, prims) && kAny)
             return true;
     }
-    return found;
+    return hit.slot >= 0;
 }
 
 // ---- full hit record of the winner (src/flat/flat_intersect.h:27-42, 53-64) ----
@@ -308,74 +305,6 @@ PT_HD inline void hit_ids(const DeviceScene &s, int32_t slot, int32_t &type, int
 
 } // namespace ptb
 
-namespace ptb {
-
-// Resumable closest-hit / any-hit traversal: the same walk as traverse<>, cut into steps of
-// one node each so a persistent warp can retire finished rays and take new ones between
-// steps (the lanes of a warp then stay busy until the ray pool is empty).
-struct Walker {
-    RayBox rb;
-    pt_ray r;
-    float dl, tmin, tmax, closest;
-    long long best_key;
-    HitInfo hit;
-    uint32_t boxes, prims;
-    int32_t node, sp;
-    bool found;
-    int error;
-    int32_t stack[kStackCapacity];
-
-    PT_HD void begin(const DeviceScene &s, const pt_ray &ray, float lo, float hi) {
-        r = ray; rb = ray_box(ray); dl = length(mk(ray.direction));
-        tmin = lo; tmax = hi; closest = hi; best_key = 0;
-        hit.slot = -1; hit.t = 0; hit.u = 0; hit.v = 0;
-        boxes = 0; prims = 0; sp = 0; found = false; error = 0;
-        node = (s.empty || s.node_count == 0) ? -1 : 0;
-    }
-    // One node: both child boxes, leaf children tested at once (nearer first), descend into
-    // the nearer inner child and push the other.  Returns true when the walk has ended.
-    template <bool kAny>
-    PT_HD bool step(const DeviceScene &s, int tie) {
-        if (node < 0) return true;
-        BvhNode n;
-        load_node(s, node, n);
-        float limit = found ? nextafterf(closest, tmax) : tmax;
-        float e0, e1;
-        bool h0 = n.child0 != kEmptyChild && box_hit(rb, n.c0lox, n.c0hix, n.c0loy, n.c0hiy, n.c0loz, n.c0hiz, tmin, limit, e0);
-        bool h1 = n.child1 != kEmptyChild && box_hit(rb, n.c1lox, n.c1hix, n.c1loy, n.c1hiy, n.c1loz, n.c1hiz, tmin, limit, e1);
-        boxes += (n.child0 != kEmptyChild) + (n.child1 != kEmptyChild);
-        int32_t first = n.child0, second = n.child1;
-        bool hf = h0, hs = h1;
-        if (h0 && h1 && e1 < e0) { first = n.child1; second = n.child0; }
-        else if (!h0) { first = n.child1; hf = h1; hs = false; }
-        int32_t inner[2];
-        int ninner = 0;
-        if (hf) {
-            if (first < 0) {
-                if (test_leaf<kAny>(s, ~first, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny) { node = -1; return true; }
-            } else inner[ninner++] = first;
-        }
-        if (hs) {
-            if (second < 0) {
-                if (test_leaf<kAny>(s, ~second, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny) { node = -1; return true; }
-            } else inner[ninner++] = second;
-        }
-        if (ninner == 2) {
-            if (sp >= kStackCapacity) { error = 1; found = false; hit.slot = -1; node = -1; return true; }
-            stack[sp++] = inner[1];
-            node = inner[0];
-        } else if (ninner == 1) {
-            node = inner[0];
-        } else {
-            if (sp == 0) { node = -1; return true; }
-            node = stack[--sp];
-        }
-        return false;
-    }
-};
-
-} // namespace ptb
-
 #ifdef __CUDACC__
 namespace ptb {
 
@@ -408,12 +337,10 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
     // walk state (registers)
     pt_ray r;
     RayBox rb;
-    float dl = 0, tmin = 0, tmax = 0, closest = 0;
-    long long best_key = 0;
+    float dl = 0, tmin = 0, limit = 0;
     HitInfo hit;
     uint32_t boxes = 0, prims = 0;
     int32_t node = -1, sp = 0;
-    bool found = false;
     int error = 0;
     size_t index = 0;
     bool busy = false, pool_empty = false;
@@ -431,13 +358,12 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
                 if (mine < count) {
                     index = mine;
                     int32_t root = 0;
-                    if constexpr (kRoot) get(index, r, tmin, tmax, root);
-                    else get(index, r, tmin, tmax);
+                    if constexpr (kRoot) get(index, r, tmin, limit, root);
+                    else get(index, r, tmin, limit);
                     rb = ray_box(r);
                     dl = length(mk(r.direction));
-                    closest = tmax; best_key = 0;
                     hit.slot = -1; hit.t = 0; hit.u = 0; hit.v = 0;
-                    boxes = 0; prims = 0; sp = 0; found = false; error = 0;
+                    boxes = 0; prims = 0; sp = 0; error = 0;
                     node = (s.empty || s.node_count == 0 || root < 0) ? -1 : root;
                     busy = true;
                 }
@@ -452,7 +378,6 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
                 else {
                     BvhNode n;
                     load_node(s, node, n);
-                    float limit = found ? nextafterf(closest, tmax) : tmax;
                     float e0, e1;
                     bool h0 = n.child0 != kEmptyChild && box_hit(rb, n.c0lox, n.c0hix, n.c0loy, n.c0hiy, n.c0loz, n.c0hiz, tmin, limit, e0);
                     bool h1 = n.child1 != kEmptyChild && box_hit(rb, n.c1lox, n.c1hix, n.c1loy, n.c1hiy, n.c1loz, n.c1hiz, tmin, limit, e1);
@@ -465,17 +390,17 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
                     int ninner = 0;
                     if (hf) {
                         if (first < 0) {
-                            if (test_leaf<kAny>(s, ~first, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny) end = true;
+                            if (test_leaf<kAny>(s, ~first, r, dl, tmin, limit, tie, hit, prims) && kAny) end = true;
                         } else { inner0 = first; ninner = 1; }
                     }
                     if (hs && !end) {
                         if (second < 0) {
-                            if (test_leaf<kAny>(s, ~second, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny) end = true;
+                            if (test_leaf<kAny>(s, ~second, r, dl, tmin, limit, tie, hit, prims) && kAny) end = true;
                         } else { if (ninner) inner1 = second; else inner0 = second; ninner++; }
                     }
                     if (!end) {
                         if (ninner == 2) {
-                            if (sp >= kStackCapacity) { error = 1; found = false; hit.slot = -1; end = true; }
+                            if (sp >= kStackCapacity) { error = 1; hit.slot = -1; end = true; }
                             else {
                                 if (sp < kSharedStack) my_stack[sp * stride] = inner1;
                                 else spill[sp - kSharedStack] = inner1;
@@ -494,7 +419,7 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
                 }
                 if (end) {
                     WalkResult res;
-                    res.t = hit.t; res.u = hit.u; res.v = hit.v; res.slot = found ? hit.slot : -1;
+                    res.t = hit.t; res.u = hit.u; res.v = hit.v; res.slot = hit.slot;
                     res.boxes = boxes; res.prims = prims; res.error = error;
                     done(index, res);
                     busy = false;
@@ -630,19 +555,18 @@ PT_HD inline int node4_children(const DeviceScene &s, int32_t node, const RayBox
 }
 
 // Tests the 1..8 slots of a leaf reference; true when `any` and a hit was found.
-PT_HD __forceinline__ bool leaf4_rt(const DeviceScene &s, int32_t ref, const pt_ray &r, float dl, float tmin, float tmax,
-                                    int tie, bool any, bool &found, float &closest, long long &best_key, HitInfo &hit,
-                                    uint32_t &prims) {
+PT_HD __forceinline__ bool leaf4_rt(const DeviceScene &s, int32_t ref, const pt_ray &r, float dl, float tmin, float &limit,
+                                    int tie, bool any, HitInfo &hit, uint32_t &prims) {
     int32_t v = ~ref;
     int32_t first = v >> 3, count = (v & 7) + 1;
     for (int32_t j = 0; j < count; j++)
-        if (test_leaf_rt(s, first + j, r, dl, tmin, tmax, tie, any, found, closest, best_key, hit, prims) && any) return true;
+        if (test_leaf_rt(s, first + j, r, dl, tmin, limit, tie, any, hit, prims) && any) return true;
     return false;
 }
 template <bool kAny>
-PT_HD __forceinline__ bool leaf4(const DeviceScene &s, int32_t ref, const pt_ray &r, float dl, float tmin, float tmax, int tie,
-                                 bool &found, float &closest, long long &best_key, HitInfo &hit, uint32_t &prims) {
-    return leaf4_rt(s, ref, r, dl, tmin, tmax, tie, kAny, found, closest, best_key, hit, prims);
+PT_HD __forceinline__ bool leaf4(const DeviceScene &s, int32_t ref, const pt_ray &r, float dl, float tmin, float &limit, int tie,
+                                 HitInfo &hit, uint32_t &prims) {
+    return leaf4_rt(s, ref, r, dl, tmin, limit, tie, kAny, hit, prims);
 }
 
 // Per-thread four-wide walk (local-memory stack), for kernels that run one ray per thread;
@@ -654,9 +578,7 @@ PT_HD inline bool traverse4_rt(const DeviceScene &s, const pt_ray &r, float tmin
     if (s.empty || s.node_count == 0 || root < 0) return false;
     RayBox4 rb = ray_box4(r);
     float dl = length(mk(r.direction));
-    bool found = false;
-    float closest = tmax, limit = tmax;
-    long long best_key = 0;
+    float limit = tmax;
     int32_t sref[3 * kStackCapacity];
     float sdist[3 * kStackCapacity];
     int sp = 0;
@@ -675,8 +597,7 @@ PT_HD inline bool traverse4_rt(const DeviceScene &s, const pt_ray &r, float tmin
                 continue;
             }
         } else {
-            if (leaf4_rt(s, cur, r, dl, tmin, tmax, tie, any, found, closest, best_key, hit, prims) && any) return true;
-            if (found) limit = nextafterf(closest, tmax);
+            if (leaf4_rt(s, cur, r, dl, tmin, limit, tie, any, hit, prims) && any) return true;
         }
         // pop the nearest entry still inside the limit
         bool next = false;
@@ -686,7 +607,7 @@ PT_HD inline bool traverse4_rt(const DeviceScene &s, const pt_ray &r, float tmin
         }
         if (!next) break;
     }
-    return found;
+    return hit.slot >= 0;
 }
 template <bool kAny>
 PT_HD inline bool traverse4(const DeviceScene &s, const pt_ray &r, float tmin, float tmax, int tie,
@@ -716,13 +637,11 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
     const unsigned lane = threadIdx.x & 31;
     pt_ray r;
     RayBox4 rb;
-    float dl = 0, tmin = 0, tmax = 0, closest = 0, limit = 0;
-    long long best_key = 0;
+    float dl = 0, tmin = 0, limit = 0;
     HitInfo hit;
     uint32_t boxes = 0, prims = 0;
     int32_t cur = -1;
     int sp = 0;
-    bool found = false;
     int error = 0;
     size_t index = 0;
     bool busy = false, pool_empty = false;
@@ -739,12 +658,11 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < count) {
                     index = mine;
-                    get(index, r, tmin, tmax);
+                    get(index, r, tmin, limit);
                     rb = ray_box4(r);
                     dl = length(mk(r.direction));
-                    closest = tmax; limit = tmax; best_key = 0;
                     hit.slot = -1; hit.t = 0; hit.u = 0; hit.v = 0;
-                    boxes = 0; prims = 0; sp = 0; found = false; error = 0;
+                    boxes = 0; prims = 0; sp = 0; error = 0;
                     cur = (s.empty || s.node_count == 0) ? kEmptyChild : 0;
                     busy = true;
                 }
@@ -760,7 +678,7 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
                     float dist[4];
                     int hits = node4_children(s, cur, rb, tmin, limit, ref, dist, boxes);
                     if (hits) {
-                        if (sp + hits - 1 > kStack4) { error = 1; found = false; end = true; }
+                        if (sp + hits - 1 > kStack4) { error = 1; hit.slot = -1; end = true; }
                         else {
 #pragma unroll
                             for (int k = 3; k >= 1; k--) {    // static indices: ref/dist stay in registers
@@ -775,8 +693,7 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
                         }
                     }
                 } else if (!end) {
-                    if (leaf4<kAny>(s, cur, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny) end = true;
-                    else if (found) limit = nextafterf(closest, tmax);
+                    if (leaf4<kAny>(s, cur, r, dl, tmin, limit, tie, hit, prims) && kAny) end = true;
                 }
                 if (!end && !descended) {
                     end = true;
@@ -788,7 +705,7 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
                 }
                 if (end) {
                     WalkResult res;
-                    res.t = hit.t; res.u = hit.u; res.v = hit.v; res.slot = found ? hit.slot : -1;
+                    res.t = hit.t; res.u = hit.u; res.v = hit.v; res.slot = hit.slot;
                     res.boxes = boxes; res.prims = prims; res.error = error;
                     done(index, res);
                     busy = false;
@@ -829,13 +746,11 @@ __device__ inline void persistent_walk4_spec(const DeviceScene &s, size_t count,
     constexpr int32_t kNone = kEmptyChild;
     pt_ray r;
     RayBox4 rb;
-    float dl = 0, tmin = 0, tmax = 0, closest = 0, limit = 0;
-    long long best_key = 0;
+    float dl = 0, tmin = 0, limit = 0;
     HitInfo hit;
     uint32_t boxes = 0, prims = 0;
     int32_t cur = kNone, leaf = kNone, leaf2 = kNone;
     int sp = 0;
-    bool found = false;
     int error = 0;
     size_t index = 0;
     bool busy = false, pool_empty = false;
@@ -861,13 +776,12 @@ __device__ inline void persistent_walk4_spec(const DeviceScene &s, size_t count,
                 if (mine < count) {
                     index = mine;
                     int32_t root = 0;
-                    if constexpr (kRoot) get(index, r, tmin, tmax, root);
-                    else get(index, r, tmin, tmax);
+                    if constexpr (kRoot) get(index, r, tmin, limit, root);
+                    else get(index, r, tmin, limit);
                     rb = ray_box4(r);
                     dl = length(mk(r.direction));
-                    closest = tmax; limit = tmax; best_key = 0;
                     hit.slot = -1; hit.t = 0; hit.u = 0; hit.v = 0;
-                    boxes = 0; prims = 0; sp = 0; found = false; error = 0;
+                    boxes = 0; prims = 0; sp = 0; error = 0;
                     cur = (s.empty || s.node_count == 0 || root < 0) ? kNone : root;
                     leaf = kNone; leaf2 = kNone;
                     busy = true;
@@ -923,15 +837,14 @@ __device__ inline void persistent_walk4_spec(const DeviceScene &s, size_t count,
                 if (leaf2 != kNone) { const int32_t v2 = ~leaf2; f2 = v2 >> 3; c2 = (v2 & 7) + 1; }
                 for (int32_t j = 0; j < c1 + c2; j++) {
                     const int32_t slot = j < c1 ? f1 + j : f2 + (j - c1);
-                    if (test_leaf<kAny>(s, slot, r, dl, tmin, tmax, tie, found, closest, best_key, hit, prims) && kAny) { end = true; break; }
+                    if (test_leaf<kAny>(s, slot, r, dl, tmin, limit, tie, hit, prims) && kAny) { end = true; break; }
                 }
-                if (!end && found) limit = nextafterf(closest, tmax);
                 leaf = kNone; leaf2 = kNone;
             }
             if (busy && (end || error || (leaf == kNone && cur == kNone))) {
                 WalkResult res;
-                if (error) found = false;
-                res.t = hit.t; res.u = hit.u; res.v = hit.v; res.slot = found ? hit.slot : -1;
+                if (error) hit.slot = -1;
+                res.t = hit.t; res.u = hit.u; res.v = hit.v; res.slot = hit.slot;
                 res.boxes = boxes; res.prims = prims; res.error = error;
                 done(index, res);
                 busy = false;
