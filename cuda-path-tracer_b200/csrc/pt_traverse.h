@@ -472,6 +472,28 @@ PT_HD inline float fma_box(float a, float b, float c) {
     return std::fma(a, b, c);
 #endif
 }
+#ifdef __CUDA_ARCH__
+// Two floats in one 64-bit register: one instruction multiplies (and adds) both, each rounded as
+// the scalar instruction rounds it.  The walk is bound by instruction issue, not by the FMA pipe
+// (2^25 rays on the 1M-triangle scene: 6.39 -> 6.35 ms with x and y of each slab in one instruction).
+using f2x = unsigned long long;
+__device__ __forceinline__ f2x f2x_make(float a, float b) {
+    f2x r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2x_split(f2x v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2x f2x_fma(f2x a, f2x b, f2x c) {
+    f2x r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2x f2x_mul(f2x a, f2x b) {
+    f2x r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+#endif
 PT_HD inline float max3(float a, float b, float c) {
 #ifdef __CUDA_ARCH__
     float r;
@@ -529,17 +551,31 @@ PT_HD inline int node4_children(const DeviceScene &s, int32_t node, const RayBox
                                 int32_t ref[4], float dist[4], uint32_t &boxes) {
     Bvh4QNode n;
     load_node4(s, node, n);
+#ifdef __CUDA_ARCH__
+    const f2x jxy = f2x_make(rb.jx, rb.jy);
+    const f2x sxy = f2x_mul(f2x_make(n.sx, n.sy), jxy), txy = f2x_fma(f2x_make(n.px, n.py), jxy, f2x_make(rb.kx, rb.ky));
+    const float sz1 = n.sz * rb.jz, tz1 = fma_box(n.pz, rb.jz, rb.kz);
+    const f2x szz = f2x_make(sz1, sz1), tzz = f2x_make(tz1, tz1);
+#else
     const float sx = n.sx * rb.jx, sy = n.sy * rb.jy, sz = n.sz * rb.jz;
     const float tx = fma_box(n.px, rb.jx, rb.kx), ty = fma_box(n.py, rb.jy, rb.ky), tz = fma_box(n.pz, rb.jz, rb.kz);
+#endif
     const uint32_t nxw = rb.nx ? n.qhi[0] : n.qlo[0], fxw = rb.nx ? n.qlo[0] : n.qhi[0];
     const uint32_t nyw = rb.ny ? n.qhi[1] : n.qlo[1], fyw = rb.ny ? n.qlo[1] : n.qhi[1];
     const uint32_t nzw = rb.nz ? n.qhi[2] : n.qlo[2], fzw = rb.nz ? n.qlo[2] : n.qhi[2];
     int hits = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-        const float ax = fma_box(qbyte(nxw, k), sx, tx), bx = fma_box(qbyte(fxw, k), sx, tx);
-        const float ay = fma_box(qbyte(nyw, k), sy, ty), by = fma_box(qbyte(fyw, k), sy, ty);
-        const float az = fma_box(qbyte(nzw, k), sz, tz), bz = fma_box(qbyte(fzw, k), sz, tz);
+        float ax, ay, az, bx, by, bz;
+#ifdef __CUDA_ARCH__
+        f2x_split(f2x_fma(f2x_make(qbyte(nxw, k), qbyte(nyw, k)), sxy, txy), ax, ay);
+        f2x_split(f2x_fma(f2x_make(qbyte(fxw, k), qbyte(fyw, k)), sxy, txy), bx, by);
+        f2x_split(f2x_fma(f2x_make(qbyte(nzw, k), qbyte(fzw, k)), szz, tzz), az, bz);
+#else
+        ax = fma_box(qbyte(nxw, k), sx, tx); bx = fma_box(qbyte(fxw, k), sx, tx);
+        ay = fma_box(qbyte(nyw, k), sy, ty); by = fma_box(qbyte(fyw, k), sy, ty);
+        az = fma_box(qbyte(nzw, k), sz, tz); bz = fma_box(qbyte(fzw, k), sz, tz);
+#endif
         const float entry = fmaxf(max3(ax, ay, az), tmin), exit = fminf(min3(bx, by, bz), limit);
         const bool h = n.child[k] != kEmptyChild && entry <= exit;
         boxes += n.child[k] != kEmptyChild;
