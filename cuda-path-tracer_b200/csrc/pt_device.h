@@ -78,7 +78,7 @@ extern QueryConfig g_query_config;
 // The scene handle: everything device-resident that queries and renderers read.
 struct pt_scene {
     ptb::DeviceScene view{};
-    ptb::DeviceBuffer nodes, nodes4, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, brute_order;
+    ptb::DeviceBuffer nodes, nodes4, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, brute_order, small;
     std::vector<pt_light> host_lights;
     float light_area = 0;
     int32_t leaf_count = 0;

@@ -32,6 +32,7 @@ struct HostLayout {
     int32_t root_leaf = 0;
     std::vector<Bvh4Node> nodes4;       // empty when the flat graph shares subtrees
     std::vector<Bvh4QNode> nodes4q;     // nodes4 quantized (what the device walks)
+    std::vector<SmallLeaf> small;       // all leaves in slot order (at most kSmallLeaves, else empty)
 };
 HostLayout relayout(const pt_scene_desc &scene);
 Bvh4QNode quantize4(const Bvh4Node &n);

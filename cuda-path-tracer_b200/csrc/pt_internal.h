@@ -77,6 +77,14 @@ struct alignas(16) SphereRecord {
 };
 static_assert(sizeof(SphereRecord) == 32, "sphere record is 32 bytes");
 
+// A leaf of a scene with at most kSmallLeaves of them: its own box and its slot (pt_small.h).
+constexpr int kSmallLeaves = 32;
+struct alignas(16) SmallLeaf {
+    float lo[3], hi[3];
+    int32_t slot, pad;
+};
+static_assert(sizeof(SmallLeaf) == 32, "small-scene leaf is 32 bytes");
+
 // Everything a kernel needs, passed by value (device pointers).
 struct DeviceScene {
     const BvhNode *nodes;
@@ -96,6 +104,8 @@ struct DeviceScene {
     int32_t empty;                  // root == -1
     float root_lo[3], root_hi[3];   // the flat root's own box (tested first by trace_world)
     int32_t root_leaf;              // flat root is itself a leaf (no branch above it)
+    const SmallLeaf *small;         // every leaf in slot order, when there are at most kSmallLeaves
+    int32_t small_count;            // 0: more leaves than that (or none)
 };
 
 // Tie rule for exact-distance hits: the lowest (type, id) (the parity rule of the query API), the leaf the

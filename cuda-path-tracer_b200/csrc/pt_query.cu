@@ -377,6 +377,7 @@ pt_status pt_scene_create(const pt_scene_desc *desc, pt_scene **out) {
             sc->tris.upload(layout.tris);
             sc->spheres.upload(layout.spheres);
             sc->brute_order.upload(layout.brute_order);
+            sc->small.upload(layout.small);
             sc->triangles.upload(desc->triangles, desc->triangle_count * sizeof(pt_triangle));
             sc->sphere_src.upload(desc->spheres, desc->sphere_count * sizeof(pt_sphere));
             sc->materials.upload(desc->materials, desc->material_count * sizeof(pt_material));
@@ -403,6 +404,8 @@ pt_status pt_scene_create(const pt_scene_desc *desc, pt_scene **out) {
             v.empty = layout.empty;
             for(int a = 0; a < 3; a++) { v.root_lo[a] = layout.root_lo[a]; v.root_hi[a] = layout.root_hi[a]; }
             v.root_leaf = layout.root_leaf;
+            v.small = sc->small.get<SmallLeaf>();
+            v.small_count = int32_t(layout.small.size());
         } catch(...) { delete sc; throw; }
         *out = sc;
     });
@@ -431,7 +434,7 @@ pt_status pt_scene_device_bytes(const pt_scene *s, size_t *bytes) {
     return guard([&]() {
         if(!s || !bytes) throw Error(PT_INVALID_ARGUMENT, "null argument");
         *bytes = s->nodes.bytes() + s->nodes4.bytes() + s->tris.bytes() + s->spheres.bytes() + s->triangles.bytes() + s->sphere_src.bytes() +
-                 s->materials.bytes() + s->textures.bytes() + s->pixels.bytes() + s->lights.bytes() + s->brute_order.bytes();
+                 s->materials.bytes() + s->textures.bytes() + s->pixels.bytes() + s->lights.bytes() + s->brute_order.bytes() + s->small.bytes();
     });
 }
 

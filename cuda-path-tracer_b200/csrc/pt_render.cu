@@ -18,6 +18,7 @@
 #include <vector>
 #include "pt_api_common.h"
 #include "pt_device.h"
+#include "pt_small.h"
 #include "pt_wavefront.h"
 
 using namespace ptb;
@@ -309,6 +310,79 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
     if (lane == 0 && rays) atomicAdd(b.rays, rays);
 }
 
+// The whole render of a scene with at most kSmallLeaves primitives: one path per lane, its pixel's
+// samples from the first camera ray to the last bounce, the scene in shared memory (pt_small.h).
+// Each round a warp walks its lanes' pending shadow rays, then their extension rays, through one
+// copy of the walk, and shades together, so all lanes stay in the same code: with the divergent
+// tree walk 10 of 32 lanes were busy and warps waited on instruction fetch.  A lane whose pixel is
+// done takes the next one from fetch[3].  The shadow contribution of bounce k is added before
+// bounce k + 1 is shaded, as in every other form.  Blocks of 64 spread a small image's paths evenly
+// over the SMs.
+constexpr int kSmallBlock = 64;
+__global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene scene, RenderParams p, RenderBuffers b, int32_t count,
+                                                                  int samples) {
+    __shared__ SmallScene sh;
+    small_load(scene, sh, 0.0f);
+    const unsigned full = 0xffffffffu;
+    ShadeCtx ctx;
+    ctx.camera = &p.camera; ctx.width = p.width; ctx.height = p.height; ctx.max_depth = p.max_depth;
+    ctx.debug = PT_DEBUG_SHADED; ctx.mis = p.mis;
+    unsigned long long rays = 0;
+    int32_t i = -1;                // the lane's pixel
+    PathState s{};
+    Pcg rng{};
+    ShadowRay sr{};
+    bool live = false, pending = false, drained = false;
+    for (;;) {
+        const bool idle = !live && !drained;
+        const unsigned m = __ballot_sync(full, idle);
+        if (m) {
+            const int leader = __ffs(m) - 1;
+            unsigned long long base = 0;
+            if ((int)lane_id() == leader) base = atomicAdd(&b.fetch[3], (unsigned long long)__popc(m));
+            base = __shfl_sync(full, base, leader);
+            if (idle) {
+                if (i >= 0) { b.rng[i] = rng; i = -1; }
+                const unsigned long long k = base + __popc(m & ((1u << lane_id()) - 1u));
+                if (k < (unsigned long long)count) {
+                    i = int32_t(k);
+                    rng = b.rng[i];
+                    camera_path(p, i, rng, s);
+                    s.samples_left = samples;
+                    live = true;
+                } else {
+                    drained = true;
+                }
+            }
+        }
+        if (!__any_sync(full, live)) break;
+        HitInfo hi;
+        bool hit = false;
+        for (int pass = __any_sync(full, pending) ? 0 : 1; pass < 2; pass++) {
+            const bool shadow_pass = pass == 0;
+            if (shadow_pass ? pending : live) {
+                rays++;   // each query counts once, as trace_color counts it (transport.h:177)
+                pt_ray r = path_ray(s);
+                if (shadow_pass) {
+                    r.origin = pt_vec3{sr.ox, sr.oy, sr.oz};
+                    r.direction = pt_vec3{sr.dx, sr.dy, sr.dz};
+                }
+                hit = small_walk(scene, sh, r, 0.001f, shadow_pass ? sr.tmax : FLT_MAX, kTieLastLeaf, shadow_pass, hi);
+                if (shadow_pass && !hit) { s.rr = s.rr + sr.cr; s.rg = s.rg + sr.cg; s.rb = s.rb + sr.cb; }
+            }
+            __syncwarp();
+        }
+        if (live) {
+            PathHit h;
+            h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = hit ? hi.slot : -1;
+            live = shade_path(scene, ctx, b.sums + 3 * size_t(i), i, i, s, h, make_uint2(0, 0), rng, sr, pending);
+        }
+        __syncwarp();
+    }
+    for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(full, rays, o);
+    if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
+}
+
 // shadow: any-hit of the NEE rays (transport.h:206-214); unoccluded ones add their contribution
 __global__ void __launch_bounds__(256, 4) shadow_kernel(DeviceScene scene, RenderParams p, RenderBuffers b, int parity, int min_active) {
     const int32_t n = b.counters[2 + parity];
@@ -390,9 +464,10 @@ struct pt_renderer {
     // threads per block of the wavefront kernels (pt_set_block_shape): 16x8 by default (config 2:
     // 64.3 ms per render against 65.1 with the reference's 16x16; config 1 unchanged)
     int block = 128;
-    int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0;
+    int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0;
     int32_t tail_paths = 0;             // live-path count below which the fused finish kernel takes over
     bool pair_tail = false;             // the tail runs two lanes per path (finish_pair_kernel)
+    bool small = false;                 // the scene fits render_small_kernel and the view is shaded
     DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba;
     RenderBuffers buf{};
     cudaStream_t stream = nullptr;
@@ -412,6 +487,7 @@ struct pt_renderer {
         grid_shadow = occupancy_grid((const void *)shadow_kernel, block, stack_bytes(block));
         grid_finish = occupancy_grid((const void *)finish_kernel, kFinishBlock);
         grid_finish_pair = occupancy_grid((const void *)finish_pair_kernel, block);
+        grid_small = occupancy_grid((const void *)render_small_kernel, kSmallBlock);
     }
 };
 
@@ -488,6 +564,7 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             constexpr size_t kSmallTreeNodes = 32;
             if (p.wide && scene->nodes4.bytes() / sizeof(Bvh4QNode) <= kSmallTreeNodes) p.wide = 0;
             r->pair_tail = p.wide != 0;
+            r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
         } catch (...) { delete r; throw; }
         *out = r;
         pt_status st = pt_reset(r, camera);
@@ -520,8 +597,15 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         cudaStream_t st = r->stream;
         PT_CUDA(cudaMemsetAsync(r->buf.rays, 0, sizeof(unsigned long long), st));
         PT_CUDA(cudaEventRecord(r->start.get(), st));
-        start_samples<<<(r->pixels + 255) / 256, 256, 0, st>>>(r->params, r->buf, r->pixels, count);
-        PT_CUDA(cudaGetLastError());
+        if (r->small) {
+            PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
+            const int blocks = std::min(r->grid_small, (r->pixels + kSmallBlock - 1) / kSmallBlock);
+            render_small_kernel<<<blocks, kSmallBlock, 0, st>>>(scene, r->params, r->buf, r->pixels, count);
+            PT_CUDA(cudaGetLastError());
+        } else {
+            start_samples<<<(r->pixels + 255) / 256, 256, 0, st>>>(r->params, r->buf, r->pixels, count);
+            PT_CUDA(cudaGetLastError());
+        }
         // Every pixel needs at most count * (max_depth + 1) extends; the loop ends earlier when
         // the queue is empty.  The queue length is read back with a lag of a few iterations.
         // Iteration k: extend k and shade k on the main stream, shadow k on the shadow stream
@@ -530,7 +614,7 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         const int64_t max_iterations = int64_t(count) * (int64_t(r->params.max_depth) + 1) + 1;
         int parity = 0;
         int64_t issued = 0, checked = 0;
-        bool done = false, tail = false;
+        bool done = r->small, tail = false;
         while (!done && !tail && issued < max_iterations) {
             extend_kernel<<<r->grid_extend, r->block, stack_bytes(r->block), st>>>(scene, r->params, r->buf, parity, g_query_config.min_active);
             if (issued > 0) PT_CUDA(cudaStreamWaitEvent(st, r->shadowed[parity ^ 1].get(), 0));
@@ -596,6 +680,7 @@ pt_status pt_renderer_tuning(pt_renderer *r, int32_t tail_paths) {
     return guard([&]() {
         if (!r || tail_paths < 0) throw Error(PT_INVALID_ARGUMENT, "invalid renderer tuning");
         r->tail_paths = tail_paths;
+        r->small = false;   // an explicit wavefront / tail split asks for the general kernels
     });
 }
 

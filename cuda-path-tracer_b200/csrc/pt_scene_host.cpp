@@ -399,6 +399,13 @@ HostLayout relayout(const pt_scene_desc &s) {
         if(!shared) build_wide(s, slot, tri_slots, out);
     }
     for(const Bvh4Node &w : out.nodes4) out.nodes4q.push_back(quantize4(w));
+    // small scenes: every leaf's own box, in slot order
+    if(tri_leaves.size() + sphere_leaves.size() <= size_t(kSmallLeaves)) {
+        for(size_t k = 0; k < tri_leaves.size() + sphere_leaves.size(); k++) {
+            const pt_node &n = nodes[k < tri_leaves.size() ? tri_leaves[k] : sphere_leaves[k - tri_leaves.size()]];
+            out.small.push_back({{n.minimum.x, n.minimum.y, n.minimum.z}, {n.maximum.x, n.maximum.y, n.maximum.z}, int32_t(k), 0});
+        }
+    }
     // brute order: leaves in flat node-array order
     for(size_t id = 0; id < s.node_count; id++) {
         if(nodes[id].type == PT_BRANCH || slot[id] < 0) continue;

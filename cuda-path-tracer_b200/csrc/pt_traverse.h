@@ -77,6 +77,18 @@ PT_HD inline float next_up(float x) {
 #endif
 }
 
+// An accepted candidate at distance t < limit on leaf `slot` becomes the running answer unless it
+// ties with a better key; returns whether it did.
+PT_HD __forceinline__ bool accept_hit(const DeviceScene &s, int32_t slot, float t, float u, float v, int tie, bool any,
+                                      float &limit, HitInfo &hit) {
+    if (!any) {
+        if (hit.slot >= 0 && !(t < hit.t) && !(tie_key(s, slot, tie) < tie_key(s, hit.slot, tie))) return false;
+        limit = next_up(t);
+    }
+    hit.t = t; hit.u = u; hit.v = v; hit.slot = slot;
+    return true;
+}
+
 // Tests leaf `slot`; updates the running answer: hit.slot < 0 until a hit is accepted, then `limit`
 // is the float above the closest distance (an accepted t is below tmax, so nextafterf(t, tmax) is
 // next_up(t)).  The limit changes only here, so it is kept instead of being recomputed before each
@@ -97,13 +109,7 @@ PT_HD __forceinline__ bool test_leaf_rt(const DeviceScene &s, int32_t slot, cons
         SphereRecord sp = s.spheres[slot - s.tri_slots];
         ok = sphere_hit(sp, r, tmin, limit, t);
     }
-    if (!ok) return false;
-    if (!any) {
-        if (hit.slot >= 0 && !(t < hit.t) && !(tie_key(s, slot, tie) < tie_key(s, hit.slot, tie))) return false;
-        limit = next_up(t);
-    }
-    hit.t = t; hit.u = u; hit.v = v; hit.slot = slot;
-    return true;
+    return ok && accept_hit(s, slot, t, u, v, tie, any, limit, hit);
 }
 template <bool kAny>
 PT_HD __forceinline__ bool test_leaf(const DeviceScene &s, int32_t slot, const pt_ray &r, float dl, float tmin,
@@ -472,7 +478,7 @@ PT_HD inline float fma_box(float a, float b, float c) {
     return std::fma(a, b, c);
 #endif
 }
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
 // Two floats in one 64-bit register: one instruction multiplies (and adds) both, each rounded as
 // the scalar instruction rounds it.  The walk is bound by instruction issue, not by the FMA pipe
 // (2^25 rays on the 1M-triangle scene: 6.39 -> 6.35 ms with x and y of each slab in one instruction).
@@ -486,6 +492,11 @@ __device__ __forceinline__ void f2x_split(f2x v, float &a, float &b) { asm("mov.
 __device__ __forceinline__ f2x f2x_fma(f2x a, f2x b, f2x c) {
     f2x r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2x f2x_add(f2x a, f2x b) {
+    f2x r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ f2x f2x_mul(f2x a, f2x b) {
