@@ -87,6 +87,7 @@ __device__ inline ShadeCtx job_ctx(const BatchJob &j, int mis) {
 __device__ inline DeviceScene job_scene(const DeviceScene &merged, const BatchJob &j) {
     DeviceScene s = merged;
     s.lights = merged.lights + j.light_offset;
+    s.shade_lights = merged.shade_lights + j.light_offset;
     s.light_count = j.light_count;
     s.light_area = j.light_area;
     return s;
@@ -364,7 +365,7 @@ struct PinnedWords {
 
 struct pt_batch {
     DeviceScene view{};
-    DeviceBuffer nodes4, nodes2, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, jobs;
+    DeviceBuffer nodes4, nodes2, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, shade_tris, shade_lights, jobs;
     DeviceBuffer sums, rng, paths, hits, shadows, slot_pixel, slot_job, queue0, queue1, shadow_queue, counters, fetch, scalars,
         job_remaining, job_done_ns, error;
     std::vector<BatchJob> host_jobs;
@@ -632,6 +633,7 @@ void merge_scenes(pt_batch *b, const pt_scene_desc *descs, int32_t count, std::v
     v.light_count = 0; v.light_area = 0;   // per job
     v.empty = nodes4.empty() ? 1 : 0;
     v.root_leaf = 0;
+    build_shading(v, lights.size(), b->shade_tris, b->shade_lights);
 }
 } // namespace
 

@@ -235,10 +235,10 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
     } else {
         pt_ray r = cache_ray(s);
         HitInfo hi; hi.t = h.t; hi.u = h.u; hi.v = h.v; hi.slot = h.slot;
-        pt_flat_hit rec;
-        finalize_hit(scene, r, hi, rec);
-        const pt_material mat = scene.materials[rec.material_id];
-        f3 d = mk(s.dx, s.dy, s.dz), pos = mk(rec.p), normal = mk(rec.normal);
+        Surface rec;
+        surface_hit(scene, r, hi, rec);
+        const pt_material mat = scene.materials[rec.material];
+        f3 d = mk(s.dx, s.dy, s.dz), pos = rec.p, normal = rec.normal;
         const float dl2 = sqlen(d);
         const float dist2 = h.t * h.t * dl2;
         const float cosine = fmaxf(fabsf(dot(normal, d)) / sqrtf(dl2), 1e-4f);
@@ -247,7 +247,7 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
         const bool suffix = s.vertices >= 0;
         if (mat.type == PT_LIGHT) {
             float weight = s.prev_pdf > 0 ? mis_weight(s.prev_pdf, hit_light_pdf(scene, mk(s.ox, s.oy, s.oz), rec)) : 1;
-            f3 e = weight * trace_texture(scene, mat.texture_id, rec.u, rec.v);
+            f3 e = weight * surface_texture(scene, mat.texture_id, rec);
             R = R + T * e;
             if (suffix) S = S + U * e;
             o.finished = true;
@@ -259,12 +259,12 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
             // glass ones (roughness = fuzz, 0 for glass; albedo 1 for glass).
             const bool cacheable = diffuse || (p.query_specular && (mat.type == PT_METAL || mat.type == PT_GLASS));
             const f3 albedo = mat.type == PT_GLASS ? mk(1, 1, 1)
-                            : mat.type == PT_METAL ? mk(mat.albedo) : trace_texture(scene, mat.texture_id, rec.u, rec.v);
+                            : mat.type == PT_METAL ? mk(mat.albedo) : surface_texture(scene, mat.texture_id, rec);
             bool stop = false;
             if (cacheable && p.use_cache) {
                 const bool at_query = !suffix && s.depth >= 1 && s.spread * s.spread > p.spread_c * s.a0;
                 pt_cache_query cq;
-                cq.position = rec.p; cq.direction = pv(-(d / sqrtf(dl2))); cq.normal = rec.normal; cq.albedo = pv(albedo);
+                cq.position = pv(pos); cq.direction = pv(-(d / sqrtf(dl2))); cq.normal = pv(normal); cq.albedo = pv(albedo);
                 cq.roughness = diffuse ? 1.0f : (mat.type == PT_METAL ? fminf(mat.fuzz, 1.0f) : 0.0f);
                 if (at_query && s.train < 0) {
                     stop = true;
@@ -304,8 +304,7 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
                         float cosl = fmaxf(0, dot(normal, direction));
                         float pdf = light_direction_pdf(scene.light_area, pos, light.point, light.normal);
                         if (cosl > 0 && pdf > 0) {
-                            const pt_material &emitter = scene.materials[light.material];
-                            f3 emission = trace_texture(scene, emitter.texture_id, light.u, light.v);
+                            f3 emission = light_emission(scene, light);
                             float bsdf_pdf = cosl / float(M_PI);
                             f3 local = albedo * emission * (bsdf_pdf * mis_weight(pdf, bsdf_pdf) / pdf);
                             f3 c = T * local, cs = U * local;

@@ -59,6 +59,9 @@ private:
 };
 
 void require_device();
+// Fills the shading records of a scene whose other arrays are on the device (`lights` emitters) and
+// points the view at them.
+void build_shading(DeviceScene &view, size_t lights, DeviceBuffer &shade_tris, DeviceBuffer &shade_lights);
 int device_sm_count();
 // Ray counters per scene: launches further apart than this many may share one counter, so a scene
 // takes at most this many persistent-kernel launches in flight at once.
@@ -78,7 +81,7 @@ extern QueryConfig g_query_config;
 // The scene handle: everything device-resident that queries and renderers read.
 struct pt_scene {
     ptb::DeviceScene view{};
-    ptb::DeviceBuffer nodes, nodes4, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, brute_order, small;
+    ptb::DeviceBuffer nodes, nodes4, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, brute_order, small, shade_tris, shade_lights;
     std::vector<pt_light> host_lights;
     float light_area = 0;
     int32_t leaf_count = 0;

@@ -85,6 +85,20 @@ struct alignas(16) SmallLeaf {
 };
 static_assert(sizeof(SmallLeaf) == 32, "small-scene leaf is 32 bytes");
 
+// What shading needs of a triangle, per slot: the geometric normal as finalize_hit computes it, and
+// the material (~material when the face has smooth normals, which are then interpolated per hit).
+struct alignas(16) ShadeTri { float nx, ny, nz; int32_t material; };
+static_assert(sizeof(ShadeTri) == 16, "triangle shading record is 16 bytes");
+// What sampling an emitter needs, per emitter: a triangle's corners and unit normal, or a sphere's
+// center (p0) and radius (p1[0]).
+struct alignas(16) ShadeLight {
+    float p0[3]; int32_t type;
+    float p1[3]; int32_t material;
+    float p2[3]; int32_t primitive;
+    float n[3], pad;
+};
+static_assert(sizeof(ShadeLight) == 64, "emitter shading record is 64 bytes");
+
 // Everything a kernel needs, passed by value (device pointers).
 struct DeviceScene {
     const BvhNode *nodes;
@@ -97,6 +111,8 @@ struct DeviceScene {
     const pt_texture *textures;
     const unsigned char *pixels;
     const pt_light *lights;
+    const ShadeTri *shade_tris;     // per triangle slot
+    const ShadeLight *shade_lights; // per emitter
     int32_t node_count;             // internal nodes (0 for an empty scene)
     int32_t tri_slots, sphere_slots;
     int32_t light_count;

@@ -160,7 +160,52 @@ __global__ void surface_rays_kernel(const pt_triangle *tris, uint64_t triangles,
     if(tmax) tmax[k] = hi;
 }
 
+// The shading records, with finalize_hit's and sample_light's operations (pt_shade.h reads them
+// instead of the caller's 116-byte triangle records).
+__global__ void shade_tris_kernel(DeviceScene s, ShadeTri *out) {
+    int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if(k >= s.tri_slots) return;
+    const TriRecord &tr = s.tris[k];
+    const pt_triangle &face = s.triangles[tr.id];
+    f3 outward = cross(mk(face.v1) - mk(face.v0), mk(face.v2) - mk(face.v0));
+    outward = div_assign(outward, length(outward));
+    out[k] = ShadeTri{outward.x, outward.y, outward.z, face.smooth ? ~face.material_id : face.material_id};
+}
+__global__ void shade_lights_kernel(DeviceScene s, int32_t count, ShadeLight *out) {
+    int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if(k >= count) return;
+    const pt_light light = s.lights[k];
+    ShadeLight o{};
+    o.type = light.type; o.primitive = light.primitive;
+    if(light.type == PT_TRIANGLE) {
+        const pt_triangle &t = s.triangles[light.primitive];
+        const f3 n = unit(cross(mk(t.v1) - mk(t.v0), mk(t.v2) - mk(t.v0)));
+        o.p0[0] = t.v0.x; o.p0[1] = t.v0.y; o.p0[2] = t.v0.z;
+        o.p1[0] = t.v1.x; o.p1[1] = t.v1.y; o.p1[2] = t.v1.z;
+        o.p2[0] = t.v2.x; o.p2[1] = t.v2.y; o.p2[2] = t.v2.z;
+        o.n[0] = n.x; o.n[1] = n.y; o.n[2] = n.z;
+        o.material = t.material_id;
+    } else {
+        const pt_sphere &p = s.sphere_src[light.primitive];
+        o.p0[0] = p.center.x; o.p0[1] = p.center.y; o.p0[2] = p.center.z;
+        o.p1[0] = p.radius;
+        o.material = p.material_id;
+    }
+    out[k] = o;
+}
+
 unsigned grid_for(size_t count, int block) { return unsigned((count + size_t(block) - 1) / size_t(block)); }
+
+void build_shading(DeviceScene &view, size_t lights, DeviceBuffer &shade_tris, DeviceBuffer &shade_lights) {
+    shade_tris.resize(size_t(view.tri_slots) * sizeof(ShadeTri));
+    shade_lights.resize(lights * sizeof(ShadeLight));
+    if(view.tri_slots) shade_tris_kernel<<<grid_for(size_t(view.tri_slots), 256), 256>>>(view, shade_tris.get<ShadeTri>());
+    if(lights) shade_lights_kernel<<<grid_for(lights, 256), 256>>>(view, int32_t(lights), shade_lights.get<ShadeLight>());
+    PT_CUDA(cudaGetLastError());
+    PT_CUDA(cudaStreamSynchronize(nullptr));
+    view.shade_tris = shade_tris.get<ShadeTri>();
+    view.shade_lights = shade_lights.get<ShadeLight>();
+}
 
 // ---- ray ordering -----------------------------------------------------------------------------
 // A batch of at least kOrderMin rays is walked in the order of a 30-bit key: the direction's
@@ -404,6 +449,7 @@ pt_status pt_scene_create(const pt_scene_desc *desc, pt_scene **out) {
             v.empty = layout.empty;
             for(int a = 0; a < 3; a++) { v.root_lo[a] = layout.root_lo[a]; v.root_hi[a] = layout.root_hi[a]; }
             v.root_leaf = layout.root_leaf;
+            build_shading(v, lights.size(), sc->shade_tris, sc->shade_lights);
             v.small = sc->small.get<SmallLeaf>();
             v.small_count = int32_t(layout.small.size());
         } catch(...) { delete sc; throw; }
@@ -434,7 +480,8 @@ pt_status pt_scene_device_bytes(const pt_scene *s, size_t *bytes) {
     return guard([&]() {
         if(!s || !bytes) throw Error(PT_INVALID_ARGUMENT, "null argument");
         *bytes = s->nodes.bytes() + s->nodes4.bytes() + s->tris.bytes() + s->spheres.bytes() + s->triangles.bytes() + s->sphere_src.bytes() +
-                 s->materials.bytes() + s->textures.bytes() + s->pixels.bytes() + s->lights.bytes() + s->brute_order.bytes() + s->small.bytes();
+                 s->materials.bytes() + s->textures.bytes() + s->pixels.bytes() + s->lights.bytes() + s->brute_order.bytes() + s->small.bytes() +
+                 s->shade_tris.bytes() + s->shade_lights.bytes();
     });
 }
 

@@ -59,7 +59,64 @@ __device__ inline f3 cosine_direction(f3 normal, Pcg &random) {
     return radius * cosf(angle) * tangent + radius * sinf(angle) * bitangent + sqrtf(1 - u) * normal;
 }
 
-struct LightSample { f3 point, normal; float u, v; int material; };
+// The winning hit as shading uses it: finalize_hit's position and normal (flat_intersect.h:27-42,
+// 53-64) with the triangle's normal read from its 16-byte record, the texture coordinates left for
+// surface_texture, which most hits never need (with the emitters' records: Cornell render 3.06 -> 2.27
+// ms, six-job batch 14.0 -> 13.7, cached 1080p frame 12.0 -> 11.7; sphere hits no longer take an
+// atan2f, an asinf and two double divisions for coordinates a constant colour ignores).
+struct Surface {
+    f3 p, normal;
+    float u, v;                 // barycentric (triangles)
+    int32_t slot, material;
+};
+
+__device__ inline void surface_hit(const DeviceScene &s, const pt_ray &r, const HitInfo &h, Surface &o) {
+    o.u = h.u; o.v = h.v; o.slot = h.slot;
+    o.p = mk(r.origin) + h.t * mk(r.direction);
+    if (h.slot < s.tri_slots) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(&s.shade_tris[h.slot]));
+        const f3 outward = mk(a.x, a.y, a.z);
+        o.normal = outward;
+        o.material = __float_as_int(a.w);
+        if (o.material < 0) {   // smooth face
+            o.material = ~o.material;
+            const pt_triangle &face = s.triangles[s.tris[h.slot].id];
+            f3 interpolated = (1 - h.u - h.v) * mk(face.n0) + h.u * mk(face.n1) + h.v * mk(face.n2);
+            float length_squared = sqlen(interpolated);
+            if (length_squared > 0 && finite(length_squared)) {
+                f3 normal = unit(interpolated);
+                if (dot(normal, outward) < 0) normal = -normal;
+                if (dot(normal, outward) == 0) normal = outward;
+                o.normal = normal;
+            }
+        }
+    } else {
+        const SphereRecord &sr = s.spheres[h.slot - s.tri_slots];
+        o.normal = (o.p - mk(sr.cx, sr.cy, sr.cz)) / sr.radius;
+        o.material = s.sphere_src[sr.id].material_id;
+    }
+}
+
+// Texture coordinates of a hit, and the texture there (out of line: textures other than constant
+// colours are the rarer case, and the code is long).
+static __device__ __noinline__ f3 surface_texel(const DeviceScene &s, int32_t id, int32_t slot, float u, float v, f3 normal) {
+    if (slot < s.tri_slots) {
+        const pt_triangle &face = s.triangles[s.tris[slot].id];
+        f3 uv = (1 - u - v) * mk(face.uv0) + u * mk(face.uv1) + v * mk(face.uv2);
+        u = uv.x; v = uv.y;
+    } else {
+        sphere_uv(normal, u, v);
+    }
+    return trace_texture(s, id, u, v);
+}
+__device__ inline f3 surface_texture(const DeviceScene &s, int32_t id, const Surface &o) {
+    const pt_texture &tex = s.textures[id];
+    if (tex.type == PT_TEX_CONSTANT) return mk(tex.color);
+    return surface_texel(s, id, o.slot, o.u, o.v, o.normal);
+}
+
+// A sampled emitter point; `u`, `v` are the two uniform draws it came from.
+struct LightSample { f3 point, normal; float u, v; int32_t index, material; };
 
 // sample_light: area-weighted emitter choice, uniform point on it (light_sampling.h:27-54)
 __device__ inline LightSample sample_light(const DeviceScene &scene, Pcg &random) {
@@ -70,26 +127,44 @@ __device__ inline LightSample sample_light(const DeviceScene &scene, Pcg &random
         if (choice < scene.lights[middle].cumulative_area) high = middle;
         else low = middle + 1;
     }
-    const pt_light &light = scene.lights[low];
-    float u = random.uniform(), v = random.uniform();
+    const float4 *rec = reinterpret_cast<const float4 *>(&scene.shade_lights[low]);
+    const float4 p0 = __ldg(rec), p1 = __ldg(rec + 1);
     LightSample result;
-    if (light.type == PT_TRIANGLE) {
-        const pt_triangle &t = scene.triangles[light.primitive];
-        float root = sqrtf(u), a = 1 - root, b = root * (1 - v), c = root * v;
-        result.point = a * mk(t.v0) + b * mk(t.v1) + c * mk(t.v2);
-        result.normal = unit(cross(mk(t.v1) - mk(t.v0), mk(t.v2) - mk(t.v0)));
-        f3 uv = a * mk(t.uv0) + b * mk(t.uv1) + c * mk(t.uv2);
-        result.u = uv.x; result.v = uv.y; result.material = t.material_id;
+    result.u = random.uniform(); result.v = random.uniform();
+    result.index = low;
+    result.material = __float_as_int(p1.w);
+    if (__float_as_int(p0.w) == PT_TRIANGLE) {
+        const float4 p2 = __ldg(rec + 2), n = __ldg(rec + 3);
+        float root = sqrtf(result.u), a = 1 - root, b = root * (1 - result.v), c = root * result.v;
+        result.point = a * mk(p0.x, p0.y, p0.z) + b * mk(p1.x, p1.y, p1.z) + c * mk(p2.x, p2.y, p2.z);
+        result.normal = mk(n.x, n.y, n.z);
     } else {
-        const pt_sphere &s = scene.sphere_src[light.primitive];
-        float z = 1 - 2 * u, radius = sqrtf(fmaxf(0, 1 - z * z)), angle = 2 * float(M_PI) * v;
+        float z = 1 - 2 * result.u, radius = sqrtf(fmaxf(0, 1 - z * z)), angle = 2 * float(M_PI) * result.v;
         result.normal = mk(radius * cosf(angle), z, radius * sinf(angle));
-        result.point = mk(s.center) + fabsf(s.radius) * result.normal;
-        if (s.radius < 0) result.normal = -result.normal;
-        sphere_uv(result.normal, result.u, result.v);
-        result.material = s.material_id;
+        result.point = mk(p0.x, p0.y, p0.z) + fabsf(p1.x) * result.normal;
+        if (p1.x < 0) result.normal = -result.normal;
     }
     return result;
+}
+
+// The emitter's texture at the sampled point.
+static __device__ __noinline__ f3 light_texel(const DeviceScene &s, int32_t id, int32_t index, float u, float v, f3 normal) {
+    const pt_light &light = s.lights[index];
+    if (light.type == PT_TRIANGLE) {
+        const pt_triangle &t = s.triangles[light.primitive];
+        float root = sqrtf(u), a = 1 - root, b = root * (1 - v), c = root * v;
+        f3 uv = a * mk(t.uv0) + b * mk(t.uv1) + c * mk(t.uv2);
+        u = uv.x; v = uv.y;
+    } else {
+        sphere_uv(normal, u, v);
+    }
+    return trace_texture(s, id, u, v);
+}
+__device__ inline f3 light_emission(const DeviceScene &s, const LightSample &l) {
+    const int32_t id = s.materials[l.material].texture_id;
+    const pt_texture &tex = s.textures[id];
+    if (tex.type == PT_TEX_CONSTANT) return mk(tex.color);
+    return light_texel(s, id, l.index, l.u, l.v, l.normal);
 }
 
 // light_direction_pdf (light_sampling.h:56-65)
@@ -103,24 +178,29 @@ __device__ inline float light_direction_pdf(float area, f3 from, f3 point, f3 no
     return finite(pdf) ? pdf : 0;
 }
 
-// hit_light_pdf (light_sampling.h:67-73)
-__device__ inline float hit_light_pdf(const DeviceScene &scene, f3 from, const pt_flat_hit &hit) {
-    f3 normal = mk(hit.normal);
-    if (hit.primitive_type == PT_TRIANGLE) {
-        const pt_triangle &t = scene.triangles[hit.primitive_id];
-        normal = unit(cross(mk(t.v1) - mk(t.v0), mk(t.v2) - mk(t.v0)));
+// hit_light_pdf (light_sampling.h:67-73); a triangle's edges are those of its walk record
+__device__ inline float hit_light_pdf(const DeviceScene &scene, f3 from, const Surface &hit) {
+    f3 normal = hit.normal;
+    if (hit.slot < scene.tri_slots) {
+        TriRecord t;
+        load_tri(scene, hit.slot, t);
+        normal = unit(cross(mk(t.e1x, t.e1y, t.e1z), mk(t.e2x, t.e2y, t.e2z)));
     }
-    return light_direction_pdf(scene.light_area, from, mk(hit.p), normal);
+    return light_direction_pdf(scene.light_area, from, hit.p, normal);
 }
+
+// Schlick's pow(1 - cosine, 5) in double, as the reference's C++ promotes it; out of line, since the
+// code is long and only glass needs it
+static __device__ __noinline__ double schlick_pow(float cosine) { return pow(1 - cosine, 5); }
 
 // trace_scatter (transport.h:115-155)
 __device__ inline bool trace_scatter(const DeviceScene &scene, const pt_material &mat, f3 in_dir,
-                                     const pt_flat_hit &rec, Pcg &random, f3 &attenuation, f3 &out_dir) {
-    f3 p = mk(rec.p), n = mk(rec.normal);
+                                     const Surface &rec, Pcg &random, f3 &attenuation, f3 &out_dir) {
+    f3 p = rec.p, n = rec.normal;
     if (mat.type == PT_DIFFUSE) {
         f3 target = p + n + sample_ball(random);
         out_dir = target - p;
-        attenuation = trace_texture(scene, mat.texture_id, rec.u, rec.v);
+        attenuation = surface_texture(scene, mat.texture_id, rec);
         return true;
     }
     if (mat.type == PT_METAL) {
@@ -149,7 +229,7 @@ __device__ inline bool trace_scatter(const DeviceScene &scene, const pt_material
             refracted = ratio * (uv - outward * dt) - outward * sqrt(discriminant);
             float r0 = (1 - mat.ref_idx) / (1 + mat.ref_idx);
             r0 *= r0;
-            probability = r0 + (1 - r0) * pow(1 - cosine, 5);
+            probability = r0 + (1 - r0) * schlick_pow(cosine);
         }
         if (random.uniform() < probability) out_dir = reflected;
         else out_dir = refracted;

@@ -61,6 +61,15 @@ __device__ inline pt_ray path_ray(const PathState &s) {
     return r;
 }
 
+// The normals, triangle-id and material-id views' colour of a hit (out of line, off the shaded path).
+static __device__ __noinline__ f3 debug_color(const DeviceScene &scene, int debug, const pt_ray &r, const HitInfo &hi) {
+    pt_flat_hit rec;
+    finalize_hit(scene, r, hi, rec);
+    if (debug == PT_DEBUG_NORMALS) return 0.5f * (mk(rec.normal) + mk(1, 1, 1));
+    if (debug == PT_DEBUG_TRIANGLE) return rec.primitive_type == PT_TRIANGLE ? id_color(rec.primitive_id) : mk(0.3f, 0.3f, 0.3f);
+    return id_color(rec.material_id);
+}
+
 // The rest of one trace_color iteration for the path in `slot`, rendering `pixel` (its index
 // inside its image) (transport.h:179-228), given its closest
 // hit: emission with its MIS weight, next-event estimation (which may emit a shadow ray),
@@ -82,25 +91,23 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
     } else {
         pt_ray r = path_ray(s);
         HitInfo hi; hi.t = h.t; hi.u = h.u; hi.v = h.v; hi.slot = h.slot;
-        pt_flat_hit rec;
-        finalize_hit(scene, r, hi, rec);
-        if (p.debug == PT_DEBUG_NORMALS) { radiance = 0.5f * (mk(rec.normal) + mk(1, 1, 1)); finished = true; }
-        else if (p.debug == PT_DEBUG_TRIANGLE) {
-            radiance = rec.primitive_type == PT_TRIANGLE ? id_color(rec.primitive_id) : mk(0.3f, 0.3f, 0.3f);
+        if (p.debug != PT_DEBUG_SHADED) {
+            radiance = debug_color(scene, p.debug, r, hi);
             finished = true;
-        } else if (p.debug == PT_DEBUG_MATERIAL) { radiance = id_color(rec.material_id); finished = true; }
-        else {
-            const pt_material mat = scene.materials[rec.material_id];
+        } else {
+            Surface rec;
+            surface_hit(scene, r, hi, rec);
+            const pt_material mat = scene.materials[rec.material];
             f3 in_dir = mk(s.dx, s.dy, s.dz);
-            f3 pos = mk(rec.p), normal = mk(rec.normal);
+            f3 pos = rec.p, normal = rec.normal;
             if (mat.type == PT_LIGHT) {
                 float weight = s.prev_pdf > 0 ? mis_weight(s.prev_pdf, hit_light_pdf(scene, mk(s.ox, s.oy, s.oz), rec)) : 1;
-                radiance = radiance + weight * throughput * trace_texture(scene, mat.texture_id, rec.u, rec.v);
+                radiance = radiance + weight * throughput * surface_texture(scene, mat.texture_id, rec);
                 finished = true;
             } else if (s.depth == p.max_depth) {
                 finished = true;
             } else if (p.mis && mat.type == PT_DIFFUSE) {
-                f3 attenuation = trace_texture(scene, mat.texture_id, rec.u, rec.v);
+                f3 attenuation = surface_texture(scene, mat.texture_id, rec);
                 if (scene.light_count) {
                     LightSample light = sample_light(scene, rng);
                     f3 delta = light.point - pos;
@@ -110,8 +117,7 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
                         float cosine = fmaxf(0, dot(normal, direction));
                         float pdf = light_direction_pdf(scene.light_area, pos, light.point, light.normal);
                         if (cosine > 0 && pdf > 0) {
-                            const pt_material &emitter = scene.materials[light.material];
-                            f3 emission = trace_texture(scene, emitter.texture_id, light.u, light.v);
+                            f3 emission = light_emission(scene, light);
                             float bsdf_pdf = cosine / float(M_PI);
                             f3 c = throughput * attenuation * emission * (bsdf_pdf * mis_weight(pdf, bsdf_pdf) / pdf);
                             sr.ox = pos.x; sr.oy = pos.y; sr.oz = pos.z; sr.tmax = distance - 0.001f;
