@@ -316,9 +316,11 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
 // copy of the walk, and shades together, so all lanes stay in the same code: with the divergent
 // tree walk 10 of 32 lanes were busy and warps waited on instruction fetch.  A lane whose pixel is
 // done takes the next one from fetch[3].  The shadow contribution of bounce k is added before
-// bounce k + 1 is shaded, as in every other form.  Blocks of 64 spread a small image's paths evenly
-// over the SMs.
-constexpr int kSmallBlock = 64;
+// bounce k + 1 is shaded, as in every other form.  The warps of a block start each walk and each
+// shading together (the two block barriers): the 70 KB of code of a round is more than the
+// instruction caches next to the schedulers hold, and warps in step fetch it once for all of them
+// (Cornell box, 64,000 paths: 2.27 ms in free-running blocks of 64, 2.0 in step in blocks of 256).
+constexpr int kSmallBlock = 256;
 __global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene scene, RenderParams p, RenderBuffers b, int32_t count,
                                                                   int samples) {
     __shared__ SmallScene sh;
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene s
                 }
             }
         }
-        if (!__any_sync(full, live)) break;
+        if (!__syncthreads_or(live)) break;
         HitInfo hi;
         bool hit = false;
         for (int pass = __any_sync(full, pending) ? 0 : 1; pass < 2; pass++) {
@@ -372,6 +374,7 @@ __global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene s
             }
             __syncwarp();
         }
+        __syncthreads();
         if (live) {
             PathHit h;
             h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = hit ? hi.slot : -1;
