@@ -15,19 +15,30 @@
 #ifdef __CUDACC__
 namespace ptb {
 
+// The boxes are stored once per sign pattern of the ray direction, entered planes first: a lane then
+// needs no selects (6 of 20 instructions a box), and the eight patterns of a leaf are 128
+// consecutive bytes, so lanes of any mix of patterns read them without bank conflicts (Cornell
+// render 2.00 -> 1.87 ms).
 struct SmallScene {                    // in shared memory
-    float4 xy[kSmallLeaves];           // box: min x, min y, max x, max y
-    float2 z[kSmallLeaves];            // min z, max z
+    ulonglong2 xy[kSmallLeaves][8];    // (near x, near y), (far x, far y) as packed floats
+    unsigned long long z[kSmallLeaves][8];   // (near z, far z)
     float4 record[kSmallLeaves][3];    // TriRecord, or SphereRecord in the first two
     int32_t slot[kSmallLeaves];
 };
 
 // Fills `sh` with the block's threads; the boxes are widened by `pad` on every side.
 __device__ inline void small_load(const DeviceScene &s, SmallScene &sh, float pad) {
+    for (int j = threadIdx.x; j < 8 * s.small_count; j += blockDim.x) {
+        const SmallLeaf leaf = s.small[j >> 3];
+        const float lo[3] = {leaf.lo[0] - pad, leaf.lo[1] - pad, leaf.lo[2] - pad};
+        const float hi[3] = {leaf.hi[0] + pad, leaf.hi[1] + pad, leaf.hi[2] + pad};
+        const bool nx = j & 1, ny = j & 2, nz = j & 4;
+        sh.xy[j >> 3][j & 7] = make_ulonglong2(f2x_make(nx ? hi[0] : lo[0], ny ? hi[1] : lo[1]),
+                                               f2x_make(nx ? lo[0] : hi[0], ny ? lo[1] : hi[1]));
+        sh.z[j >> 3][j & 7] = f2x_make(nz ? hi[2] : lo[2], nz ? lo[2] : hi[2]);
+    }
     for (int k = threadIdx.x; k < s.small_count; k += blockDim.x) {
         const SmallLeaf leaf = s.small[k];
-        sh.xy[k] = make_float4(leaf.lo[0] - pad, leaf.lo[1] - pad, leaf.hi[0] + pad, leaf.hi[1] + pad);
-        sh.z[k] = make_float2(leaf.lo[2] - pad, leaf.hi[2] + pad);
         sh.slot[k] = leaf.slot;
         if (leaf.slot < s.tri_slots) {
             const float4 *p = reinterpret_cast<const float4 *>(&s.tris[leaf.slot]);
@@ -47,15 +58,15 @@ __device__ __forceinline__ bool small_walk(const DeviceScene &s, const SmallScen
     const RayBox rb = ray_box(r);
     const f2x oxy = f2x_make(-rb.ox, -rb.oy), ozz = f2x_make(-rb.oz, -rb.oz);   // a - b and a + (-b) round alike
     const f2x ixy = f2x_make(rb.ix, rb.iy), izz = f2x_make(rb.iz, rb.iz);
+    const int pattern = (rb.nx ? 1 : 0) | (rb.ny ? 2 : 0) | (rb.nz ? 4 : 0);
     uint32_t passed = 0;
 #pragma unroll 4
     for (int k = 0; k < s.small_count; k++) {
-        const float4 b = sh.xy[k];
-        const float2 z = sh.z[k];
+        const ulonglong2 xy = sh.xy[k][pattern];
         float ax, ay, az, bx, by, bz;
-        f2x_split(f2x_mul(f2x_add(f2x_make(rb.nx ? b.z : b.x, rb.ny ? b.w : b.y), oxy), ixy), ax, ay);
-        f2x_split(f2x_mul(f2x_add(f2x_make(rb.nx ? b.x : b.z, rb.ny ? b.y : b.w), oxy), ixy), bx, by);
-        f2x_split(f2x_mul(f2x_add(f2x_make(rb.nz ? z.y : z.x, rb.nz ? z.x : z.y), ozz), izz), az, bz);
+        f2x_split(f2x_mul(f2x_add(xy.x, oxy), ixy), ax, ay);
+        f2x_split(f2x_mul(f2x_add(xy.y, oxy), ixy), bx, by);
+        f2x_split(f2x_mul(f2x_add(sh.z[k][pattern], ozz), izz), az, bz);
         const float lo = fmaxf(max3(tmin, ax, ay), az), hi = fminf(min3(tmax, bx, by), bz);
         if (hi > lo) passed |= 1u << k;
     }
