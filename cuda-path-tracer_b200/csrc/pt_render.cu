@@ -18,6 +18,7 @@
 #include <vector>
 #include "pt_api_common.h"
 #include "pt_device.h"
+#include "pt_paths.h"
 #include "pt_small.h"
 #include "pt_wavefront.h"
 
@@ -45,6 +46,9 @@ struct RenderBuffers {
     int32_t *error;
     float *sums;
     Pcg *rng;
+    PathState *lane_paths;  // per lane of render_paths_kernel
+    ShadowRay *lane_shadows;
+    int32_t *claims;        // samples of each pixel drawn and not yet run (render_paths_kernel; zero between launches)
 };
 
 __device__ inline void camera_path(const RenderParams &p, int32_t pixel, Pcg &rng, PathState &s) {
@@ -261,6 +265,7 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
                 i = b.queue[parity][k];
                 s = b.paths[i];
                 rng = b.rng[i];
+                if (s.samples_left < 0) { s.samples_left = b.claims[i]; b.claims[i] = 0; }   // from render_paths_kernel
                 live = true;
             } else {
                 drained = true;
@@ -386,6 +391,79 @@ __global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene s
     if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
 }
 
+// The whole render in one kernel (four-wide tree, shaded view): pt_paths.h's loop over the image's
+// pixels.  Path and shadow records are the lane's (lane_paths, lane_shadows).  What a sample reads of
+// the pixel's earlier ones (stream and sum) goes past the L1, since they may have run on another SM.
+struct RenderOps {
+    const DeviceScene &scene;
+    const RenderParams &p;
+    const RenderBuffers &b;
+    ShadeCtx ctx;
+    uint32_t pixels;
+    uint32_t lane;              // index of the lane's records
+    int32_t i;                  // the pixel
+    __device__ void first_ray() {
+        const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(&b.rng[i]));
+        Pcg rng;
+        rng.state = w.x; rng.increment = w.y;
+        PathState s;
+        camera_path(p, i, rng, s);
+        s.samples_left = 1;
+        b.lane_paths[lane] = s;
+        b.rng[i] = rng;
+    }
+    __device__ bool claim(unsigned long long item, int32_t &root) {
+        i = (item >> 32) ? int32_t(item % pixels) : int32_t(uint32_t(item) % pixels);
+        if (atomicAdd(&b.claims[i], 1) != 0) return false;   // the lane running this pixel will see it
+        __threadfence();
+        root = 0;
+        first_ray();
+        return true;
+    }
+    __device__ bool again() {
+        __threadfence();                                     // the stream and the sum, before the claim goes
+        if (atomicSub(&b.claims[i], 1) == 1) return false;
+        first_ray();
+        return true;
+    }
+    // to finish_pair_kernel's queue; how many of the pixel's samples are claimed is only known once
+    // this kernel has ended, so the tail kernel reads it (samples_left < 0)
+    __device__ void hand_over() {
+        PathState s = b.lane_paths[lane];
+        s.samples_left = -1;
+        b.paths[i] = s;
+        b.queue[0][atomicAdd(&b.counters[0], 1)] = i;
+    }
+    __device__ void shade(const PathHit &h, NextWalk &n) {
+        PathState s = b.lane_paths[lane];
+        Pcg rng = b.rng[i];
+        ShadowRay sr;
+        n.live = shade_path(scene, ctx, b.sums + 3 * size_t(i), i, i, s, h, make_uint2(0, 0), rng, sr, n.shadow);
+        b.rng[i] = rng;
+        if (n.live) b.lane_paths[lane] = s;
+        if (n.shadow) b.lane_shadows[lane] = sr;
+    }
+    __device__ void ray(bool shadow, pt_ray &r, float &tmax) { lane_ray(b.lane_paths[lane], b.lane_shadows[lane], shadow, r, tmax); }
+    __device__ void unblocked() {
+        PathState &s = b.lane_paths[lane];
+        const ShadowRay &sr = b.lane_shadows[lane];
+        s.rr = s.rr + sr.cr; s.rg = s.rg + sr.cg; s.rb = s.rb + sr.cb;
+    }
+};
+
+__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) render_paths_kernel(DeviceScene scene, RenderParams p, RenderBuffers b,
+                                                                                     int32_t pixels, int samples, bool hand_over) {
+    ShadeCtx ctx;
+    ctx.camera = &p.camera; ctx.width = p.width; ctx.height = p.height; ctx.max_depth = p.max_depth;
+    ctx.debug = PT_DEBUG_SHADED; ctx.mis = p.mis;
+    RenderOps ops{scene, p, b, ctx, uint32_t(pixels), blockIdx.x * blockDim.x + threadIdx.x, 0};
+    unsigned long long rays = 0;
+    persistent_paths4(scene, ops, (unsigned long long)pixels * (unsigned long long)samples, &b.fetch[3], hand_over, kTieLastLeaf, rays,
+                      b.error);
+    for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(0xffffffffu, rays, o);
+    if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
+}
+
 // shadow: any-hit of the NEE rays (transport.h:206-214); unoccluded ones add their contribution
 __global__ void __launch_bounds__(256, 4) shadow_kernel(DeviceScene scene, RenderParams p, RenderBuffers b, int parity, int min_active) {
     const int32_t n = b.counters[2 + parity];
@@ -467,11 +545,12 @@ struct pt_renderer {
     // threads per block of the wavefront kernels (pt_set_block_shape): 16x8 by default (config 2:
     // 64.3 ms per render against 65.1 with the reference's 16x16; config 1 unchanged)
     int block = 128;
-    int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0;
+    int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0, grid_paths = 0;
     int32_t tail_paths = 0;             // live-path count below which the fused finish kernel takes over
     bool pair_tail = false;             // the tail runs two lanes per path (finish_pair_kernel)
+    bool fused = false;                 // four-wide tree and shaded view: render_paths_kernel where the image's size suits it
     bool small = false;                 // the scene fits render_small_kernel and the view is shaded
-    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba;
+    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lane_paths, lane_shadows;
     RenderBuffers buf{};
     cudaStream_t stream = nullptr;
     cudaStream_t shadow_stream = nullptr;   // shadow kernel k runs beside extend k+1
@@ -490,6 +569,10 @@ struct pt_renderer {
         grid_shadow = occupancy_grid((const void *)shadow_kernel, block, stack_bytes(block));
         grid_finish = occupancy_grid((const void *)finish_kernel, kFinishBlock);
         grid_finish_pair = occupancy_grid((const void *)finish_pair_kernel, block);
+        grid_paths = occupancy_grid((const void *)render_paths_kernel, kPathsBlock, stack_bytes(kPathsBlock));
+        lane_paths.resize(size_t(grid_paths) * kPathsBlock * sizeof(PathState));
+        lane_shadows.resize(size_t(grid_paths) * kPathsBlock * sizeof(ShadowRay));
+        buf.lane_paths = lane_paths.get<PathState>(); buf.lane_shadows = lane_shadows.get<ShadowRay>();
         grid_small = occupancy_grid((const void *)render_small_kernel, kSmallBlock);
     }
 };
@@ -543,6 +626,8 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             r->ray_total.resize(sizeof(unsigned long long));
             r->error.resize(sizeof(int32_t));
             r->sums.resize(n * 3 * sizeof(float));
+            r->claims.resize(n * sizeof(int32_t));
+            PT_CUDA(cudaMemset(r->claims.get(), 0, n * sizeof(int32_t)));
             r->rng.resize(n * sizeof(Pcg));
             RenderBuffers &b = r->buf;
             b.paths = r->paths.get<PathState>(); b.hits = r->hits.get<PathHit>(); b.stats = r->stats.get<uint2>();
@@ -551,7 +636,7 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             b.shadow_queue = r->shadow_queue.get<int32_t>(); b.counters = r->counters.get<int32_t>();
             b.fetch = r->fetch.get<unsigned long long>();
             b.rays = r->ray_total.get<unsigned long long>(); b.error = r->error.get<int32_t>();
-            b.sums = r->sums.get<float>(); b.rng = r->rng.get<Pcg>();
+            b.sums = r->sums.get<float>(); b.rng = r->rng.get<Pcg>(); b.claims = r->claims.get<int32_t>();
             PT_CUDA(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking));
             PT_CUDA(cudaStreamCreateWithFlags(&r->shadow_stream, cudaStreamNonBlocking));
             PT_CUDA(cudaMallocHost(&r->host_counters, kIterationRing * sizeof(int32_t)));
@@ -567,6 +652,7 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             constexpr size_t kSmallTreeNodes = 32;
             if (p.wide && scene->nodes4.bytes() / sizeof(Bvh4QNode) <= kSmallTreeNodes) p.wide = 0;
             r->pair_tail = p.wide != 0;
+            r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
             r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
         } catch (...) { delete r; throw; }
         *out = r;
@@ -600,11 +686,31 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         cudaStream_t st = r->stream;
         PT_CUDA(cudaMemsetAsync(r->buf.rays, 0, sizeof(unsigned long long), st));
         PT_CUDA(cudaEventRecord(r->start.get(), st));
+        // One kernel for the whole render (render_paths_kernel) where every resident lane has a pixel: with
+        // fewer, the tail kernel's two lanes per path are faster (240x150, 16 spp: 3.7 ms against 5.0; 320x240
+        // 6.7 against 6.2), except for one or two samples, where the wavefront's launches are most of the time
+        // (240x150: 0.88 ms against 0.47).  Up to 40 pixels per lane: from there on the wavefront's queues are long
+        // enough to hide their slowest rays and its walk kernels hold twice the warps (1920x1080 30.4 ms
+        // against 29.0; 3840x2160 91.8 against 111.8).
+        const int64_t lanes = int64_t(r->grid_paths) * kPathsBlock;
+        const bool whole = r->fused && r->pixels <= 40 * lanes && (r->pixels >= lanes || count <= 2);
         if (r->small) {
             PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
             const int blocks = std::min(r->grid_small, (r->pixels + kSmallBlock - 1) / kSmallBlock);
             render_small_kernel<<<blocks, kSmallBlock, 0, st>>>(scene, r->params, r->buf, r->pixels, count);
             PT_CUDA(cudaGetLastError());
+        } else if (whole) {
+            PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
+            PT_CUDA(cudaMemsetAsync(r->buf.counters, 0, sizeof(int32_t), st));
+            const bool hand_over = count > 2;
+            const int blocks = std::min(r->grid_paths, (r->pixels + 31) / 32);
+            render_paths_kernel<<<blocks, kPathsBlock, stack_bytes(kPathsBlock), st>>>(scene, r->params, r->buf, r->pixels, count, hand_over);
+            PT_CUDA(cudaGetLastError());
+            if (hand_over) {
+                PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
+                finish_pair_kernel<<<r->grid_finish_pair, r->block, 0, st>>>(scene, r->params, r->buf, 0);
+                PT_CUDA(cudaGetLastError());
+            }
         } else {
             start_samples<<<(r->pixels + 255) / 256, 256, 0, st>>>(r->params, r->buf, r->pixels, count);
             PT_CUDA(cudaGetLastError());
@@ -617,7 +723,7 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         const int64_t max_iterations = int64_t(count) * (int64_t(r->params.max_depth) + 1) + 1;
         int parity = 0;
         int64_t issued = 0, checked = 0;
-        bool done = r->small, tail = false;
+        bool done = r->small || whole, tail = false;
         while (!done && !tail && issued < max_iterations) {
             extend_kernel<<<r->grid_extend, r->block, stack_bytes(r->block), st>>>(scene, r->params, r->buf, parity, g_query_config.min_active);
             if (issued > 0) PT_CUDA(cudaStreamWaitEvent(st, r->shadowed[parity ^ 1].get(), 0));
@@ -683,7 +789,7 @@ pt_status pt_renderer_tuning(pt_renderer *r, int32_t tail_paths) {
     return guard([&]() {
         if (!r || tail_paths < 0) throw Error(PT_INVALID_ARGUMENT, "invalid renderer tuning");
         r->tail_paths = tail_paths;
-        r->small = false;   // an explicit wavefront / tail split asks for the general kernels
+        r->small = r->fused = false;   // an explicit wavefront / tail split asks for the general kernels
     });
 }
 

@@ -148,7 +148,8 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
     }
     if (finished) {
         // accumulated += trace_pixel_sample(...) (src/cuda/cuda_renderer.cu:81)
-        sum[0] = sum[0] + radiance.x; sum[1] = sum[1] + radiance.y; sum[2] = sum[2] + radiance.z;
+        // (read past the L1: a pixel's samples may run on different SMs, pt_paths.h)
+        __stcg(sum, __ldcg(sum) + radiance.x); __stcg(sum + 1, __ldcg(sum + 1) + radiance.y); __stcg(sum + 2, __ldcg(sum + 2) + radiance.z);
         s.samples_left--;
         if (s.samples_left > 0) {
             int left = s.samples_left;

@@ -244,7 +244,9 @@ pt_status pt_set_block_shape(pt_renderer *renderer, int width, int height);
 /* Live-path count below which add_samples stops the wavefront and runs the remaining paths to
  * completion in one fused kernel (two threads per path on four-wide trees: one walks the path's
  * next ray while the other walks its last shadow ray; default max(65536, pixels/4); 0 keeps the
- * wavefront to the end).  Results do not depend on it. */
+ * wavefront to the end).  Until this is called, shaded renders of scenes of at most 32 primitives, and
+ * of images that give every resident GPU thread one to forty pixels, run as one kernel from the first
+ * camera ray to the last bounce; calling it asks for the wavefront.  Results do not depend on it. */
 pt_status pt_renderer_tuning(pt_renderer *renderer, int32_t tail_paths);
 /* Linear FP32 radiance sums (3 floats per pixel, row 0 at the bottom, not divided by spp). */
 pt_status pt_get_sums(const pt_renderer *renderer, float *rgb_sums, size_t floats);
