@@ -19,7 +19,7 @@
 #include <vector>
 #include "pt_api_common.h"
 #include "pt_device.h"
-#include "pt_wavefront.h"
+#include "pt_paths.h"
 
 using namespace ptb;
 
@@ -59,6 +59,10 @@ struct BatchBuffers {
     unsigned long long *start_ns;
     int32_t *error;
     unsigned long long *iterations;
+    PathState *lane_paths;            // per lane of batch_paths
+    ShadowRay *lane_shadows;
+    int32_t *claims;                  // per pixel: samples drawn and not yet run (batch_paths; zero between runs)
+    int32_t *done;                    // per pixel: samples run by batch_paths
 };
 
 __device__ inline unsigned long long globaltimer() {
@@ -101,6 +105,7 @@ __global__ void batch_init(BatchBuffers b) {
     b.sums[3 * g] = 0; b.sums[3 * g + 1] = 0; b.sums[3 * g + 2] = 0;
     Pcg r; r.seed(j.seed, uint64_t(g - j.pixel_offset));
     b.rng[g] = r;
+    if (b.done) b.done[g] = 0;
 }
 
 // A slot starts pixel g: its first camera ray.
@@ -292,6 +297,7 @@ __global__ void __launch_bounds__(256, 2) batch_finish_pair(DeviceScene scene, B
                 if (k < (unsigned long long)n) {
                     slot = b.queue[0][k];
                     s = b.paths[slot]; g = b.slot_pixel[slot]; jid = b.slot_job[slot]; rng = b.rng[g];
+                    if (s.samples_left < 0) { s.samples_left = b.claims[g]; b.claims[g] = 0; }   // from batch_paths
                     live = true;
                 } else {
                     drained = true;
@@ -350,6 +356,98 @@ __global__ void __launch_bounds__(256, 2) batch_finish_pair(DeviceScene scene, B
     if (lane == 0 && rays) atomicAdd(b.rays, rays);
 }
 
+// The whole batch in one kernel (four-wide trees): pt_paths.h's loop over all jobs' pixels, a sample at
+// a time; a pixel's items past its job's sample count start nothing.  What a sample reads of the pixel's
+// earlier ones (stream, sum, count of samples run) goes past the L1.  The last paths go to
+// batch_finish_pair.
+struct BatchOps {
+    const DeviceScene &merged;
+    const BatchBuffers &b;
+    uint32_t lane;              // index of the lane's records
+    int32_t jid;
+    int64_t g;                  // the pixel
+    __device__ void first_ray() {
+        const BatchJob &j = b.jobs[jid];
+        const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(&b.rng[g]));
+        Pcg rng;
+        rng.state = w.x; rng.increment = w.y;
+        PathState s;
+        camera_path(j.camera, j.width, j.height, int32_t(g - j.pixel_offset), rng, s);
+        s.samples_left = 1;
+        b.lane_paths[lane] = s;
+        b.rng[g] = rng;
+    }
+    __device__ bool claim(unsigned long long item, int32_t &root) {
+        const unsigned long long pixels = (unsigned long long)b.total_pixels;
+        unsigned long long pass;
+        if ((item | pixels) >> 32) { pass = item / pixels; g = int64_t(item % pixels); }
+        else { pass = uint32_t(item) / uint32_t(pixels); g = uint32_t(item) % uint32_t(pixels); }
+        jid = job_of(b, g);
+        const BatchJob &j = b.jobs[jid];
+        if (pass >= (unsigned long long)j.samples) return false;
+        if (atomicAdd(&b.claims[g], 1) != 0) return false;   // the lane running this pixel will see it
+        __threadfence();
+        root = j.root;
+        first_ray();
+        return true;
+    }
+    __device__ bool again() {
+        const int32_t done = __ldcg(&b.done[g]) + 1;
+        __stcg(&b.done[g], done);
+        if (done == b.jobs[jid].samples && atomicSub(&b.job_remaining[jid], 1) == 1) b.job_done_ns[jid] = globaltimer();
+        __threadfence();                                     // stream, sum and count, before the claim goes
+        if (atomicSub(&b.claims[g], 1) == 1) return false;
+        first_ray();
+        return true;
+    }
+    __device__ void shade(const PathHit &h, NextWalk &n) {
+        const BatchJob &j = b.jobs[jid];
+        DeviceScene js = job_scene(merged, j);
+        PathState s = b.lane_paths[lane];
+        Pcg rng = b.rng[g];
+        ShadowRay sr;
+        n.live = shade_path(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), int32_t(lane), s, h, make_uint2(0, 0),
+                            rng, sr, n.shadow);
+        b.rng[g] = rng;
+        if (n.live) b.lane_paths[lane] = s;
+        if (n.shadow) b.lane_shadows[lane] = sr;
+    }
+    __device__ void ray(bool shadow, pt_ray &r, float &tmax) { lane_ray(b.lane_paths[lane], b.lane_shadows[lane], shadow, r, tmax); }
+    __device__ void unblocked() {
+        PathState &s = b.lane_paths[lane];
+        const ShadowRay &sr = b.lane_shadows[lane];
+        s.rr = s.rr + sr.cr; s.rg = s.rg + sr.cg; s.rb = s.rb + sr.cb;
+    }
+    // batch_finish_pair's queue; the tail reads the pixel's claims once this kernel has ended (samples_left < 0)
+    __device__ void hand_over() {
+        PathState s = b.lane_paths[lane];
+        s.samples_left = -1;
+        const int32_t slot = atomicAdd(&b.counters[0], 1);   // at most one per lane, and there are as many slots
+        b.paths[slot] = s;
+        b.slot_pixel[slot] = g;
+        b.slot_job[slot] = jid;
+        b.queue[0][slot] = slot;
+    }
+};
+
+__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) batch_paths(DeviceScene scene, BatchBuffers b,
+                                                                             unsigned long long items, bool hand_over) {
+    BatchOps ops{scene, b, blockIdx.x * blockDim.x + threadIdx.x, 0, 0};
+    unsigned long long rays = 0;
+    persistent_paths4(scene, ops, items, &b.fetch[0], hand_over, kTieLastLeaf, rays, b.error);
+    for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(0xffffffffu, rays, o);
+    if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
+}
+
+// What batch_paths and the tail after it expect: no slot queued, no pixel left to start.
+__global__ void batch_paths_start(BatchBuffers b) {
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    b.counters[0] = 0;
+    b.fetch[0] = 0; b.fetch[3] = 0;
+    *b.cursor = (unsigned long long)b.total_pixels;
+    *b.start_ns = globaltimer();
+}
+
 } // namespace ptb
 
 namespace ptb {
@@ -367,7 +465,7 @@ struct pt_batch {
     DeviceScene view{};
     DeviceBuffer nodes4, nodes2, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, shade_tris, shade_lights, jobs;
     DeviceBuffer sums, rng, paths, hits, shadows, slot_pixel, slot_job, queue0, queue1, shadow_queue, counters, fetch, scalars,
-        job_remaining, job_done_ns, error;
+        job_remaining, job_done_ns, error, lane_paths, lane_shadows, claims, done;
     std::vector<BatchJob> host_jobs;
     int64_t total_pixels = 0;
     uint64_t total_triangles = 0;
@@ -423,7 +521,34 @@ struct pt_batch {
         buf.paths = paths.get<PathState>(); buf.hits = hits.get<PathHit>(); buf.shadows = shadows.get<ShadowRay>();
         buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
         buf.queue[0] = queue0.get<int32_t>(); buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
+        if (one_kernel() && !buf.claims) {
+            const size_t lanes = size_t(grid_paths()) * kPathsBlock;
+            lane_paths.resize(lanes * sizeof(PathState)); lane_shadows.resize(lanes * sizeof(ShadowRay));
+            claims.resize(size_t(total_pixels) * sizeof(int32_t)); done.resize(size_t(total_pixels) * sizeof(int32_t));
+            PT_CUDA(cudaMemset(claims.get(), 0, claims.bytes()));
+            buf.lane_paths = lane_paths.get<PathState>(); buf.lane_shadows = lane_shadows.get<ShadowRay>();
+            buf.claims = claims.get<int32_t>(); buf.done = done.get<int32_t>();
+        }
         drop_graph();
+    }
+    int grid_paths() const {
+        int per_sm = 0;
+        PT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)batch_paths, kPathsBlock,
+                                                              size_t(kSharedStack4) * sizeof(int2) * kPathsBlock));
+        return device_sm_count() * (per_sm > 0 ? per_sm : 1);
+    }
+    int32_t max_samples() const {
+        int32_t most = 0;
+        for (const auto &j : host_jobs) most = std::max(most, j.samples);
+        return most;
+    }
+    // Whether a graph-form run of four-wide nodes is one batch_paths launch: for the pixel counts where that is
+    // the faster form (the renderer's rule, pt_add_samples), if every lane could queue its path for the tail.
+    // Six jobs, device time of the graph form and of this: 129,000 pixels 6.8 and 3.2 ms, 534,000 11.9 and 7.0, 1.2M
+    // 32.0 and 25.8, 2.3M 20.6 and 19.5.
+    bool one_kernel() const {
+        const int64_t lanes = int64_t(grid_paths()) * kPathsBlock;
+        return total_pixels <= 40 * lanes && total_pixels >= lanes && slots >= lanes;
     }
     unsigned long long max_iterations() const {
         // every pixel needs at most samples * (depth + 1) extends; slots run pixels back to back
@@ -484,9 +609,20 @@ struct pt_batch {
         PT_CUDA(cudaMemsetAsync(buf.error, 0, sizeof(int32_t), st));
         batch_init<<<unsigned((total_pixels + 255) / 256), 256, 0, st>>>(buf);
         PT_CUDA(cudaEventRecord(start.get(), st));
-        batch_start<<<(slots + 255) / 256, 256, 0, st>>>(buf, slots);
+        const bool whole = use_graph && wide && buf.claims && one_kernel();
+        if (whole) {
+            const size_t smem = size_t(kSharedStack4) * sizeof(int2) * kPathsBlock;
+            batch_paths_start<<<1, 32, 0, st>>>(buf);
+            batch_paths<<<grid_paths(), kPathsBlock, smem, st>>>(view, buf, (unsigned long long)total_pixels * (unsigned long long)max_samples(),
+                                                                 true);
+            PT_CUDA(cudaGetLastError());
+            launch_finish(st);
+        } else {
+            batch_start<<<(slots + 255) / 256, 256, 0, st>>>(buf, slots);
+        }
         PT_CUDA(cudaGetLastError());
-        if (use_graph) {
+        if (whole) {
+        } else if (use_graph) {
             if (!exec) build_graph();
             PT_CUDA(cudaGraphLaunch(exec, st));
         } else {

@@ -285,7 +285,9 @@ pt_status pt_batch_get_sums(const pt_batch *batch, int32_t job, float *rgb_sums,
 pt_status pt_batch_stats(const pt_batch *batch, float *kernel_ms, uint64_t *rays, double *job_completion_ms, size_t jobs);
 /* path_capacity: path slots (0 = min(pixels, 2^22)); block: 64, 128 or 256 threads; min_active:
  * traversal refill threshold; tail_paths: live paths below which the fused kernel finishes;
- * use_graph: 1 = one graph launch with a device-side loop, 0 = host-driven loop. */
+ * use_graph: 1 = the loop runs on the device (one graph launch; or, on four-wide nodes, with one to
+ * forty pixels per resident GPU thread and a slot for each such thread, one kernel that walks and
+ * shades, which takes no block or refill setting), 0 = host-driven loop. */
 pt_status pt_batch_tuning(pt_batch *batch, int32_t path_capacity, int32_t block, int32_t min_active, int32_t tail_paths,
                           int32_t use_graph);
 /* Node fetch width of the batch's walks: 1 = four-wide nodes (default), 0 = the two-wide layout.

@@ -50,3 +50,34 @@ def test_equals_wavefront_after_reset_and_on_a_large_image(scene):
         results.append((r.sums().tobytes(), r.rays_traced()))
     assert results[0] == results[1]
     assert np.frombuffer(results[0][0], np.float32).max() > 0
+
+
+def test_batch_in_one_kernel_equals_its_graph_form_and_lone_renderers():
+    """Uneven jobs (1 to 9 samples, an empty scene, a scene without emitters) past one pixel per resident thread."""
+    a, cam_a = pt.procedural_scene(300, 200, sphere_count=4, segments=24, rings=13, seed=2, glass_fraction=0.5)
+    b, cam_b = pt.cornell_box(180, 150)
+    c, cam_c = pt.procedural_scene(90, 70, sphere_count=2, segments=16, rings=9, seed=7, light_fraction=0.0)
+    scenes = [a, b, c, pt.FlatScene()]
+    jobs = [dict(scene=0, camera=cam_a, width=300, height=200, samples=9, max_depth=9, seed=1),
+            dict(scene=1, camera=cam_b, width=180, height=150, samples=2, max_depth=6, seed=2),
+            dict(scene=2, camera=cam_c, width=90, height=70, samples=1, max_depth=3, seed=3),
+            dict(scene=3, camera=cam_c, width=33, height=5, samples=4, max_depth=2, seed=4),
+            dict(scene=0, camera=cam_a, width=300, height=200, samples=3, max_depth=0, seed=5)]
+    batch = pt.Batch(scenes, jobs)
+    forms = []
+    for capacity in (0, 40000, 0):         # all pixels have a slot; a pool of 40,000 (graph loop); again after it
+        batch.tuning(path_capacity=capacity)
+        for _ in range(2):                 # a second run starts from a fresh state
+            batch.run()
+        ms, rays, done = batch.stats()
+        assert (done > 0).all() and (done <= ms * 1.01 + 0.1).all()
+        forms.append(([batch.sums(k).tobytes() for k in range(len(jobs))], rays))
+    assert forms[0] == forms[1] == forms[2]
+    for k, j in enumerate(jobs):
+        if j["scene"] == 3:
+            assert not np.frombuffer(forms[0][0][k], np.float32).any()
+            continue
+        r = pt.CudaRenderer(scenes[j["scene"]], j["camera"], j["width"], j["height"], j["seed"], max_depth=j["max_depth"])
+        r.set_tail_paths(0)
+        r.add_samples(j["samples"])
+        assert r.sums().tobytes() == forms[0][0][k]
