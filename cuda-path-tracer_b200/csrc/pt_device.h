@@ -49,13 +49,22 @@ private:
 
 class Event {
 public:
-    Event() { PT_CUDA(cudaEventCreate(&e_)); }
+    explicit Event(unsigned flags = cudaEventDefault) { PT_CUDA(cudaEventCreateWithFlags(&e_, flags)); }
     ~Event() { cudaEventDestroy(e_); }
     Event(const Event &) = delete;
     Event &operator=(const Event &) = delete;
     cudaEvent_t get() const { return e_; }
 private:
     cudaEvent_t e_{};
+};
+
+// Held by every handle that copies through the pinned chunk pool (pt_stage.h); the pool is freed with
+// the last of them.
+struct StageUser {
+    StageUser();
+    ~StageUser();
+    StageUser(const StageUser &) = delete;
+    StageUser &operator=(const StageUser &) = delete;
 };
 
 void require_device();
@@ -80,6 +89,7 @@ extern QueryConfig g_query_config;
 
 // The scene handle: everything device-resident that queries and renderers read.
 struct pt_scene {
+    ptb::StageUser stage;
     ptb::DeviceScene view{};
     ptb::DeviceBuffer nodes, nodes4, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, brute_order, small, shade_tris, shade_lights;
     std::vector<pt_light> host_lights;
@@ -89,7 +99,12 @@ struct pt_scene {
     // host-buffer query workspace (reused between calls)
     ptb::DeviceBuffer work_rays[3], work_tmax[3], work_hits[3], work_stats[3];
     cudaStream_t streams[3] = {nullptr, nullptr, nullptr};
-    std::mutex work_mutex;                  // one pt_query_rays call at a time uses the workspace above
+    // the same per worker thread of a query from pageable memory (small chunks)
+    struct HostWorker {
+        ptb::DeviceBuffer rays, tmax, hits, stats;
+        cudaStream_t stream = nullptr;
+    } workers[8];
+    std::mutex work_mutex;                  // one pt_query_rays call at a time uses the workspaces above
     ptb::DeviceBuffer ray_counter;          // per-launch ray counters of the persistent query kernel (a ring)
     std::atomic<unsigned> counter_slot{0};
     cudaMemPool_t order_pool = nullptr;     // stream-ordered scratch of the ray ordering (kept, not released)

@@ -145,8 +145,9 @@ enum { PT_QUERY_CLOSEST = 0, PT_QUERY_ANY = 1 };
 pt_status pt_query_rays_device(const pt_scene *scene, const pt_ray *rays, size_t count, int mode,
                                float tmin, const float *tmax, pt_hit *hits, pt_ray_stats *stats,
                                void *stream);
-/* Host buffers: uploads, traces and downloads in overlapped chunks (2^20 rays each, on three
- * streams; the copies overlap the walk only from pinned host memory); returns when `hits` is
+/* Host buffers: uploads, traces and downloads in overlapped chunks: from pinned memory 2^20 rays each
+ * on three streams; 2^19 rays and more from or to pageable memory through up to eight threads, each
+ * with a pinned 2 MiB chunk of a pool that lives as long as a scene does; returns when `hits` is
  * filled.  Calls on one scene from several host threads take turns (the staging buffers are the
  * scene's). */
 pt_status pt_query_rays(const pt_scene *scene, const pt_ray *rays, size_t count, int mode,
