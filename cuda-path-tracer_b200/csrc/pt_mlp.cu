@@ -77,8 +77,8 @@ __device__ inline void fence_after() { asm volatile("tcgen05.fence::after_thread
 __device__ inline void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ inline void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-__device__ inline void bar_init(uint64_t *bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(bar)) : "memory");
+__device__ inline void bar_init(uint64_t *bar, uint32_t arrivals = 1) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(bar)), "r"(arrivals) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 // bounded wait for the phase with parity `phase` to complete: at most `attempts` try_waits
@@ -103,6 +103,21 @@ __device__ inline void tmem_ld16(uint32_t taddr, float v[16]) {
     wait_ld();
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 32 consecutive FP32 columns
+__device__ inline void tmem_ld32(uint32_t taddr, float v[32]) {
+    uint32_t r[32];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr));
+    wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
 // writes 8 bf16 values (columns 8c..8c+7 of row r) into a core-matrix layout buffer
@@ -143,22 +158,26 @@ struct RowWriter {
     }
 };
 
-// Input encoding of one query (see the file comment); 64 values, zero padded.
+// Input encoding of one query (see the file comment); 64 values, zero padded: all of them
+// (kPart 0), or values 0..31 (1) or 32..63 (2) when two threads share a row.
+template <int kPart = 0>
 __device__ __forceinline__ void encode(const pt_cache_query &q, float3 lo, float3 inv_extent, RowWriter &put) {
     const float p3[3] = {(q.position.x - lo.x) * inv_extent.x, (q.position.y - lo.y) * inv_extent.y,
                          (q.position.z - lo.z) * inv_extent.z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
+        if (kPart == 2 && a < 2) continue;
         float sn, cs;
         sincosf(3.14159265358979f * p3[a], &sn, &cs);
 #pragma unroll
         for (int f = 0; f < 6; f++) {          // frequencies 2^f pi p by the double-angle identities
-            put(sn); put(cs);
+            if (kPart == 0 || (kPart == 1) == (12 * a + 2 * f < 32)) { put(sn); put(cs); }
             float s2 = 2.0f * sn * cs;
             cs = (cs - sn) * (cs + sn);
             sn = s2;
         }
     }
+    if (kPart == 1) return;
     float dx = q.direction.x, dy = q.direction.y, dz = q.direction.z;
     float xx = dx * dx, yy = dy * dy, zz = dz * dz;
     put(0.28209479177387814f);
@@ -207,16 +226,19 @@ __device__ inline void load_weights(unsigned char *w, const unsigned char *g) {
 }
 
 // X (128 x 64, rows = queries) into the core-matrix layout; rows past `count` are zero.
-// `r` is the calling thread's row of the tile.
+// `r` is the calling thread's row of the tile; kPart as encode's.
+template <int kPart = 0>
 __device__ inline void encode_tile(unsigned char *x, const pt_cache_query *q, size_t first, size_t count, float3 lo,
                                    float3 inv_extent, uint32_t r) {
     size_t row = first + r;
+    constexpr int c0 = kPart == 2 ? 4 : 0, c1 = kPart == 1 ? 4 : 8;
     if (row < count) {
         RowWriter put{x, r};
-        encode(q[row], lo, inv_extent, put);
+        put.k = 8 * c0;
+        encode<kPart>(q[row], lo, inv_extent, put);
     } else {
         const float zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int c = 0; c < 8; c++) store8(x, r, c, 64, zero);
+        for (int c = c0; c < c1; c++) store8(x, r, c, 64, zero);
     }
 }
 
@@ -249,20 +271,19 @@ __device__ inline void mma_tn(uint32_t d, const unsigned char *a, const unsigned
     }
 }
 
-// Thread 0 commits the MMAs it issued to the barrier; every thread waits (bounded).  Returns, the
-// same in every thread of the CTA, whether all of them saw the MMAs complete.
+// The issuing threads commit their MMAs to the barrier; every thread waits (bounded) for all of them.
+// Returns whether this thread saw them complete: the threads agree at their next block barrier.
 struct Sync {
     Scratch *h;
     long long attempts;
     uint32_t phase = 0;
     bool pending = false;       // this thread's wait ran out on phase pending_phase
     uint32_t pending_phase = 0;
-    __device__ bool wait_all() {
-        if (threadIdx.x == 0) commit(&h->bar);
-        bool ok = bar_wait(&h->bar, phase, attempts);
+    __device__ bool wait(bool issuer) {
+        if (issuer) commit(&h->bar);
+        const bool ok = bar_wait(&h->bar, phase, attempts);
         if (!ok) { pending = true; pending_phase = phase; }
         phase ^= 1;
-        ok = __syncthreads_and(ok) != 0;
         fence_after();
         return ok;
     }
@@ -376,27 +397,42 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtasPerSm) forward_kernel(con
 }
 
 // ---- training (forward + relative-L2 loss + backward) --------------------------------------
-// TMEM columns: [0,64) forward scratch, [64,80) output, [96,112) dW5, [128,192) dH scratch,
-// [192 + 64 l, 256 + 64 l) dW_l for l = 0..4.
-// smem: header | W | pad | H0..H5 (each + pad) | dZ + pad | dZ5 + pad
-constexpr size_t kTrainSmem = 256 + kWeightBytes + kPad + 6 * (kActBytes + kPad) + (kActBytes + kPad) + (kOutActBytes + kPad);
+// A CTA takes 256 samples at a time: two 128-row MMA tiles in step, sixteen warps, two threads per
+// sample (columns 0..31 and 32..63).  Each of the twelve steps of a pass is a chain of MMA -> commit ->
+// TMEM load -> store -> barrier whose latency, not its work, is the time (one tile of four warps per CTA
+// took 15 us a pass at 5 % of the tensor peak), so a pass carries twice the samples at half the work
+// per thread: the gradients of 2^16 samples 61 -> 39 us.  To hold two tiles in 227 KB, H1 overwrites
+// the encoded inputs, each dZ overwrites the H it masks, and the inputs are encoded again, into the
+// buffer of a dZ already used, while layer 1's MMAs run.
+// TMEM columns: [64 g, 64 g + 64) layer outputs and dH of tile g, [128, 144) dW5,
+// [192 + 64 l, 256 + 64 l) dW_l for l = 0..4 (both tiles accumulate there).
+// smem: header | W | per tile: B1..B5, dZ5 | pad (mma_tn reads past its last operand)
+constexpr int kTrainTiles = 2;
+constexpr int kTrainRows = kTrainTiles * kTile;
+constexpr int kTrainThreads = 2 * kTrainRows;
+constexpr size_t kTrainTileBytes = 5 * kActBytes + kOutActBytes;
+constexpr size_t kTrainSmem = 256 + kWeightBytes + kTrainTiles * kTrainTileBytes + kPad;
+static_assert(kTrainSmem <= 232448, "shared memory of a CTA");
 
-__global__ void __launch_bounds__(kTile, 1) train_kernel(const unsigned char *weights, const pt_cache_query *queries,
-                                                         const float *targets, size_t count, const int32_t *count_dev,
-                                                         float3 lo, float3 hi, float *partial, float *loss_partial, int *status,
-                                                         long long attempts) {
+__global__ void __launch_bounds__(kTrainThreads, 1) train_kernel(const unsigned char *weights, const pt_cache_query *queries,
+                                                                 const float *targets, size_t count, const int32_t *count_dev,
+                                                                 float3 lo, float3 hi, float *partial, float *loss_partial, int *status,
+                                                                 long long attempts) {
     if (count_dev) count = min(count, size_t(max(0, *count_dev)));
     const float grad_scale = count ? 1.0f / float(count * kOut) : 0.0f;   // mean over samples and channels
     extern __shared__ __align__(1024) unsigned char smem[];
     Scratch *h = reinterpret_cast<Scratch *>(smem);
     unsigned char *w = smem + 256;
-    unsigned char *act[6];
-    act[0] = w + kWeightBytes + kPad;
-    for (int i = 1; i < 6; i++) act[i] = act[i - 1] + kActBytes + kPad;
-    unsigned char *dz = act[5] + kActBytes + kPad;
-    unsigned char *dz5 = dz + kActBytes + kPad;
+    const int warp = threadIdx.x >> 5;
+    const int g = (threadIdx.x / kTile) % kTrainTiles, half = threadIdx.x / kTrainRows;   // this thread's tile and column half
+    const uint32_t r = threadIdx.x % kTile;                                               // its row of the tile
+    auto tile = [&](int k) { return w + kWeightBytes + size_t(k) * kTrainTileBytes; };
+    auto buffer = [&](int k, int l) { return tile(k) + size_t(l - 1) * kActBytes; };      // B_l of tile k, l = 1..5
+    auto grad_out = [&](int k) { return tile(k) + 5 * size_t(kActBytes); };               // dZ5 of tile k
     const float3 ie = make_float3(1.0f / fmaxf(hi.x - lo.x, 1e-30f), 1.0f / fmaxf(hi.y - lo.y, 1e-30f), 1.0f / fmaxf(hi.z - lo.z, 1e-30f));
-    if (threadIdx.x == 0) bar_init(&h->bar);
+    // two issuing threads, in warps of different schedulers: the serial issue of up to 24 MMAs is shared
+    const bool issuer0 = threadIdx.x == 0, issuer1 = threadIdx.x == 32;
+    if (issuer0) bar_init(&h->bar, 2);
     tmem_alloc(h, 512);
     load_weights(w, weights);
     fence_async_smem();
@@ -404,109 +440,130 @@ __global__ void __launch_bounds__(kTile, 1) train_kernel(const unsigned char *we
     __syncthreads();
     fence_after();
     const uint32_t tbase = h->tmem;
-    const uint32_t lane_base = tbase + ((uint32_t)(threadIdx.x & ~31u) << 16);
+    const uint32_t lanes = (uint32_t)(r & ~31u) << 16;                     // warp w reads lanes 32 (w % 4) ..
+    const uint32_t mine_col = tbase + lanes + 64u * uint32_t(g) + 32u * uint32_t(half);
     Sync sync{h, attempts};
+    // shared-memory stores and TMEM loads before the next MMAs; whether every thread is still on time
+    auto publish = [&](bool on_time) {
+        fence_async_smem();
+        fence_before();
+        const bool all = __syncthreads_and(on_time) != 0;
+        fence_after();
+        return all;
+    };
+    auto encode_inputs = [&](unsigned char *x, size_t first) {
+        if (half == 0) encode_tile<1>(x, queries, first, count, lo, ie, r);
+        else encode_tile<2>(x, queries, first, count, lo, ie, r);
+    };
     bool ok = true, first = true;
     float loss = 0.0f;
-    const size_t tiles = (count + kTile - 1) / kTile;
+    const size_t tiles = (count + kTrainRows - 1) / kTrainRows;
     for (size_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const size_t row = t * kTile + threadIdx.x;
-        encode_tile(act[0], queries, t * kTile, count, lo, ie, threadIdx.x);
-        fence_async_smem();
-        fence_before();
-        __syncthreads();
-        fence_after();
-        for (int layer = 0; layer < kHidden && ok; layer++) {
-            if (threadIdx.x == 0) mma_kk(tbase, act[layer], 64, w + layer * kMatBytes, 64, 64, 64, false);
-            ok = sync.wait_all();
-            if (!ok) break;
-            for (int c = 0; c < 4; c++) {
-                float v[16];
-                tmem_ld16(lane_base + c * 16, v);
-                store8_relu(act[layer + 1], threadIdx.x, 2 * c, 64, v);
-                store8_relu(act[layer + 1], threadIdx.x, 2 * c + 1, 64, v + 8);
+        const size_t tile_first = t * kTrainRows + size_t(g) * kTile, row = tile_first + r;
+        float target[kOut] = {0, 0, 0};                                    // read now, used five layers later
+        if (half == 0 && row < count)
+            for (int c = 0; c < kOut; c++) target[c] = targets[3 * row + c];
+        if (const size_t ahead = row + size_t(gridDim.x) * kTrainRows; half == 1 && ahead < count)
+            asm volatile("prefetch.global.L2 [%0];" :: "l"(queries + ahead));
+        encode_inputs(buffer(g, 1), tile_first);
+        publish(true);
+        bool done = true;
+        for (int layer = 0; layer < kHidden; layer++) {
+            const unsigned char *wl = w + layer * kMatBytes;
+            if (issuer0) mma_kk(tbase, buffer(0, layer ? layer : 1), 64, wl, 64, 64, 64, false);
+            if (issuer1) mma_kk(tbase + 64, buffer(1, layer ? layer : 1), 64, wl, 64, 64, 64, false);
+            done = sync.wait(issuer0 || issuer1);
+            if (done) {
+                float v[32];
+                tmem_ld32(mine_col, v);
+                for (int c = 0; c < 4; c++) store8_relu(buffer(g, layer + 1), r, uint32_t(4 * half + c), 64, v + 8 * c);
             }
-            fence_async_smem();
-            fence_before();
-            __syncthreads();
-            fence_after();
+            ok = publish(done);
+            if (!ok) break;
         }
         if (!ok) break;
-        if (threadIdx.x == 0) mma_kk(tbase + 64, act[5], 64, w + kHidden * kMatBytes, 64, kOutPad, 64, false);
-        ok = sync.wait_all();
-        if (!ok) break;
-        {
+        if (issuer0) mma_kk(tbase, buffer(0, 5), 64, w + kHidden * kMatBytes, 64, kOutPad, 64, false);
+        if (issuer1) mma_kk(tbase + 64, buffer(1, 5), 64, w + kHidden * kMatBytes, 64, kOutPad, 64, false);
+        done = sync.wait(issuer0 || issuer1);
+        if (done) {
             // relative L2 loss, sum_c (y - t)^2 / (sg(y)^2 + 0.01) with y = exp(z): dL/dz = 2 (y - t) y / (y^2 + 0.01)
-            float v[16], g[16];
-            tmem_ld16(lane_base + 64, v);
-            for (int i = 0; i < 16; i++) g[i] = 0.0f;
-            if (row < count) {
-                for (int c = 0; c < kOut; c++) {
-                    float y = expf(v[c]), target = targets[3 * row + c];
-                    float denom = y * y + 0.01f, diff = y - target;
-                    loss += diff * diff / denom;
-                    g[c] = grad_scale * 2.0f * diff * y / denom;
+            float d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (half == 0) {
+                float v[16];
+                tmem_ld16(mine_col, v);
+                if (row < count) {
+                    for (int c = 0; c < kOut; c++) {
+                        float y = expf(v[c]);
+                        float denom = y * y + 0.01f, diff = y - target[c];
+                        loss += diff * diff / denom;
+                        d[c] = grad_scale * 2.0f * diff * y / denom;
+                    }
                 }
             }
-            store8(dz5, threadIdx.x, 0, kOutPad, g);
-            store8(dz5, threadIdx.x, 1, kOutPad, g + 8);
+            store8(grad_out(g), r, uint32_t(half), kOutPad, d);            // columns 8..15 are padding
         }
-        fence_async_smem();
-        fence_before();
-        __syncthreads();
-        fence_after();
-        // dW5 += H5^T dZ5 ; dH5 = dZ5 W5^T
-        if (threadIdx.x == 0) {
-            mma_tn(tbase + 96, act[5], dz5, kOutPad, kOutPad, !first);
-            mma_kmn(tbase + 128, dz5, kOutPad, w + kHidden * kMatBytes, 64, 64, kOutPad, false);
-        }
-        ok = sync.wait_all();
+        ok = publish(done);
         if (!ok) break;
-        for (int layer = kHidden - 1; layer >= 0 && ok; layer--) {
-            // dZ_layer = dH_{layer+1} * [H_{layer+1} > 0]
-            for (int c = 0; c < 4; c++) {
-                float v[16], a[16];
-                tmem_ld16(lane_base + 128 + c * 16, v);
-                load8(act[layer + 1], threadIdx.x, 2 * c, 64, a);
-                load8(act[layer + 1], threadIdx.x, 2 * c + 1, 64, a + 8);
-                for (int i = 0; i < 16; i++) v[i] = a[i] > 0.0f ? v[i] : 0.0f;
-                store8(dz, threadIdx.x, 2 * c, 64, v);
-                store8(dz, threadIdx.x, 2 * c + 1, 64, v + 8);
+        // dW5 += H5^T dZ5 ; dH5 = dZ5 W5^T
+        if (issuer0)
+            for (int k = 0; k < kTrainTiles; k++) mma_tn(tbase + 128, buffer(k, 5), grad_out(k), kOutPad, kOutPad, !first || k);
+        if (issuer1)
+            for (int k = 0; k < kTrainTiles; k++) mma_kmn(tbase + 64 * k, grad_out(k), kOutPad, w + kHidden * kMatBytes, 64, 64, kOutPad, false);
+        done = sync.wait(issuer0 || issuer1);
+        for (int layer = kHidden - 1; layer >= 0; layer--) {
+            // dZ_layer = dH_{layer+1} * [H_{layer+1} > 0], over H_{layer+1}
+            if (done) {
+                float v[32];
+                tmem_ld32(mine_col, v);
+                for (int c = 0; c < 4; c++) {
+                    float a[8];
+                    load8(buffer(g, layer + 1), r, uint32_t(4 * half + c), 64, a);
+                    for (int i = 0; i < 8; i++) a[i] = a[i] > 0.0f ? v[8 * c + i] : 0.0f;
+                    store8(buffer(g, layer + 1), r, uint32_t(4 * half + c), 64, a);
+                }
             }
-            fence_async_smem();
-            fence_before();
-            __syncthreads();
-            fence_after();
-            if (threadIdx.x == 0) {
-                mma_tn(tbase + 192 + 64 * layer, act[layer], dz, 64, 64, !first);        // dW_layer += H^T dZ
-                if (layer > 0) mma_kmn(tbase + 128, dz, 64, w + layer * kMatBytes, 64, 64, 64, false);   // dH = dZ W^T
-            }
-            ok = sync.wait_all();
+            ok = publish(done);
+            if (!ok) break;
+            if (issuer0)
+                for (int k = 0; k < kTrainTiles; k++)                      // dW_layer += H^T dZ
+                    mma_tn(tbase + 192 + 64 * layer, buffer(k, layer ? layer : 3), buffer(k, layer + 1), 64, 64, !first || k);
+            if (issuer1 && layer > 0)
+                for (int k = 0; k < kTrainTiles; k++)                      // dH = dZ W^T
+                    mma_kmn(tbase + 64 * k, buffer(k, layer + 1), 64, w + layer * kMatBytes, 64, 64, 64, false);
+            if (layer == 1) encode_inputs(buffer(g, 3), tile_first);       // dZ_2's MMAs have completed
+            done = sync.wait(issuer0 || issuer1);
         }
+        if (!ok) break;
+        ok = publish(done);                                                // the next pass overwrites what the last MMAs read
         first = false;
     }
-    // per-CTA partial gradients (rows k of the dW accumulators live in TMEM lanes 0..63)
+    // per-CTA partial gradients (rows k of the dW accumulators live in TMEM lanes 0..63: the first two
+    // warps of each group of four; group j writes columns 16 j ..)
     float *mine = partial + size_t(blockIdx.x) * kMasterFloats;
-    if (ok) {
-        for (int layer = 0; layer < kHidden; layer++) {
-            for (int c = 0; c < 4; c++) {
-                float v[16];
-                tmem_ld16(lane_base + 192 + 64 * layer + c * 16, v);
-                if (threadIdx.x < 64)
-                    for (int i = 0; i < 16; i++) mine[layer * 4096 + threadIdx.x * 64 + c * 16 + i] = first ? 0.0f : v[i];
-            }
-        }
+    if (ok && r < 64) {
+        const int j = warp >> 2;
         float v[16];
-        tmem_ld16(lane_base + 96, v);
-        if (threadIdx.x < 64)
-            for (int i = 0; i < kOut; i++) mine[kHidden * 4096 + threadIdx.x * kOut + i] = first ? 0.0f : v[i];
+        for (int layer = 0; layer < kHidden; layer++) {
+            tmem_ld16(tbase + lanes + 192 + 64 * layer + 16 * j, v);
+            float4 *to = reinterpret_cast<float4 *>(mine + layer * 4096 + r * 64 + 16 * j);
+            for (int i = 0; i < 4; i++)
+                to[i] = first ? make_float4(0, 0, 0, 0) : make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
+        if (j == 0) {
+            tmem_ld16(tbase + lanes + 128, v);
+            for (int i = 0; i < kOut; i++) mine[kHidden * 4096 + r * kOut + i] = first ? 0.0f : v[i];
+        }
     }
     // loss partial
     for (int o = 16; o; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
-    __shared__ float warp_loss[4];
-    if ((threadIdx.x & 31) == 0) warp_loss[threadIdx.x >> 5] = loss;
+    __shared__ float warp_loss[kTrainThreads / 32];
+    if ((threadIdx.x & 31) == 0) warp_loss[warp] = loss;
     __syncthreads();
-    if (threadIdx.x == 0) loss_partial[blockIdx.x] = warp_loss[0] + warp_loss[1] + warp_loss[2] + warp_loss[3];
+    if (threadIdx.x == 0) {
+        float sum = 0.0f;
+        for (int k = 0; k < kTrainRows / 32; k++) sum += warp_loss[k];     // the other half's threads carry none
+        loss_partial[blockIdx.x] = sum;
+    }
     if (!ok && threadIdx.x == 0) atomicExch(status, int(PT_TIMEOUT));
     sync.drain();                                 // no MMA may still write TMEM when it is freed
     fence_before();
@@ -556,8 +613,16 @@ __global__ void __launch_bounds__(32 * kReduceSlices) reduce_step_kernel(const f
     const int i = blockIdx.x * 32 + lane;
     const size_t n = count_dev ? min(count, size_t(max(0, *count_dev))) : count;
     float s = 0.0f;
-    if (i < kMasterFloats)
-        for (int c = slice; c < ctas; c += kReduceSlices) s += partial[size_t(c) * kMasterFloats + i];
+    if (i < kMasterFloats) {
+        // the additions are in order, the loads of eight rows in flight at a time
+        for (int c = slice; c < ctas; c += 8 * kReduceSlices) {
+            float x[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) x[k] = c + k * kReduceSlices < ctas ? __ldg(partial + size_t(c + k * kReduceSlices) * kMasterFloats + i) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) if (c + k * kReduceSlices < ctas) s += x[k];
+        }
+    }
     sums[slice][lane] = s;
     __syncthreads();
     if (slice == 0 && i < kMasterFloats) {
@@ -589,12 +654,15 @@ __global__ void __launch_bounds__(32 * kReduceSlices) reduce_step_kernel(const f
         last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
+    if (last && threadIdx.x < 32) {     // fixed order again: lane k sums partials k, k + 32, ..., then a shuffle tree
         float l = 0.0f;
-        for (int c = 0; c < ctas; c++) l += loss_partial[c];
-        loss[0] = n ? l / float(n * kOut) : 0.0f;
-        if (n && advance) { step[0] += 1; step[1] += 1; }
-        *done = 0;
+        for (int c = threadIdx.x; c < ctas; c += 32) l += loss_partial[c];
+        for (int o = 16; o; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+        if (threadIdx.x == 0) {
+            loss[0] = n ? l / float(n * kOut) : 0.0f;
+            if (n && advance) { step[0] += 1; step[1] += 1; }
+            *done = 0;
+        }
     }
 }
 
@@ -644,9 +712,9 @@ float3 hi3(const pt_cache *c) { return make_float3(c->hi[0], c->hi[1], c->hi[2])
 // the same reduction launch; no host synchronisation
 void gradients(pt_cache *c, const pt_cache_query *q, const float *targets, size_t count, const int32_t *count_dev, bool train,
                cudaStream_t st) {
-    size_t tiles = (count + kTile - 1) / kTile;
+    size_t tiles = (count + kTrainRows - 1) / kTrainRows;
     int grid = count_dev ? c->ctas : int(std::min<size_t>(tiles ? tiles : 1, size_t(c->ctas)));
-    train_kernel<<<grid, kTile, kTrainSmem, st>>>(c->weights.get<unsigned char>(), q, targets, count, count_dev, lo3(c), hi3(c),
+    train_kernel<<<grid, kTrainThreads, kTrainSmem, st>>>(c->weights.get<unsigned char>(), q, targets, count, count_dev, lo3(c), hi3(c),
                                                    c->partial.get<float>(), c->loss_partial.get<float>(), c->status.get<int>(),
                                                    c->attempts);
     PT_CUDA(cudaGetLastError());
