@@ -122,6 +122,7 @@ struct DeviceScene {
     int32_t root_leaf;              // flat root is itself a leaf (no branch above it)
     const SmallLeaf *small;         // every leaf in slot order, when there are at most kSmallLeaves
     int32_t small_count;            // 0: more leaves than that (or none)
+    float small_pad;                // how much query_small_kernel widens their boxes
 };
 
 // Tie rule for exact-distance hits: the lowest (type, id) (the parity rule of the query API), the leaf the

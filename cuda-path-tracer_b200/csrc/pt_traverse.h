@@ -319,6 +319,16 @@ namespace ptb {
 // at most one entry per level, so a validated tree (depth <= 64) never needs more than 63.
 constexpr int kSharedStack = 32;
 
+// First of the work items the warp's `idle` lanes take: from the shared counter, or without one the
+// warp's own first item (then there are no more).
+__device__ __forceinline__ unsigned long long take_items(unsigned long long *next, unsigned idle, size_t warp_first) {
+    if (!next) return warp_first;
+    const int leader = __ffs(idle) - 1;
+    unsigned long long base = 0;
+    if (int(threadIdx.x & 31) == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
+    return __shfl_sync(0xffffffffu, base, leader);
+}
+
 // Result of a finished walk, handed to the consumer.
 struct WalkResult { float t, u, v; int32_t slot; uint32_t boxes, prims; int error; };
 
@@ -354,11 +364,8 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (idle && !pool_empty) {
-            int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if ((int)lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + __popc(idle) >= count) pool_empty = true;
+            const unsigned long long base = take_items(next, idle, warp_first);
+            if (!next || base + __popc(idle) >= count) pool_empty = true;
             if (!busy) {
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < count) {
@@ -696,11 +703,8 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (idle && !pool_empty) {
-            int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if ((int)lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + __popc(idle) >= count) pool_empty = true;
+            const unsigned long long base = take_items(next, idle, warp_first);
+            if (!next || base + __popc(idle) >= count) pool_empty = true;
             if (!busy) {
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < count) {
@@ -813,11 +817,8 @@ __device__ inline void persistent_walk4_spec(const DeviceScene &s, size_t count,
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (idle && !pool_empty) {
-            int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if ((int)lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base + __popc(idle) >= count) pool_empty = true;
+            const unsigned long long base = take_items(next, idle, warp_first);
+            if (!next || base + __popc(idle) >= count) pool_empty = true;
             if (!busy) {
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < count) {

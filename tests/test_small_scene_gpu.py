@@ -62,3 +62,71 @@ def test_parallel_and_degenerate_camera_rays():
         r.add_samples(4)
     assert a.sums().tobytes() == b.sums().tobytes() and a.rays_traced() == b.rays_traced()
     assert Oracle().validate(scene)
+
+
+def flat_boxes(scene: pt.FlatScene) -> pt.FlatScene:
+    """The same tree with every box shrunk to its primitives' bounds (flat for axis-aligned triangles)."""
+    s = scene.copy()
+    lo, hi = np.zeros((len(s.nodes), 3), np.float32), np.zeros((len(s.nodes), 3), np.float32)
+
+    def fit(k):
+        n = s.nodes[k]
+        if n["type"] == 0:
+            a, b = fit(int(n["left"])), fit(int(n["right"]))
+            lo[k], hi[k] = np.minimum(a[0], b[0]), np.maximum(a[1], b[1])
+        elif n["type"] == 1:
+            t = s.triangles[n["primitive"]]
+            v = np.stack([t["v0"], t["v1"], t["v2"]])
+            lo[k], hi[k] = v.min(axis=0), v.max(axis=0)
+        else:
+            p = s.spheres[n["primitive"]]
+            r = np.nextafter(p["radius"], np.float32(np.inf)) * np.float32(1.000001)
+            lo[k], hi[k] = p["center"] - r, p["center"] + r
+        return lo[k], hi[k]
+
+    fit(s.root)
+    s.nodes["minimum"], s.nodes["maximum"] = lo, hi
+    return s
+
+
+@pytest.mark.parametrize("primitives", [1, 2, 3, 31, 32, 33])
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("count", [1, 31, 64, 1000, 200_001])
+def test_query_equals_general_walk_and_brute_force(primitives, flat, count):
+    """Random and axis-parallel rays; the single-loop walk and the brute-force scan never use the shared-memory form.
+    200,001 rays are more than the resident grid of either kernel holds at once."""
+    import torch
+    scene = box_scene(primitives)
+    scene.triangles["v1"][0::2, 1] = scene.triangles["v0"][0::2, 1]      # every other triangle axis-aligned
+    scene.triangles["v2"][0::2, 1] = scene.triangles["v0"][0::2, 1]
+    scene = scene.build_bvh()
+    if flat:
+        scene = flat_boxes(scene)
+    assert Oracle().validate(scene)
+    g = np.random.default_rng(count)
+    rays = np.zeros(count, pt.RAY)
+    rays["origin"] = g.uniform(-2, 2, (count, 3))
+    rays["direction"] = g.normal(size=(count, 3))
+    rays["direction"][::5, 0] = 0
+    rays["direction"][::7, 2] = 0
+    rays["direction"][::35, 1] = 0                                       # some have no direction at all
+    d = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
+    tmax = torch.from_numpy(g.uniform(0.1, 5, count).astype(np.float32)).cuda()
+    dev = pt.Scene(scene)
+
+    def query(mode, t, brute=False):
+        out = torch.full((count * 16,), 255, dtype=torch.uint8, device="cuda")
+        dev.query_device(d, count, out, mode=mode, tmax=t, brute=brute)
+        torch.cuda.synchronize()
+        return out.cpu().numpy().view(pt.HIT)
+
+    for t in (None, tmax):
+        got, brute = query(pt.QUERY_CLOSEST, t), query(pt.QUERY_CLOSEST, t, True)
+        blocked = query(pt.QUERY_ANY, t)["primitive_type"] != 0
+        pt.query_walk(0)
+        try:
+            walk = query(pt.QUERY_CLOSEST, t)
+        finally:
+            pt.query_walk(1)
+        assert got.tobytes() == walk.tobytes() == brute.tobytes()
+        assert (blocked == (got["primitive_type"] != 0)).all()
