@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kQueryBlock) query_kernel(DeviceScene s, const
 // Persistent form: a fixed grid of warps; each warp takes rays from a global counter and,
 // between traversal steps, hands a new ray to every lane whose ray has ended once fewer than
 // `min_active` lanes are still busy.  next_ray must be zero at launch.
-// With next_ray null every warp walks its own 32 rays and takes no more.
+// kWalk 3 is the phased four-wide walk in which every warp takes its own `min_active` rays and no more.
 // `order` (may be null) lists the rays in the order they are taken: the k-th ray taken is
 // rays[order[k]], and its answer goes to hits[order[k]].
 template <bool kAny, bool kStats, int kWalk>
@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(kQueryBlock, 8) query_persistent_kernel(Device
         reinterpret_cast<int4 *>(hits)[i] = make_int4(__float_as_int(hit ? w.t : 0.0f), id, type, w.error);
         if (kStats) { stats[i].boxes = w.boxes; stats[i].primitives = w.prims; }
     };
-    if (kWalk == 2) persistent_walk4_spec<kAny>(s, count, next_ray, min_active, tie, get, done);
+    if (kWalk == 3) persistent_walk4_spec<kAny, false, true>(s, count, next_ray, min_active, tie, get, done);
+    else if (kWalk == 2) persistent_walk4_spec<kAny>(s, count, next_ray, min_active, tie, get, done);
     else if (kWalk == 1) persistent_walk4<kAny>(s, count, next_ray, min_active, tie, get, done);
     else persistent_walk<kAny>(s, count, next_ray, min_active, tie, get, done);
 }
@@ -328,7 +329,7 @@ void launch_query(const pt_scene *sc, const pt_ray *rays, size_t count, int mode
         };
         if (s.small_count && wide && g_query_config.speculative && !stats) {
             auto fn = any ? query_small_kernel<true> : query_small_kernel<false>;
-            const int bps = blocks_per_sm(sc->device, 12 + any, (const void *)fn, 0);
+            const int bps = blocks_per_sm(sc->device, 16 + any, (const void *)fn, 0);
             const unsigned grid = unsigned(std::min<size_t>(grid_for(count, kQueryBlock), size_t(device_sm_count()) * size_t(bps > 0 ? bps : 1)));
             event(0);
             fn<<<grid, kQueryBlock, 0, stream>>>(s, rays, count, tmin, tmax, hits, tie);
@@ -338,13 +339,17 @@ void launch_query(const pt_scene *sc, const pt_ray *rays, size_t count, int mode
         }
         using Fn = void (*)(DeviceScene, const pt_ray *, size_t, float, const float *, pt_hit *, pt_ray_stats *, int,
                             unsigned long long *, int, const uint32_t *);
-        static const Fn table[12] = {
+        static const Fn table[16] = {
             query_persistent_kernel<false, false, 0>, query_persistent_kernel<false, false, 1>, query_persistent_kernel<false, false, 2>,
+            query_persistent_kernel<false, false, 3>,
             query_persistent_kernel<false, true, 0>, query_persistent_kernel<false, true, 1>, query_persistent_kernel<false, true, 2>,
+            query_persistent_kernel<false, true, 3>,
             query_persistent_kernel<true, false, 0>, query_persistent_kernel<true, false, 1>, query_persistent_kernel<true, false, 2>,
-            query_persistent_kernel<true, true, 0>, query_persistent_kernel<true, true, 1>, query_persistent_kernel<true, true, 2>};
-        int walk = wide ? (g_query_config.speculative ? 2 : 1) : 0;
-        int k = (any ? 6 : 0) + (stats ? 3 : 0) + walk;
+            query_persistent_kernel<true, false, 3>,
+            query_persistent_kernel<true, true, 0>, query_persistent_kernel<true, true, 1>, query_persistent_kernel<true, true, 2>,
+            query_persistent_kernel<true, true, 3>};
+        const int walk = wide ? (g_query_config.speculative ? 2 : 1) : 0;
+        int k = (any ? 8 : 0) + (stats ? 4 : 0) + walk;
         Fn fn = table[k];
         const size_t smem = wide ? size_t(kSharedStack4) * kQueryBlock * sizeof(int2) : size_t(kSharedStack) * kQueryBlock * sizeof(int32_t);
         const int occupancy = blocks_per_sm(sc->device, k, (const void *)fn, smem);
@@ -353,9 +358,20 @@ void launch_query(const pt_scene *sc, const pt_ray *rays, size_t count, int mode
         size_t want = (count + kQueryBlock - 1) / kQueryBlock;
         const size_t resident = size_t(device_sm_count()) * size_t(bps > 0 ? bps : 1);
         unsigned grid = unsigned(std::min<size_t>(want, resident));
-        // a batch that the grid holds at once needs no counter: every warp takes its own 32 rays
         unsigned long long *counter = nullptr;
-        if (want > resident) {
+        int refill = g_query_config.min_active;
+        if (want <= resident && walk == 2) {
+            // a batch that the grid holds at once needs no counter: every warp takes its own rays.  A few rays a
+            // warp while they leave warps idle: lanes that share a warp wait for each other's steps (random rays
+            // on 1M triangles, 64 rays 30.7 us with 32 a warp, 25.6 with 8, 22.2 with 4; 1000 rays on 10,000
+            // triangles 23.6, 18.5, 18.4), but coherent ones share their node fetches (10,000 camera rays 16.8,
+            // 16.9, 17.7), and from one ray for every second lane on a full warp is the faster (60,000
+            // random rays 75 us, 84 with 13 a warp).
+            const size_t warps = resident * (kQueryBlock / 32);
+            refill = count <= warps ? 4 : count <= 4 * warps ? 8 : 32;
+            grid = grid_for((count + size_t(refill) - 1) / size_t(refill) * 32, kQueryBlock);
+            fn = table[k + 1];
+        } else {
             counter = m->ray_counter.get<unsigned long long>() + (m->counter_slot.fetch_add(1) % kRayCounters);
             PT_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream));
         }
@@ -367,8 +383,7 @@ void launch_query(const pt_scene *sc, const pt_ray *rays, size_t count, int mode
             if (capture == cudaStreamCaptureStatusNone) order = order_rays(sc, rays, count, stream, scratch);   // not inside a graph capture
         }
         event(0);
-        fn<<<grid, kQueryBlock, smem, stream>>>(s, rays, count, tmin, tmax, hits, stats, tie, counter, g_query_config.min_active,
-                                                 order);
+        fn<<<grid, kQueryBlock, smem, stream>>>(s, rays, count, tmin, tmax, hits, stats, tie, counter, refill, order);
         PT_CUDA(cudaGetLastError());
         event(1);
         if (scratch) PT_CUDA(cudaFreeAsync(scratch, stream));
@@ -820,11 +835,12 @@ pt_status pt_query_rays_static(const pt_scene *scene, const pt_ray *rays, size_t
             query_persistent_kernel<true, false, 0>, query_persistent_kernel<true, false, 1>, query_persistent_kernel<true, false, 2>,
             query_persistent_kernel<true, true, 0>, query_persistent_kernel<true, true, 1>, query_persistent_kernel<true, true, 2>};
         const int k = (any ? 6 : 0) + (stats ? 3 : 0) + walk;
+        const int key = (any ? 8 : 0) + (stats ? 4 : 0) + walk;   // launch_query's key of the same kernel
         Fn fn = table[k];
         const size_t smem = wide ? size_t(kSharedStack4) * kQueryBlock * sizeof(int2) : size_t(kSharedStack) * kQueryBlock * sizeof(int32_t);
         int dev = 0;
         PT_CUDA(cudaGetDevice(&dev));
-        const int per_sm = blocks_per_sm(dev, k, (const void *)fn, smem);
+        const int per_sm = blocks_per_sm(dev, key, (const void *)fn, smem);
         size_t want = (count + kQueryBlock - 1) / kQueryBlock;
         unsigned grid = unsigned(std::min<size_t>(want, size_t(device_sm_count()) * size_t(per_sm > 0 ? per_sm : 1)));
         fn<<<grid, kQueryBlock, smem, st>>>(s, d_rays, count, tmin, d_tmax, d_hits, d_stats, kTieLowestId, counter,

@@ -319,16 +319,6 @@ namespace ptb {
 // at most one entry per level, so a validated tree (depth <= 64) never needs more than 63.
 constexpr int kSharedStack = 32;
 
-// First of the work items the warp's `idle` lanes take: from the shared counter, or without one the
-// warp's own first item (then there are no more).
-__device__ __forceinline__ unsigned long long take_items(unsigned long long *next, unsigned idle, size_t warp_first) {
-    if (!next) return warp_first;
-    const int leader = __ffs(idle) - 1;
-    unsigned long long base = 0;
-    if (int(threadIdx.x & 31) == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
-    return __shfl_sync(0xffffffffu, base, leader);
-}
-
 // Result of a finished walk, handed to the consumer.
 struct WalkResult { float t, u, v; int32_t slot; uint32_t boxes, prims; int error; };
 
@@ -364,8 +354,11 @@ __device__ inline void persistent_walk(const DeviceScene &s, size_t count, unsig
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (idle && !pool_empty) {
-            const unsigned long long base = take_items(next, idle, warp_first);
-            if (!next || base + __popc(idle) >= count) pool_empty = true;
+            int leader = __ffs(idle) - 1;
+            unsigned long long base = 0;
+            if ((int)lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (base + __popc(idle) >= count) pool_empty = true;
             if (!busy) {
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < count) {
@@ -703,8 +696,11 @@ __device__ inline void persistent_walk4(const DeviceScene &s, size_t count, unsi
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (idle && !pool_empty) {
-            const unsigned long long base = take_items(next, idle, warp_first);
-            if (!next || base + __popc(idle) >= count) pool_empty = true;
+            int leader = __ffs(idle) - 1;
+            unsigned long long base = 0;
+            if ((int)lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (base + __popc(idle) >= count) pool_empty = true;
             if (!busy) {
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < count) {
@@ -783,11 +779,12 @@ namespace ptb {
 // persistent_walk4 (a leaf tested after a nearer hit was found only costs time: the triangle
 // tests take the current closest distance as their limit).
 // With kRoot, get() also returns the walk's root node (several trees in one node array; < 0 for
-// an empty tree).
-template <bool kAny, bool kRoot = false, class Get, class Done>
+// an empty tree).  With kOwn every warp takes `min_active` items of its own and no more (`next` unused).
+template <bool kAny, bool kRoot = false, bool kOwn = false, class Get, class Done>
 __device__ inline void persistent_walk4_spec(const DeviceScene &s, size_t count, unsigned long long *next, int min_active,
                                              int tie, Get get, Done done) {
-    const size_t warp_first = (size_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u));
+    const size_t warp_first = kOwn ? (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * size_t(min_active)
+                                   : (size_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31u));
     if (warp_first >= count) return;
     extern __shared__ int32_t shared_stack[];
     int2 *my_stack = reinterpret_cast<int2 *>(shared_stack) + threadIdx.x;
@@ -817,11 +814,19 @@ __device__ inline void persistent_walk4_spec(const DeviceScene &s, size_t count,
     for (;;) {
         unsigned idle = __ballot_sync(0xffffffffu, !busy);
         if (idle && !pool_empty) {
-            const unsigned long long base = take_items(next, idle, warp_first);
-            if (!next || base + __popc(idle) >= count) pool_empty = true;
+            unsigned long long base = warp_first;
+            if constexpr (kOwn) {
+                pool_empty = true;
+            } else {
+                int leader = __ffs(idle) - 1;
+                base = 0;
+                if ((int)lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
+                base = __shfl_sync(0xffffffffu, base, leader);
+                if (base + __popc(idle) >= count) pool_empty = true;
+            }
             if (!busy) {
                 size_t mine = base + __popc(idle & ((1u << lane) - 1u));
-                if (mine < count) {
+                if (mine < count && (!kOwn || (int)lane < min_active)) {
                     index = mine;
                     int32_t root = 0;
                     if constexpr (kRoot) get(index, r, tmin, limit, root);

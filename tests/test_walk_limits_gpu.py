@@ -54,3 +54,33 @@ def test_ties_and_signed_distances_match_oracle(wide, speculative, persistent, c
         pt.query_layout(1)
         pt.query_walk(1)
         pt.query_tuning(1, 24, 0)
+
+
+@pytest.mark.parametrize("mode", [pt.QUERY_CLOSEST, pt.QUERY_ANY])
+def test_batches_of_every_size_class(mode):
+    """Around the counts where a warp takes 4, 8 or 32 rays of its own and where the shared counter starts, for
+    every walk form: each prefix of a batch has the prefix of its answers."""
+    import torch
+    scene, cam = pt.procedural_scene(512, 400, sphere_count=4, segments=24, rings=13, seed=2)
+    dev = pt.Scene(scene)
+    total = 204_800
+    rays = torch.empty((total, 7), dtype=torch.float32, device="cuda")
+    pt.camera_rays_device(cam, 512, 400, 3, 0, total, rays)
+
+    def query(n):
+        out = torch.full((n, 4), -7, dtype=torch.int32, device="cuda")
+        dev.query_device(rays, n, out, mode=mode)
+        torch.cuda.synchronize()
+        return (out[:, 2] != 0) if mode == pt.QUERY_ANY else out
+
+    try:
+        for wide, speculative in ((1, 1), (1, 0), (0, 1)):
+            pt.query_layout(wide)
+            pt.query_walk(speculative)
+            whole = query(total)                       # more rays than the grid holds: the shared counter
+            assert (whole != 0).any()
+            for n in (1, 3, 4, 5, 31, 33, 127, 129, 4735, 4736, 4737, 18_943, 18_945, 75_777, 151_551, 151_552, 151_553):
+                assert torch.equal(query(n), whole[:n]), (wide, speculative, n)
+    finally:
+        pt.query_layout(1)
+        pt.query_walk(1)
