@@ -29,3 +29,27 @@ def test_gradients_match_oracle_at_tile_edges(n):
         assert cos > 0.999 and rel < 2e-2, (l, cos, rel)
     again = cache.gradients(dq, dt, n)              # deterministic
     assert again[0] == loss and np.array_equal(again[1], g)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1024, 1025, 148 * 8 * 128, 148 * 8 * 128 * 2 + 77])
+def test_forward_at_tile_edges_and_unaligned_queries(n):
+    """Whole tiles come by bulk copy, partial tiles and queries off a 16-byte boundary by plain loads: the same bits
+    wherever a query lies, nothing written past the last one, and the oracle's values."""
+    import torch
+    cache = pt.RadianceCache(LO, HI, seed=9)
+    q = queries(n, n)
+    want = None
+    for shift in (0, 1, 4):                        # 52-byte records: shifts of 0, 52 and 208 bytes
+        raw = torch.zeros((n + 8) * 52, dtype=torch.uint8, device="cuda")
+        raw[shift * 52:(shift + n) * 52] = to_dev(q)
+        out = torch.full((n * 3 + 64,), -7.0, dtype=torch.float32, device="cuda")
+        cache.query(raw[shift * 52:], n, out)
+        cache.sync()
+        got = out.cpu().numpy()
+        assert (got[3 * n:] == -7.0).all()
+        if want is None:
+            want = got
+            m = min(n, 4096)
+            ref = mo.forward(cache.weights(), mo.encode(q[:m], LO, HI))
+            assert (np.abs(got[:3 * m].reshape(m, 3) - ref) / np.maximum(np.abs(ref), 1e-6)).max() < 2e-2
+        assert got.tobytes() == want.tobytes()
