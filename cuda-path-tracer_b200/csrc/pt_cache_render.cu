@@ -34,7 +34,7 @@
 #include "pt_api_common.h"
 #include "pt_cache_internal.h"
 #include "pt_device.h"
-#include "pt_wavefront.h"
+#include "pt_paths.h"
 
 using namespace ptb;
 
@@ -120,6 +120,10 @@ struct Buffers {
     int32_t *pixel_query_count;
     TrainVertex *vertices;
     TrainEnd *ends;
+    CachePath *lane_paths;              // per lane of frame_kernel
+    CacheShadow *lane_shadows;
+    int32_t *claims;                    // per pixel: samples drawn and not yet run (frame_kernel; zero between frames)
+    int32_t *done;                      // per pixel: samples of this frame run by frame_kernel
     pt_cache_query *samples;            // steps x bucket_capacity
     float *targets;                     // steps x bucket_capacity x 3
 };
@@ -353,16 +357,17 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
 // returns whether the path goes on.
 __device__ inline bool retire(const Params &p, const Buffers &b, int32_t i, CachePath &s, Pcg &rng, const ShadeOut &o, int32_t q) {
     if (p.accumulate) {
+        // (read past the L1: a pixel's samples may run on different SMs, pt_paths.h)
         float *sum = b.sums + 3 * size_t(i);
-        sum[0] += s.rr; sum[1] += s.rg; sum[2] += s.rb;
+        __stcg(sum, __ldcg(sum) + s.rr); __stcg(sum + 1, __ldcg(sum + 1) + s.rg); __stcg(sum + 2, __ldcg(sum + 2) + s.rb);
     }
     if (o.query) {
         b.queries[q] = o.q;
         b.aux[q] = o.aux;
         if (p.accumulate) {
-            int32_t j = b.pixel_query_count[i];
+            int32_t j = __ldcg(&b.pixel_query_count[i]);
             b.pixel_queries[size_t(i) * p.spf + j] = q;
-            b.pixel_query_count[i] = j + 1;
+            __stcg(&b.pixel_query_count[i], j + 1);
         }
     }
     if (s.train >= 0) {
@@ -495,6 +500,7 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
                 i = b.queue[parity][k];
                 s = b.paths[i];
                 rng = b.rng[i];
+                if (s.samples_left < 0) { s.samples_left = b.claims[i]; b.claims[i] = 0; }   // from frame_kernel
                 live = true;
             } else {
                 drained = true;
@@ -549,6 +555,87 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
     if (!odd && i >= 0) { b.paths[i] = s; b.rng[i] = rng; }
     for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(full, rays, o);
     if (lane == 0 && rays) atomicAdd(&b.totals[0], rays);
+}
+
+// A whole frame's paths in one kernel (four-wide tree): pt_paths.h's loop over the pixels, a sample at a
+// time; a training pixel trains on its first sample.  What a sample reads of the pixel's earlier ones
+// (stream, sum, query count, samples run) goes past the L1.  The last paths go to finish_pair_kernel.
+struct FrameOps {
+    const DeviceScene &scene;
+    const Params &p;
+    const Buffers &b;
+    uint32_t pixels;
+    uint32_t lane;              // index of the lane's records
+    int32_t i;                  // the pixel
+    __device__ void first_ray() {
+        int32_t train = -1;
+        if (!__ldcg(&b.done[i])) {
+            __stcg(&b.pixel_query_count[i], 0);
+            if (p.train_threshold && pixel_hash(p.seed, *b.frame, i) < p.train_threshold) {
+                train = atomicAdd(&b.counters[4], 1);
+                if (train >= p.train_capacity) train = -1;
+            }
+        }
+        const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2 *>(&b.rng[i]));
+        Pcg rng;
+        rng.state = w.x; rng.increment = w.y;
+        CachePath s;
+        camera_sample(p, i, rng, train, 1, s);
+        b.lane_paths[lane] = s;
+        b.rng[i] = rng;
+    }
+    __device__ bool claim(unsigned long long item, int32_t &root) {
+        i = (item >> 32) ? int32_t(item % pixels) : int32_t(uint32_t(item) % pixels);
+        if (atomicAdd(&b.claims[i], 1) != 0) return false;   // the lane running this pixel will see it
+        __threadfence();
+        root = 0;
+        first_ray();
+        return true;
+    }
+    __device__ bool again() {
+        __stcg(&b.done[i], __ldcg(&b.done[i]) + 1);
+        __threadfence();                                     // what the next sample reads, before the claim goes
+        if (atomicSub(&b.claims[i], 1) == 1) return false;
+        first_ray();
+        return true;
+    }
+    __device__ void shade(const PathHit &h, NextWalk &n) {
+        CachePath s = b.lane_paths[lane];
+        Pcg rng = b.rng[i];
+        ShadeOut o;
+        nrc::shade(scene, p, b, i, s, h, rng, o);
+        if (o.finished) {
+            const int32_t q = o.query ? atomicAdd(&b.counters[3], 1) : -1;
+            retire(p, b, i, s, rng, o, q);                   // one sample left: starts no other
+        } else {
+            b.lane_paths[lane] = s;
+        }
+        b.rng[i] = rng;
+        if (o.shadow) b.lane_shadows[lane] = o.sr;
+        n.live = o.live; n.shadow = o.shadow;
+    }
+    __device__ void ray(bool shadow, pt_ray &r, float &tmax) { lane_ray(b.lane_paths[lane], b.lane_shadows[lane], shadow, r, tmax); }
+    __device__ void unblocked() {
+        CachePath &s = b.lane_paths[lane];
+        const CacheShadow &sr = b.lane_shadows[lane];
+        s.rr += sr.cr; s.rg += sr.cg; s.rb += sr.cb;
+        if (sr.suffix) { s.sr += sr.sr; s.sg += sr.sg; s.sb += sr.sb; }
+    }
+    // finish_pair_kernel's queue; it reads the pixel's claims once this kernel has ended (samples_left < 0)
+    __device__ void hand_over() {
+        CachePath s = b.lane_paths[lane];
+        s.samples_left = -1;
+        b.paths[i] = s;
+        b.queue[0][atomicAdd(&b.counters[0], 1)] = i;
+    }
+};
+
+__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) frame_kernel(DeviceScene scene, Params p, Buffers b, int32_t pixels) {
+    FrameOps ops{scene, p, b, uint32_t(pixels), blockIdx.x * blockDim.x + threadIdx.x, 0};
+    unsigned long long rays = 0;
+    persistent_paths4(scene, ops, (unsigned long long)pixels * (unsigned long long)p.spf, &b.fetch[0], true, kTieLastLeaf, rays, b.error);
+    for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(0xffffffffu, rays, o);
+    if (lane_id() == 0 && rays) atomicAdd(&b.totals[0], rays);
 }
 
 __global__ void __launch_bounds__(256, 4) shadow_kernel(DeviceScene scene, Params p, Buffers b, int parity, int min_active) {
@@ -662,9 +749,10 @@ struct pt_cached_renderer {
     int frames = 0;
     float milliseconds = 0;
     int block = 256;
-    int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0;
+    int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0, grid_frame = 0;
+    bool whole = false;                 // frames that render every pixel run as one frame_kernel
     DeviceBuffer paths, hits, shadows, queue0, queue1, shadow_queue, counters, fetch, totals, error, sums, rng, frame;
-    DeviceBuffer queries, aux, pred, pixel_queries, pixel_query_count, vertices, ends, samples, targets;
+    DeviceBuffer queries, aux, pred, pixel_queries, pixel_query_count, vertices, ends, samples, targets, lane_paths, lane_shadows, claims, done;
     Buffers buf{};
     cudaStream_t stream = nullptr, body_stream = nullptr, shadow_stream = nullptr;
     Event shaded[2], shadowed[2];
@@ -699,6 +787,13 @@ struct pt_cached_renderer {
         PT_CUDA(cudaMemsetAsync(buf.counters, 0, kCounters * sizeof(int32_t), st));
         PT_CUDA(cudaMemsetAsync(buf.fetch, 0, 4 * sizeof(unsigned long long), st));
         PT_CUDA(cudaMemsetAsync(buf.pairs, 0, sizeof(unsigned long long), st));
+        if (whole && p.accumulate) {
+            const size_t smem = size_t(kSharedStack4) * sizeof(int2) * kPathsBlock;
+            PT_CUDA(cudaMemsetAsync(buf.done, 0, size_t(pixels) * sizeof(int32_t), st));
+            frame_kernel<<<grid_frame, kPathsBlock, smem, st>>>(scene->view, p, buf, pixels);
+            PT_CUDA(cudaGetLastError());
+            return;
+        }
         start_kernel<<<(pixels + 255) / 256, 256, 0, st>>>(p, buf, pixels);
         PT_CUDA(cudaGetLastError());
     }
@@ -747,7 +842,7 @@ struct pt_cached_renderer {
         cudaStream_t st = stream;
         prologue(p, st);
         const unsigned long long bound = max_pairs(p);
-        for (unsigned long long pair = 0;; pair++) {
+        for (unsigned long long pair = 0; !(whole && accumulate); pair++) {
             iteration_pair(p, st);
             PT_CUDA(cudaMemcpyAsync(live_host, &buf.counters[0], sizeof(int32_t), cudaMemcpyDeviceToHost, st));
             PT_CUDA(cudaStreamSynchronize(st));
@@ -763,6 +858,7 @@ struct pt_cached_renderer {
         PT_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
             prologue(p, stream);
+            if (!(whole && accumulate)) {
             cudaStreamCaptureStatus status;
             cudaGraph_t g = nullptr;
             const cudaGraphNode_t *deps = nullptr;
@@ -784,6 +880,7 @@ struct pt_cached_renderer {
             PT_CUDA(cudaGetLastError());
             PT_CUDA(cudaStreamEndCapture(body_stream, &body));
             PT_CUDA(cudaStreamUpdateCaptureDependencies(stream, &loop, 1, cudaStreamSetCaptureDependencies));
+            }
             epilogue(p, stream);
         } catch (...) {
             cudaGraph_t g = nullptr;
@@ -942,6 +1039,22 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
             r->grid_finish = occupancy_grid((const void *)finish_kernel, r->block, 0);
             r->grid_finish_pair = occupancy_grid((const void *)finish_pair_kernel, r->block, 0);
             r->grid_small = device_sm_count() * 4;
+            r->grid_frame = occupancy_grid((const void *)frame_kernel, kPathsBlock, size_t(kSharedStack4) * sizeof(int2) * kPathsBlock);
+            // Frames as one kernel, unless a tail length asks for the wavefront: from one pixel per resident lane (or with
+            // one sample) to twenty, and to twenty-eight when the bounces of a frame are many.  Wavefront and this, ms a
+            // frame (1M triangles, bounce limit 12): 480x300 one sample 0.89 and 0.69, four 3.0 and 2.2; 960x600 4.8
+            // and 3.0; 1920x1080 one 2.1 and 2.3, two 4.07 and 3.94, four 7.8 and 7.25, four of limit 4 6.5 and 6.6;
+            // 2560x1440 11.0 and 12.2; 200x120 on 65,000 triangles two samples 0.26 and 0.30.
+            const int64_t lanes = int64_t(r->grid_frame) * kPathsBlock;
+            const bool deep = int64_t(p.spf) * p.max_depth >= 24;
+            r->whole = p.wide == 2 && cfg.tail_paths == 0 && (int64_t(n) >= lanes || p.spf == 1) && int64_t(n) <= (deep ? 28 : 20) * lanes;
+            if (r->whole) {
+                r->lane_paths.resize(size_t(lanes) * sizeof(CachePath)); r->lane_shadows.resize(size_t(lanes) * sizeof(CacheShadow));
+                r->claims.resize(n * sizeof(int32_t)); r->done.resize(n * sizeof(int32_t));
+                PT_CUDA(cudaMemset(r->claims.get(), 0, n * sizeof(int32_t)));
+                b.lane_paths = r->lane_paths.get<CachePath>(); b.lane_shadows = r->lane_shadows.get<CacheShadow>();
+                b.claims = r->claims.get<int32_t>(); b.done = r->done.get<int32_t>();
+            }
             // pixel RNG streams as the plain renderer seeds them (pixel_rng.seed(seed, pixel))
             std::vector<Pcg> streams(n);
             for (size_t i = 0; i < n; i++) streams[i].seed(seed, uint64_t(i));

@@ -33,8 +33,9 @@ namespace ptb {
 constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 4;   // 128 registers
 constexpr int kPathsActive = 5;   // lanes of a warp still walking below which the others shade
 
-// The lane's next ray: path and shadow records hold origin and direction at the same places.
-__device__ inline void lane_ray(const PathState &path, const ShadowRay &shadow_ray, bool shadow, pt_ray &r, float &tmax) {
+// The lane's next ray: path and shadow records begin with origin and (shadow) tmax, then the direction.
+template <class Path, class Shadow>
+__device__ inline void lane_ray(const Path &path, const Shadow &shadow_ray, bool shadow, pt_ray &r, float &tmax) {
     const float4 *rec = shadow ? reinterpret_cast<const float4 *>(&shadow_ray) : reinterpret_cast<const float4 *>(&path);
     const float4 o = rec[0], d = rec[1];
     r.origin = pt_vec3{o.x, o.y, o.z};

@@ -81,3 +81,45 @@ def test_batch_in_one_kernel_equals_its_graph_form_and_lone_renderers():
         r.set_tail_paths(0)
         r.add_samples(j["samples"])
         assert r.sums().tobytes() == forms[0][0][k]
+
+
+@pytest.mark.parametrize("width,height,spf,depth", [(64, 40, 1, 9), (400, 200, 1, 5), (401, 203, 3, 9), (320, 260, 8, 3)])
+@pytest.mark.parametrize("use_cache,graph", [(True, True), (True, False), (False, True)])
+def test_cached_frames_in_one_kernel_equal_the_wavefront(scene, width, height, spf, depth, use_cache, graph):
+    """A frozen network: frames are the same bits whichever kernels ran them (a tail length asks for the wavefront)."""
+    flat, dev = scene
+    _, cam = pt.procedural_scene(width, height, sphere_count=6, segments=24, rings=13, seed=3)
+    results = []
+    for tail in (0, 20000):
+        r = pt.CachedRenderer(dev, cam, width, height, seed=4, max_depth=depth, samples_per_frame=spf, train=False, use_cache=use_cache,
+                              use_graph=graph, tail_paths=tail)
+        for k in range(3):
+            if k == 2:
+                r.clear()
+            r.frames(1)
+        s = r.stats()
+        results.append((r.sums().tobytes(), s["rays"], s["queries"], s["frames"]))
+    assert results[0] == results[1]
+    assert np.frombuffer(results[0][0], np.float32).max() > 0 and (results[0][2] > 0) == use_cache
+
+
+def test_cached_training_in_one_kernel(scene):
+    """Online training: the first frame's image uses the initial weights, so it and the counts are the wavefront's; the
+    loss falls as it does there, and training-only frames mix with image frames."""
+    flat, dev = scene
+    _, cam = pt.procedural_scene(400, 220, sphere_count=6, segments=24, rings=13, seed=3)
+    first, last = [], []
+    for tail in (0, 20000):
+        r = pt.CachedRenderer(dev, cam, 400, 220, seed=4, max_depth=8, samples_per_frame=2, training_paths=8192, tail_paths=tail)
+        r.frames(1)
+        s = r.stats()
+        first.append((r.sums().tobytes(), s["rays"], s["queries"], s["samples"]))
+        r.train(20)
+        r.frames(10)
+        last.append(r.stats())
+    assert first[0] == first[1] and first[0][3] > 0
+    for s in last:
+        assert np.isfinite(s["loss"]) and s["frames"] == 22
+    # the same number of training samples within the scatter of two differently trained networks' path ends
+    assert abs(last[0]["samples"] - last[1]["samples"]) <= 0.02 * last[1]["samples"]
+    assert abs(last[0]["loss"] - last[1]["loss"]) <= 0.25 * last[1]["loss"]
