@@ -465,7 +465,7 @@ struct pt_batch {
     DeviceScene view{};
     DeviceBuffer nodes4, nodes2, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, shade_tris, shade_lights, jobs;
     DeviceBuffer sums, rng, paths, hits, shadows, slot_pixel, slot_job, queue0, queue1, shadow_queue, counters, fetch, scalars,
-        job_remaining, job_done_ns, error, lane_paths, lane_shadows, claims, done;
+        job_remaining, job_done_ns, error, lane_records;
     std::vector<BatchJob> host_jobs;
     int64_t total_pixels = 0;
     uint64_t total_triangles = 0;
@@ -515,21 +515,43 @@ struct pt_batch {
         int32_t want = capacity > 0 ? capacity : int32_t(std::min<int64_t>(total_pixels, 1 << 22));
         slots = int32_t(std::min<int64_t>(want, total_pixels));
         size_t n = size_t(std::max(slots, 1));
-        paths.resize(n * sizeof(PathState)); hits.resize(n * sizeof(PathHit)); shadows.resize(n * sizeof(ShadowRay));
-        slot_pixel.resize(n * sizeof(int64_t)); slot_job.resize(n * sizeof(int32_t));
-        queue0.resize(n * sizeof(int32_t)); queue1.resize(n * sizeof(int32_t)); shadow_queue.resize(n * sizeof(int32_t));
-        buf.paths = paths.get<PathState>(); buf.hits = hits.get<PathHit>(); buf.shadows = shadows.get<ShadowRay>();
+        const bool one = one_kernel();
+        const size_t handed = one ? size_t(grid_paths()) * kPathsBlock : 0;   // batch_paths queues at most a path per lane
+        const size_t records = one ? handed : n;
+        paths.resize(records * sizeof(PathState));
+        slot_pixel.resize(records * sizeof(int64_t)); slot_job.resize(records * sizeof(int32_t));
+        queue0.resize(records * sizeof(int32_t));
+        buf.paths = paths.get<PathState>();
         buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
-        buf.queue[0] = queue0.get<int32_t>(); buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
-        if (one_kernel() && !buf.claims) {
-            const size_t lanes = size_t(grid_paths()) * kPathsBlock;
-            lane_paths.resize(lanes * sizeof(PathState)); lane_shadows.resize(lanes * sizeof(ShadowRay));
-            claims.resize(size_t(total_pixels) * sizeof(int32_t)); done.resize(size_t(total_pixels) * sizeof(int32_t));
-            PT_CUDA(cudaMemset(claims.get(), 0, claims.bytes()));
-            buf.lane_paths = lane_paths.get<PathState>(); buf.lane_shadows = lane_shadows.get<ShadowRay>();
-            buf.claims = claims.get<int32_t>(); buf.done = done.get<int32_t>();
+        buf.queue[0] = queue0.get<int32_t>();
+        buf.hits = nullptr;
+        if (!one) wavefront_buffers();
+        if (one && !buf.claims) {
+            const size_t per_pixel = size_t(total_pixels) * sizeof(int32_t);
+            lane_records.resize(handed * (sizeof(PathState) + sizeof(ShadowRay)) + 2 * per_pixel);
+            unsigned char *at = lane_records.get<unsigned char>();
+            buf.lane_paths = reinterpret_cast<PathState *>(at); at += handed * sizeof(PathState);
+            buf.lane_shadows = reinterpret_cast<ShadowRay *>(at); at += handed * sizeof(ShadowRay);
+            buf.claims = reinterpret_cast<int32_t *>(at); at += per_pixel;
+            buf.done = reinterpret_cast<int32_t *>(at);
+            PT_CUDA(cudaMemset(buf.claims, 0, per_pixel));
         }
         drop_graph();
+    }
+    // a record per slot for the loop's kernels, allocated with the first run that needs them
+    void wavefront_buffers() {
+        if (buf.hits) return;
+        const size_t n = size_t(std::max(slots, 1));
+        drop_graph();
+        paths.reserve(n * sizeof(PathState)); slot_pixel.reserve(n * sizeof(int64_t)); slot_job.reserve(n * sizeof(int32_t));
+        queue0.reserve(n * sizeof(int32_t));
+        hits.resize(n * sizeof(PathHit)); shadows.resize(n * sizeof(ShadowRay));
+        queue1.resize(n * sizeof(int32_t)); shadow_queue.resize(n * sizeof(int32_t));
+        buf.paths = paths.get<PathState>();
+        buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
+        buf.queue[0] = queue0.get<int32_t>(); buf.queue[1] = queue1.get<int32_t>();
+        buf.shadows = shadows.get<ShadowRay>(); buf.shadow_queue = shadow_queue.get<int32_t>();
+        buf.hits = hits.get<PathHit>();
     }
     int grid_paths() const {
         int per_sm = 0;
@@ -600,6 +622,8 @@ struct pt_batch {
     }
     void run() {
         cudaStream_t st = stream;
+        const bool whole = use_graph && wide && buf.claims && one_kernel();
+        if (!whole) wavefront_buffers();
         int32_t njobs = int32_t(host_jobs.size());
         std::vector<int32_t> remaining(static_cast<size_t>(njobs));
         for (int32_t k = 0; k < njobs; k++) remaining[size_t(k)] = host_jobs[size_t(k)].pixel_count;
@@ -609,7 +633,6 @@ struct pt_batch {
         PT_CUDA(cudaMemsetAsync(buf.error, 0, sizeof(int32_t), st));
         batch_init<<<unsigned((total_pixels + 255) / 256), 256, 0, st>>>(buf);
         PT_CUDA(cudaEventRecord(start.get(), st));
-        const bool whole = use_graph && wide && buf.claims && one_kernel();
         if (whole) {
             const size_t smem = size_t(kSharedStack4) * sizeof(int2) * kPathsBlock;
             batch_paths_start<<<1, 32, 0, st>>>(buf);

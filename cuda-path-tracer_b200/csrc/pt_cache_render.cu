@@ -752,7 +752,7 @@ struct pt_cached_renderer {
     int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0, grid_frame = 0;
     bool whole = false;                 // frames that render every pixel run as one frame_kernel
     DeviceBuffer paths, hits, shadows, queue0, queue1, shadow_queue, counters, fetch, totals, error, sums, rng, frame;
-    DeviceBuffer queries, aux, pred, pixel_queries, pixel_query_count, vertices, ends, samples, targets, lane_paths, lane_shadows, claims, done;
+    DeviceBuffer queries, aux, pred, pixel_queries, pixel_query_count, vertices, ends, samples, targets, lane_records;
     Buffers buf{};
     cudaStream_t stream = nullptr, body_stream = nullptr, shadow_stream = nullptr;
     Event shaded[2], shadowed[2];
@@ -769,6 +769,15 @@ struct pt_cached_renderer {
         if (body_stream) cudaStreamDestroy(body_stream);
         if (shadow_stream) cudaStreamDestroy(shadow_stream);
         if (stream) cudaStreamDestroy(stream);
+    }
+    // the wavefront's records and queues, allocated with the first frame that needs them
+    void wavefront_buffers() {
+        if (buf.shadow_queue) return;
+        const size_t n = size_t(pixels);
+        hits.resize(n * sizeof(PathHit)); shadows.resize(n * sizeof(CacheShadow));
+        queue1.resize(n * sizeof(int32_t)); shadow_queue.resize(n * sizeof(int32_t));
+        buf.hits = hits.get<PathHit>(); buf.shadows = shadows.get<CacheShadow>();
+        buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
     }
     // the launches of one frame (also what a graph captures)
     Params frame_params(int accumulate) const {
@@ -859,27 +868,27 @@ struct pt_cached_renderer {
         try {
             prologue(p, stream);
             if (!(whole && accumulate)) {
-            cudaStreamCaptureStatus status;
-            cudaGraph_t g = nullptr;
-            const cudaGraphNode_t *deps = nullptr;
-            size_t ndeps = 0;
-            PT_CUDA(cudaStreamGetCaptureInfo(stream, &status, nullptr, &g, &deps, &ndeps));
-            cudaGraphConditionalHandle handle;
-            PT_CUDA(cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault));
-            cudaGraphNodeParams cp{};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = handle;
-            cp.conditional.type = cudaGraphCondTypeWhile;
-            cp.conditional.size = 1;
-            cudaGraphNode_t loop;
-            PT_CUDA(cudaGraphAddNode(&loop, g, deps, ndeps, &cp));
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            PT_CUDA(cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-            iteration_pair(p, body_stream);
-            control_kernel<<<1, 32, 0, body_stream>>>(buf, handle, tail_paths, max_pairs(p));
-            PT_CUDA(cudaGetLastError());
-            PT_CUDA(cudaStreamEndCapture(body_stream, &body));
-            PT_CUDA(cudaStreamUpdateCaptureDependencies(stream, &loop, 1, cudaStreamSetCaptureDependencies));
+                cudaStreamCaptureStatus status;
+                cudaGraph_t g = nullptr;
+                const cudaGraphNode_t *deps = nullptr;
+                size_t ndeps = 0;
+                PT_CUDA(cudaStreamGetCaptureInfo(stream, &status, nullptr, &g, &deps, &ndeps));
+                cudaGraphConditionalHandle handle;
+                PT_CUDA(cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault));
+                cudaGraphNodeParams cp{};
+                cp.type = cudaGraphNodeTypeConditional;
+                cp.conditional.handle = handle;
+                cp.conditional.type = cudaGraphCondTypeWhile;
+                cp.conditional.size = 1;
+                cudaGraphNode_t loop;
+                PT_CUDA(cudaGraphAddNode(&loop, g, deps, ndeps, &cp));
+                cudaGraph_t body = cp.conditional.phGraph_out[0];
+                PT_CUDA(cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+                iteration_pair(p, body_stream);
+                control_kernel<<<1, 32, 0, body_stream>>>(buf, handle, tail_paths, max_pairs(p));
+                PT_CUDA(cudaGetLastError());
+                PT_CUDA(cudaStreamEndCapture(body_stream, &body));
+                PT_CUDA(cudaStreamUpdateCaptureDependencies(stream, &loop, 1, cudaStreamSetCaptureDependencies));
             }
             epilogue(p, stream);
         } catch (...) {
@@ -988,11 +997,7 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
                 for (int a = 0; a < 3; a++) p.radiance_max[a] = bound[a];
             }
             r->paths.resize(n * sizeof(CachePath));
-            r->hits.resize(n * sizeof(PathHit));
-            r->shadows.resize(n * sizeof(CacheShadow));
             r->queue0.resize(n * sizeof(int32_t));
-            r->queue1.resize(n * sizeof(int32_t));
-            r->shadow_queue.resize(n * sizeof(int32_t));
             r->counters.resize(kCounters * sizeof(int32_t));
             r->fetch.resize(4 * sizeof(unsigned long long));
             r->totals.resize(3 * sizeof(unsigned long long));
@@ -1016,9 +1021,8 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
                 r->targets.resize(total * 3 * sizeof(float));
             }
             Buffers &b = r->buf;
-            b.paths = r->paths.get<CachePath>(); b.hits = r->hits.get<PathHit>(); b.shadows = r->shadows.get<CacheShadow>();
-            b.queue[0] = r->queue0.get<int32_t>(); b.queue[1] = r->queue1.get<int32_t>();
-            b.shadow_queue = r->shadow_queue.get<int32_t>(); b.counters = r->counters.get<int32_t>();
+            b.paths = r->paths.get<CachePath>();
+            b.queue[0] = r->queue0.get<int32_t>(); b.counters = r->counters.get<int32_t>();
             b.fetch = r->fetch.get<unsigned long long>(); b.totals = r->totals.get<unsigned long long>();
             b.error = r->error.get<int32_t>(); b.sums = r->sums.get<float>(); b.rng = r->rng.get<Pcg>();
             b.frame = r->frame.get<uint32_t>();
@@ -1049,11 +1053,16 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
             const bool deep = int64_t(p.spf) * p.max_depth >= 24;
             r->whole = p.wide == 2 && cfg.tail_paths == 0 && (int64_t(n) >= lanes || p.spf == 1) && int64_t(n) <= (deep ? 28 : 20) * lanes;
             if (r->whole) {
-                r->lane_paths.resize(size_t(lanes) * sizeof(CachePath)); r->lane_shadows.resize(size_t(lanes) * sizeof(CacheShadow));
-                r->claims.resize(n * sizeof(int32_t)); r->done.resize(n * sizeof(int32_t));
-                PT_CUDA(cudaMemset(r->claims.get(), 0, n * sizeof(int32_t)));
-                b.lane_paths = r->lane_paths.get<CachePath>(); b.lane_shadows = r->lane_shadows.get<CacheShadow>();
-                b.claims = r->claims.get<int32_t>(); b.done = r->done.get<int32_t>();
+                const size_t l = size_t(lanes), per_pixel = n * sizeof(int32_t);
+                r->lane_records.resize(l * (sizeof(CachePath) + sizeof(CacheShadow)) + 2 * per_pixel);
+                unsigned char *at = r->lane_records.get<unsigned char>();
+                b.lane_paths = reinterpret_cast<CachePath *>(at); at += l * sizeof(CachePath);
+                b.lane_shadows = reinterpret_cast<CacheShadow *>(at); at += l * sizeof(CacheShadow);
+                b.claims = reinterpret_cast<int32_t *>(at); at += per_pixel;
+                b.done = reinterpret_cast<int32_t *>(at);
+                PT_CUDA(cudaMemset(b.claims, 0, per_pixel));
+            } else {
+                r->wavefront_buffers();
             }
             // pixel RNG streams as the plain renderer seeds them (pixel_rng.seed(seed, pixel))
             std::vector<Pcg> streams(n);
@@ -1078,6 +1087,7 @@ pt_status pt_cached_frames(pt_cached_renderer *r, int frames, int accumulate) {
             throw Error(PT_INVALID_ARGUMENT, "invalid accumulated sample count");
         if (!accumulate && !(r->params.train_threshold && r->training))
             throw Error(PT_INVALID_ARGUMENT, "training-only frames need online training");
+        if (!(r->whole && accumulate)) r->wavefront_buffers();
         cudaGraphExec_t g = r->cfg.use_graph ? r->graph(accumulate) : nullptr;
         PT_CUDA(cudaEventRecord(r->start.get(), r->stream));
         for (int f = 0; f < frames; f++) {

@@ -550,7 +550,7 @@ struct pt_renderer {
     bool pair_tail = false;             // the tail runs two lanes per path (finish_pair_kernel)
     bool fused = false;                 // four-wide tree and shaded view: render_paths_kernel where the image's size suits it
     bool small = false;                 // the scene fits render_small_kernel and the view is shaded
-    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lane_paths, lane_shadows;
+    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lanes;
     RenderBuffers buf{};
     cudaStream_t stream = nullptr;
     cudaStream_t shadow_stream = nullptr;   // shadow kernel k runs beside extend k+1
@@ -563,6 +563,46 @@ struct pt_renderer {
         if (shadow_stream) cudaStreamDestroy(shadow_stream);
         if (stream) cudaStreamDestroy(stream);
     }
+    // What the kernels of this renderer's form need, allocated when it is first used: path records and the
+    // queue of render_paths_kernel's tail with its lanes' records and claims, and the wavefront's other
+    // records and queues.
+    void path_buffers() {
+        const size_t n = size_t(pixels);
+        if (buf.paths) return;
+        paths.resize(n * sizeof(PathState)); queue0.resize(n * sizeof(int32_t));
+        buf.paths = paths.get<PathState>(); buf.queue[0] = queue0.get<int32_t>();
+    }
+    void lane_buffers() {
+        path_buffers();
+        if (buf.claims) return;
+        const size_t l = size_t(grid_paths) * kPathsBlock, claimed = size_t(pixels) * sizeof(int32_t);
+        lanes.resize(l * (sizeof(PathState) + sizeof(ShadowRay)) + claimed);
+        unsigned char *at = lanes.get<unsigned char>();
+        buf.lane_paths = reinterpret_cast<PathState *>(at);
+        buf.lane_shadows = reinterpret_cast<ShadowRay *>(at + l * sizeof(PathState));
+        buf.claims = reinterpret_cast<int32_t *>(at + l * (sizeof(PathState) + sizeof(ShadowRay)));
+        PT_CUDA(cudaMemsetAsync(buf.claims, 0, claimed, stream));
+    }
+    void wavefront_buffers() {
+        path_buffers();
+        if (buf.hits) return;
+        const size_t n = size_t(pixels);
+        hits.resize(n * sizeof(PathHit));
+        if (params.debug == PT_DEBUG_BVH || params.debug == PT_DEBUG_INTERSECTIONS) stats.resize(n * sizeof(uint2));
+        shadows.resize(n * sizeof(ShadowRay)); queue1.resize(n * sizeof(int32_t)); shadow_queue.resize(n * sizeof(int32_t));
+        buf.hits = hits.get<PathHit>(); buf.stats = stats.get<uint2>(); buf.shadows = shadows.get<ShadowRay>();
+        buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
+    }
+    // One kernel for the whole render (render_paths_kernel) where every resident lane has a pixel: with
+    // fewer, the tail kernel's two lanes per path are faster (240x150, 16 spp: 3.7 ms against 5.0; 320x240
+    // 6.7 against 6.2), except for one or two samples, where the wavefront's launches are most of the time
+    // (240x150: 0.88 ms against 0.47).  Up to 40 pixels per lane: from there on the wavefront's queues are long
+    // enough to hide their slowest rays and its walk kernels hold twice the warps (1920x1080 30.4 ms
+    // against 29.0; 3840x2160 91.8 against 111.8).
+    bool whole(int count) const {
+        const int64_t l = int64_t(grid_paths) * kPathsBlock;
+        return fused && pixels <= 40 * l && (pixels >= l || count <= 2);
+    }
     void grids() {
         grid_extend = occupancy_grid((const void *)extend_kernel, block, stack_bytes(block));
         grid_shade = occupancy_grid((const void *)shade_kernel, block);
@@ -570,9 +610,6 @@ struct pt_renderer {
         grid_finish = occupancy_grid((const void *)finish_kernel, kFinishBlock);
         grid_finish_pair = occupancy_grid((const void *)finish_pair_kernel, block);
         grid_paths = occupancy_grid((const void *)render_paths_kernel, kPathsBlock, stack_bytes(kPathsBlock));
-        lane_paths.resize(size_t(grid_paths) * kPathsBlock * sizeof(PathState));
-        lane_shadows.resize(size_t(grid_paths) * kPathsBlock * sizeof(ShadowRay));
-        buf.lane_paths = lane_paths.get<PathState>(); buf.lane_shadows = lane_shadows.get<ShadowRay>();
         grid_small = occupancy_grid((const void *)render_small_kernel, kSmallBlock);
     }
 };
@@ -614,29 +651,17 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             p.debug = debug_mode; p.mis = (flags & PT_RENDER_MIS) ? 1 : 0; p.brute = (flags & PT_RENDER_BRUTE) ? 1 : 0;
             p.leaves = scene->leaf_count; p.brute_order = scene->brute_order.get<int32_t>();
             p.wide = (g_query_config.wide && scene->view.nodes4) ? (g_query_config.speculative ? 2 : 1) : 0;
-            r->paths.resize(n * sizeof(PathState));
-            r->hits.resize(n * sizeof(PathHit));
-            if (debug_mode == PT_DEBUG_BVH || debug_mode == PT_DEBUG_INTERSECTIONS) r->stats.resize(n * sizeof(uint2));
-            r->shadows.resize(n * sizeof(ShadowRay));
-            r->queue0.resize(n * sizeof(int32_t));
-            r->queue1.resize(n * sizeof(int32_t));
-            r->shadow_queue.resize(n * sizeof(int32_t));
             r->counters.resize(4 * sizeof(int32_t));
             r->fetch.resize(4 * sizeof(unsigned long long));
             r->ray_total.resize(sizeof(unsigned long long));
             r->error.resize(sizeof(int32_t));
             r->sums.resize(n * 3 * sizeof(float));
-            r->claims.resize(n * sizeof(int32_t));
-            PT_CUDA(cudaMemset(r->claims.get(), 0, n * sizeof(int32_t)));
             r->rng.resize(n * sizeof(Pcg));
             RenderBuffers &b = r->buf;
-            b.paths = r->paths.get<PathState>(); b.hits = r->hits.get<PathHit>(); b.stats = r->stats.get<uint2>();
-            b.shadows = r->shadows.get<ShadowRay>();
-            b.queue[0] = r->queue0.get<int32_t>(); b.queue[1] = r->queue1.get<int32_t>();
-            b.shadow_queue = r->shadow_queue.get<int32_t>(); b.counters = r->counters.get<int32_t>();
+            b.counters = r->counters.get<int32_t>();
             b.fetch = r->fetch.get<unsigned long long>();
             b.rays = r->ray_total.get<unsigned long long>(); b.error = r->error.get<int32_t>();
-            b.sums = r->sums.get<float>(); b.rng = r->rng.get<Pcg>(); b.claims = r->claims.get<int32_t>();
+            b.sums = r->sums.get<float>(); b.rng = r->rng.get<Pcg>();
             PT_CUDA(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking));
             PT_CUDA(cudaStreamCreateWithFlags(&r->shadow_stream, cudaStreamNonBlocking));
             PT_CUDA(cudaMallocHost(&r->host_counters, kIterationRing * sizeof(int32_t)));
@@ -654,6 +679,10 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             r->pair_tail = p.wide != 0;
             r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
             r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
+            if (!r->small) {                             // what the first call will most likely use
+                if (r->whole(3)) r->lane_buffers();
+                else r->wavefront_buffers();
+            }
         } catch (...) { delete r; throw; }
         *out = r;
         pt_status st = pt_reset(r, camera);
@@ -684,16 +713,11 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         if (count <= 0 || count > INT32_MAX - r->samples) throw Error(PT_INVALID_ARGUMENT, "invalid accumulated sample count");
         const DeviceScene &scene = r->scene->view;
         cudaStream_t st = r->stream;
+        const bool whole = !r->small && r->whole(count);
+        if (whole) r->lane_buffers();
+        else if (!r->small) r->wavefront_buffers();
         PT_CUDA(cudaMemsetAsync(r->buf.rays, 0, sizeof(unsigned long long), st));
         PT_CUDA(cudaEventRecord(r->start.get(), st));
-        // One kernel for the whole render (render_paths_kernel) where every resident lane has a pixel: with
-        // fewer, the tail kernel's two lanes per path are faster (240x150, 16 spp: 3.7 ms against 5.0; 320x240
-        // 6.7 against 6.2), except for one or two samples, where the wavefront's launches are most of the time
-        // (240x150: 0.88 ms against 0.47).  Up to 40 pixels per lane: from there on the wavefront's queues are long
-        // enough to hide their slowest rays and its walk kernels hold twice the warps (1920x1080 30.4 ms
-        // against 29.0; 3840x2160 91.8 against 111.8).
-        const int64_t lanes = int64_t(r->grid_paths) * kPathsBlock;
-        const bool whole = r->fused && r->pixels <= 40 * lanes && (r->pixels >= lanes || count <= 2);
         if (r->small) {
             PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
             const int blocks = std::min(r->grid_small, (r->pixels + kSmallBlock - 1) / kSmallBlock);
