@@ -1047,8 +1047,8 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
             // Frames as one kernel, unless a tail length asks for the wavefront: from one pixel per resident lane (or with
             // one sample) to twenty, and to twenty-eight when the bounces of a frame are many.  Wavefront and this, ms a
             // frame (1M triangles, bounce limit 12): 480x300 one sample 0.89 and 0.69, four 3.0 and 2.2; 960x600 4.8
-            // and 3.0; 1920x1080 one 2.1 and 2.3, two 4.07 and 3.94, four 7.8 and 7.25, four of limit 4 6.5 and 6.6;
-            // 2560x1440 11.0 and 12.2; 200x120 on 65,000 triangles two samples 0.26 and 0.30.
+            // and 3.0; with four blocks per SM 1920x1080 one 2.1 and 2.3, two 4.07 and 3.94, four 7.8 and 7.25, four of
+            // limit 4 6.5 and 6.6; 2560x1440 11.0 and 12.2; 200x120 on 65,000 triangles two samples 0.26 and 0.30.
             const int64_t lanes = int64_t(r->grid_frame) * kPathsBlock;
             const bool deep = int64_t(p.spf) * p.max_depth >= 24;
             r->whole = p.wide == 2 && cfg.tail_paths == 0 && (int64_t(n) >= lanes || p.spf == 1) && int64_t(n) <= (deep ? 28 : 20) * lanes;

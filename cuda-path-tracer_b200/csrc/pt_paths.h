@@ -16,13 +16,14 @@
 // finds the claim when its sample ends and runs the next sample itself.  No lane waits for another,
 // and a heavy pixel runs without a break from the first pass on.
 //
-// What it measured (1M triangles, bounce limit 8, 16 spp; wavefront and pair tail before): 960x600
-// 15.1 -> 9.4 ms, 480x300 8.4 -> 6.3, 1920x1080 30.4 -> 29.0; 65,000 triangles at 960x600 5.4 -> 2.9.
+// What it measured (kernel time, 1M triangles, bounce limit 8, 16 spp; wavefront and pair tail before):
+// 960x600 15.1 -> 9.4 ms, 480x300 8.4 -> 7.0, 1920x1080 30.4 -> 27.0; 65,000 triangles at 960x600 5.4 -> 2.8.
 // Lanes that shade together cost one pass through 60 KB of shading code whether 8 or 28 of them do, so
-// a warp waits until fewer than kPathsActive still walk (24: 13.0 ms, 16: 12.3, 8: 11.35, 5: 10.9, 2:
-// 11.5 for the whole call), and 128 registers without spills beat more warps (5 blocks of 128 per SM:
-// 0.6 ms slower, 8: 2.2).  Shading 32 at a time from rings of 64 paths per warp filled the lanes better
-// (8.2 ms until the items ran out) but doubled the time a heavy pixel waits for each bounce (12.6 ms).
+// a warp waits until fewer than kPathsActive still walk (the 960x600 call: 24 13.0 ms, 16 12.3, 8 11.35, 5
+// 10.9, 2 11.5).  Five blocks of 128 per SM, since records became the lanes' own and stay in L1: with four
+// 1920x1080 takes 29.2 ms (480x300 6.8), with six 960x600 10 % more.  Shading 32 at a time from rings of 64
+// paths per warp filled the lanes better (8.2 ms until the items ran out, records in the pixels' slots) but
+// doubled the time a heavy pixel waits for each bounce (12.6 ms in all).
 #pragma once
 
 #include "pt_wavefront.h"
@@ -30,8 +31,8 @@
 #ifdef __CUDACC__
 namespace ptb {
 
-constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 4;   // 128 registers
-constexpr int kPathsActive = 5;   // lanes of a warp still walking below which the others shade
+constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 5;   // 96 registers
+constexpr int kPathsActive = 4;   // lanes of a warp still walking below which the others shade
 
 // The lane's next ray: path and shadow records begin with origin and (shadow) tmax, then the direction.
 template <class Path, class Shadow>

@@ -594,11 +594,11 @@ struct pt_renderer {
         buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
     }
     // One kernel for the whole render (render_paths_kernel) where every resident lane has a pixel: with
-    // fewer, the tail kernel's two lanes per path are faster (240x150, 16 spp: 3.7 ms against 5.0; 320x240
-    // 6.7 against 6.2), except for one or two samples, where the wavefront's launches are most of the time
-    // (240x150: 0.88 ms against 0.47).  Up to 40 pixels per lane: from there on the wavefront's queues are long
-    // enough to hide their slowest rays and its walk kernels hold twice the warps (1920x1080 30.4 ms
-    // against 29.0; 3840x2160 91.8 against 111.8).
+    // fewer, the tail kernel's two lanes per path are faster (wavefront and this, 240x150, 16 spp: 3.7 and 5.0 ms;
+    // 320x240 6.7 and 6.3), except for one or two samples, where the wavefront's launches are most of the time
+    // (240x150: 0.88 and 0.47).  Up to 40 pixels per lane: from there on the wavefront's queues are long enough
+    // to hide their slowest rays and its walk kernels hold more warps (1920x1080 30.4 and 27.0; with four
+    // blocks per SM 3840x2160 91.8 and 111.8).
     bool whole(int count) const {
         const int64_t l = int64_t(grid_paths) * kPathsBlock;
         return fused && pixels <= 40 * l && (pixels >= l || count <= 2);

@@ -29,7 +29,7 @@ def render(scene, width, height, batches, depth, mis, tail):
 
 # pixels below, at and above the resident threads; one to many samples (each side of the hand-over to the
 # tail kernel, and of the samples below which few pixels run in one kernel); single pixels; several calls
-@pytest.mark.parametrize("width,height,batches", [(1, 1, [2]), (1, 1, [1, 1, 2]), (31, 1, [2]), (33, 7, [1, 2]), (320, 240, [3]),
+@pytest.mark.parametrize("width,height,batches", [(1, 1, [2]), (1, 1, [1, 1, 2]), (31, 1, [2]), (33, 7, [1, 2]), (320, 240, [3]), (430, 260, [3]),
                                                   (400, 200, [1, 5, 2]), (401, 199, [24]), (512, 300, [4, 1])])
 @pytest.mark.parametrize("depth,mis", [(0, True), (3, False), (12, True)])
 def test_equals_wavefront(scene, width, height, batches, depth, mis):
