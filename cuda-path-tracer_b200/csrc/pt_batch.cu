@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256, 2) batch_finish_pair(DeviceScene scene, B
     Pcg rng{};
     bool live = false;             // even lane: the path has a ray to walk
     bool pending = false;          // even lane: a shadow ray from the last shading waits
-    bool drained = false;          // even lane: neither pixels nor queued slots are left
+    bool drained = int(lane >> 1) >= pairs_per_warp(n);   // even lane: neither pixels nor queued slots are left
     ShadowRay sr{};
     bool walk_shadow = false;      // odd lane: walks the pair's pending shadow ray this round
     pt_ray q{};
@@ -431,10 +431,10 @@ struct BatchOps {
 };
 
 __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) batch_paths(DeviceScene scene, BatchBuffers b,
-                                                                             unsigned long long items, bool hand_over) {
+                                                                             unsigned long long items) {
     BatchOps ops{scene, b, blockIdx.x * blockDim.x + threadIdx.x, 0, 0};
     unsigned long long rays = 0;
-    persistent_paths4(scene, ops, items, &b.fetch[0], hand_over, kTieLastLeaf, rays, b.error);
+    persistent_paths4(scene, ops, items, &b.fetch[0], kTieLastLeaf, rays, b.error);
     for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(0xffffffffu, rays, o);
     if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
 }
@@ -516,7 +516,7 @@ struct pt_batch {
         slots = int32_t(std::min<int64_t>(want, total_pixels));
         size_t n = size_t(std::max(slots, 1));
         const bool one = one_kernel();
-        const size_t handed = one ? size_t(grid_paths()) * kPathsBlock : 0;   // batch_paths queues at most a path per lane
+        const size_t handed = one ? size_t(lane_count()) : 0;   // batch_paths queues at most a path per lane
         const size_t records = one ? handed : n;
         paths.resize(records * sizeof(PathState));
         slot_pixel.resize(records * sizeof(int64_t)); slot_job.resize(records * sizeof(int32_t));
@@ -525,7 +525,7 @@ struct pt_batch {
         buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
         buf.queue[0] = queue0.get<int32_t>();
         buf.hits = nullptr;
-        if (!one) wavefront_buffers();
+        if (!one && !tail_alone()) wavefront_buffers();
         if (one && !buf.claims) {
             const size_t per_pixel = size_t(total_pixels) * sizeof(int32_t);
             lane_records.resize(handed * (sizeof(PathState) + sizeof(ShadowRay)) + 2 * per_pixel);
@@ -564,14 +564,14 @@ struct pt_batch {
         for (const auto &j : host_jobs) most = std::max(most, j.samples);
         return most;
     }
-    // Whether a graph-form run of four-wide nodes is one batch_paths launch: for the pixel counts where that is
-    // the faster form (the renderer's rule, pt_add_samples), if every lane could queue its path for the tail.
-    // Six jobs, device time of the graph form and of this: 129,000 pixels 6.8 and 3.2 ms, 534,000 11.9 and 7.0, 1.2M
-    // 32.0 and 25.8, 2.3M 20.6 and 19.5.
-    bool one_kernel() const {
-        const int64_t lanes = int64_t(grid_paths()) * kPathsBlock;
-        return total_pixels <= 40 * lanes && total_pixels >= lanes && slots >= lanes;
-    }
+    // The renderer's rule (pt_renderer::whole and tail_alone) for graph-form runs of four-wide nodes, where every
+    // lane, or every pixel, has a slot.  Six jobs, ms: the graph's loop and the tail kernel
+    // alone 3,900 pixels 0.53 and 0.30, 23,000 1.54 and 0.93, 88,000 4.7 and 2.3; one kernel and the tail kernel alone
+    // 129,000 3.1 and 3.2, 175,000 3.6 and 3.2; the loop and one kernel (four blocks per SM) 534,000 11.9 and 7.0,
+    // 1.2M 32.0 and 25.8, 2.3M 20.6 and 19.5.
+    int64_t lane_count() const { return int64_t(grid_paths()) * kPathsBlock; }
+    bool one_kernel() const { return total_pixels > 2 * lane_count() && total_pixels <= 40 * lane_count() && slots >= lane_count(); }
+    bool tail_alone() const { return total_pixels <= 2 * lane_count() && slots >= total_pixels; }
     unsigned long long max_iterations() const {
         // every pixel needs at most samples * (depth + 1) extends; slots run pixels back to back
         unsigned long long worst = 0;
@@ -623,7 +623,8 @@ struct pt_batch {
     void run() {
         cudaStream_t st = stream;
         const bool whole = use_graph && wide && buf.claims && one_kernel();
-        if (!whole) wavefront_buffers();
+        const bool alone = use_graph && wide && tail_alone();
+        if (!whole && !alone) wavefront_buffers();
         int32_t njobs = int32_t(host_jobs.size());
         std::vector<int32_t> remaining(static_cast<size_t>(njobs));
         for (int32_t k = 0; k < njobs; k++) remaining[size_t(k)] = host_jobs[size_t(k)].pixel_count;
@@ -636,8 +637,7 @@ struct pt_batch {
         if (whole) {
             const size_t smem = size_t(kSharedStack4) * sizeof(int2) * kPathsBlock;
             batch_paths_start<<<1, 32, 0, st>>>(buf);
-            batch_paths<<<grid_paths(), kPathsBlock, smem, st>>>(view, buf, (unsigned long long)total_pixels * (unsigned long long)max_samples(),
-                                                                 true);
+            batch_paths<<<grid_paths(), kPathsBlock, smem, st>>>(view, buf, (unsigned long long)total_pixels * (unsigned long long)max_samples());
             PT_CUDA(cudaGetLastError());
             launch_finish(st);
         } else {
@@ -645,6 +645,9 @@ struct pt_batch {
         }
         PT_CUDA(cudaGetLastError());
         if (whole) {
+            // batch_paths and its tail are under way
+        } else if (alone) {
+            launch_finish(st);
         } else if (use_graph) {
             if (!exec) build_graph();
             PT_CUDA(cudaGraphLaunch(exec, st));

@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
     Pcg rng{};
     bool live = false;             // even lane: the path has a ray to walk
     bool pending = false;          // even lane: a shadow ray from the last shading waits
-    bool drained = false;          // even lane: the queue had no entry left for this pair
+    bool drained = int(lane >> 1) >= pairs_per_warp(n);   // even lane: the queue had no entry left for this pair
     CacheShadow sr{};              // even lane: the pending shadow ray
     bool walk_shadow = false;      // odd lane: walks the pair's pending shadow ray this round
     pt_ray q{};
@@ -633,7 +633,7 @@ struct FrameOps {
 __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) frame_kernel(DeviceScene scene, Params p, Buffers b, int32_t pixels) {
     FrameOps ops{scene, p, b, uint32_t(pixels), blockIdx.x * blockDim.x + threadIdx.x, 0};
     unsigned long long rays = 0;
-    persistent_paths4(scene, ops, (unsigned long long)pixels * (unsigned long long)p.spf, &b.fetch[0], true, kTieLastLeaf, rays, b.error);
+    persistent_paths4(scene, ops, (unsigned long long)pixels * (unsigned long long)p.spf, &b.fetch[0], kTieLastLeaf, rays, b.error);
     for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(0xffffffffu, rays, o);
     if (lane_id() == 0 && rays) atomicAdd(&b.totals[0], rays);
 }
@@ -751,6 +751,7 @@ struct pt_cached_renderer {
     int block = 256;
     int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0, grid_frame = 0;
     bool whole = false;                 // frames that render every pixel run as one frame_kernel
+    bool alone = false;                 // their paths run in the tail kernel alone
     DeviceBuffer paths, hits, shadows, queue0, queue1, shadow_queue, counters, fetch, totals, error, sums, rng, frame;
     DeviceBuffer queries, aux, pred, pixel_queries, pixel_query_count, vertices, ends, samples, targets, lane_records;
     Buffers buf{};
@@ -851,7 +852,7 @@ struct pt_cached_renderer {
         cudaStream_t st = stream;
         prologue(p, st);
         const unsigned long long bound = max_pairs(p);
-        for (unsigned long long pair = 0; !(whole && accumulate); pair++) {
+        for (unsigned long long pair = 0; !((whole || alone) && accumulate); pair++) {
             iteration_pair(p, st);
             PT_CUDA(cudaMemcpyAsync(live_host, &buf.counters[0], sizeof(int32_t), cudaMemcpyDeviceToHost, st));
             PT_CUDA(cudaStreamSynchronize(st));
@@ -867,7 +868,7 @@ struct pt_cached_renderer {
         PT_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
             prologue(p, stream);
-            if (!(whole && accumulate)) {
+            if (!((whole || alone) && accumulate)) {
                 cudaStreamCaptureStatus status;
                 cudaGraph_t g = nullptr;
                 const cudaGraphNode_t *deps = nullptr;
@@ -1044,14 +1045,19 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
             r->grid_finish_pair = occupancy_grid((const void *)finish_pair_kernel, r->block, 0);
             r->grid_small = device_sm_count() * 4;
             r->grid_frame = occupancy_grid((const void *)frame_kernel, kPathsBlock, size_t(kSharedStack4) * sizeof(int2) * kPathsBlock);
-            // Frames as one kernel, unless a tail length asks for the wavefront: from one pixel per resident lane (or with
-            // one sample) to twenty, and to twenty-eight when the bounces of a frame are many.  Wavefront and this, ms a
-            // frame (1M triangles, bounce limit 12): 480x300 one sample 0.89 and 0.69, four 3.0 and 2.2; 960x600 4.8
-            // and 3.0; with four blocks per SM 1920x1080 one 2.1 and 2.3, two 4.07 and 3.94, four 7.8 and 7.25, four of
-            // limit 4 6.5 and 6.6; 2560x1440 11.0 and 12.2; 200x120 on 65,000 triangles two samples 0.26 and 0.30.
-            const int64_t lanes = int64_t(r->grid_frame) * kPathsBlock;
-            const bool deep = int64_t(p.spf) * p.max_depth >= 24;
-            r->whole = p.wide == 2 && cfg.tail_paths == 0 && (int64_t(n) >= lanes || p.spf == 1) && int64_t(n) <= (deep ? 28 : 20) * lanes;
+            // A frame that renders every pixel, unless a tail length asks for the wavefront: up to three pixels per resident
+            // lane by the tail kernel alone, whose two lanes per path walk extension and shadow rays side by side; up to
+            // twenty, or twenty-eight when the bounces of a frame are many, by frame_kernel; above by the wavefront.
+            // Tail kernel alone and frame_kernel, ms a frame (1M triangles, bounce limit 12; three pixels per lane are
+            // 284,000): 100x80 one sample 0.34 and 0.43, four 0.91 and 1.24; 480x300 0.64 and 0.74, 2.18 and 2.34;
+            // 640x400 0.74 and 0.86, 2.54 and 2.67; 960x600 1.16 and 1.10, 4.2 and 3.1; 65,000 triangles 200x120 two
+            // samples 0.15 and 0.28 (wavefront 0.26), 640x400 0.31 and 0.42, 960x600 0.51 and 0.51.  Wavefront and
+            // frame_kernel: 960x600 four 4.8 and 3.0; with four blocks per SM 1920x1080 one 2.1 and 2.3, two 4.07 and
+            // 3.94, four 7.8 and 7.25, four of limit 4 6.5 and 6.6; 2560x1440 11.0 and 12.2.
+            const int64_t lanes = int64_t(r->grid_frame) * kPathsBlock, count = int64_t(n);
+            const bool deep = int64_t(p.spf) * p.max_depth >= 24, chosen = p.wide == 2 && cfg.tail_paths == 0;
+            r->alone = chosen && count <= 3 * lanes;
+            r->whole = chosen && !r->alone && count <= (deep ? 28 : 20) * lanes;
             if (r->whole) {
                 const size_t l = size_t(lanes), per_pixel = n * sizeof(int32_t);
                 r->lane_records.resize(l * (sizeof(CachePath) + sizeof(CacheShadow)) + 2 * per_pixel);
@@ -1061,7 +1067,7 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
                 b.claims = reinterpret_cast<int32_t *>(at); at += per_pixel;
                 b.done = reinterpret_cast<int32_t *>(at);
                 PT_CUDA(cudaMemset(b.claims, 0, per_pixel));
-            } else {
+            } else if (!r->alone) {
                 r->wavefront_buffers();
             }
             // pixel RNG streams as the plain renderer seeds them (pixel_rng.seed(seed, pixel))
@@ -1087,7 +1093,7 @@ pt_status pt_cached_frames(pt_cached_renderer *r, int frames, int accumulate) {
             throw Error(PT_INVALID_ARGUMENT, "invalid accumulated sample count");
         if (!accumulate && !(r->params.train_threshold && r->training))
             throw Error(PT_INVALID_ARGUMENT, "training-only frames need online training");
-        if (!(r->whole && accumulate)) r->wavefront_buffers();
+        if (!((r->whole || r->alone) && accumulate)) r->wavefront_buffers();
         cudaGraphExec_t g = r->cfg.use_graph ? r->graph(accumulate) : nullptr;
         PT_CUDA(cudaEventRecord(r->start.get(), r->stream));
         for (int f = 0; f < frames; f++) {

@@ -61,7 +61,7 @@ struct NextWalk {
 // dynamic shared memory.
 template <class Ops>
 __device__ inline void persistent_paths4(const DeviceScene &s, Ops &ops, unsigned long long items, unsigned long long *next,
-                                         bool hand_over, int tie, unsigned long long &rays, int32_t *error_flag) {
+                                         int tie, unsigned long long &rays, int32_t *error_flag) {
     extern __shared__ int32_t shared_stack[];
     int2 *my_stack = reinterpret_cast<int2 *>(shared_stack) + threadIdx.x;
     const int stride = blockDim.x;
@@ -120,7 +120,7 @@ __device__ inline void persistent_paths4(const DeviceScene &s, Ops &ops, unsigne
             if (base + __popc(m) >= items) drained = true;
         }
         // ---- with no items left, paths go to the tail kernel at their next extension ray
-        if (hand_over && drained && path && !walking && !any) { ops.hand_over(); path = false; }
+        if (drained && path && !walking && !any) { ops.hand_over(); path = false; }
         if (path && !walking) {
             float tmax = FLT_MAX;
             ops.ray(any, r, tmax);

@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
     Pcg rng{};
     bool live = false;             // even lane: the path has an extension ray to walk
     bool pending = false;          // even lane: a shadow ray from the last shading waits
-    bool drained = false;          // even lane: the queue had no entry left for this pair
+    bool drained = int(lane >> 1) >= pairs_per_warp(n);   // even lane: the queue had no entry left for this pair
     ShadowRay sr{};
     bool walk_shadow = false;      // odd lane: walks the pair's pending shadow ray this round
     pt_ray q{};
@@ -452,14 +452,13 @@ struct RenderOps {
 };
 
 __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) render_paths_kernel(DeviceScene scene, RenderParams p, RenderBuffers b,
-                                                                                     int32_t pixels, int samples, bool hand_over) {
+                                                                                     int32_t pixels, int samples) {
     ShadeCtx ctx;
     ctx.camera = &p.camera; ctx.width = p.width; ctx.height = p.height; ctx.max_depth = p.max_depth;
     ctx.debug = PT_DEBUG_SHADED; ctx.mis = p.mis;
     RenderOps ops{scene, p, b, ctx, uint32_t(pixels), blockIdx.x * blockDim.x + threadIdx.x, 0};
     unsigned long long rays = 0;
-    persistent_paths4(scene, ops, (unsigned long long)pixels * (unsigned long long)samples, &b.fetch[3], hand_over, kTieLastLeaf, rays,
-                      b.error);
+    persistent_paths4(scene, ops, (unsigned long long)pixels * (unsigned long long)samples, &b.fetch[3], kTieLastLeaf, rays, b.error);
     for (int o = 16; o; o >>= 1) rays += __shfl_down_sync(0xffffffffu, rays, o);
     if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
 }
@@ -548,7 +547,7 @@ struct pt_renderer {
     int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_finish = 0, grid_finish_pair = 0, grid_small = 0, grid_paths = 0;
     int32_t tail_paths = 0;             // live-path count below which the fused finish kernel takes over
     bool pair_tail = false;             // the tail runs two lanes per path (finish_pair_kernel)
-    bool fused = false;                 // four-wide tree and shaded view: render_paths_kernel where the image's size suits it
+    bool fused = false;                 // four-wide tree and shaded view: the form goes by the image's size (whole, tail_alone)
     bool small = false;                 // the scene fits render_small_kernel and the view is shaded
     DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lanes;
     RenderBuffers buf{};
@@ -575,7 +574,7 @@ struct pt_renderer {
     void lane_buffers() {
         path_buffers();
         if (buf.claims) return;
-        const size_t l = size_t(grid_paths) * kPathsBlock, claimed = size_t(pixels) * sizeof(int32_t);
+        const size_t l = size_t(lane_count()), claimed = size_t(pixels) * sizeof(int32_t);
         lanes.resize(l * (sizeof(PathState) + sizeof(ShadowRay)) + claimed);
         unsigned char *at = lanes.get<unsigned char>();
         buf.lane_paths = reinterpret_cast<PathState *>(at);
@@ -593,16 +592,20 @@ struct pt_renderer {
         buf.hits = hits.get<PathHit>(); buf.stats = stats.get<uint2>(); buf.shadows = shadows.get<ShadowRay>();
         buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
     }
-    // One kernel for the whole render (render_paths_kernel) where every resident lane has a pixel: with
-    // fewer, the tail kernel's two lanes per path are faster (wavefront and this, 240x150, 16 spp: 3.7 and 5.0 ms;
-    // 320x240 6.7 and 6.3), except for one or two samples, where the wavefront's launches are most of the time
-    // (240x150: 0.88 and 0.47).  Up to 40 pixels per lane: from there on the wavefront's queues are long enough
-    // to hide their slowest rays and its walk kernels hold more warps (1920x1080 30.4 and 27.0; with four
-    // blocks per SM 3840x2160 91.8 and 111.8).
-    bool whole(int count) const {
-        const int64_t l = int64_t(grid_paths) * kPathsBlock;
-        return fused && pixels <= 40 * l && (pixels >= l || count <= 2);
-    }
+    // Which kernels render an image of a four-wide scene in the shaded view, unless pt_renderer_tuning asked
+    // for the wavefront.  Up to two pixels per lane of render_paths_kernel: the tail kernel alone, whose two
+    // lanes per path walk extension and shadow rays side by side.  Up to forty: render_paths_kernel.  From
+    // there on the wavefront: its queues are long enough to hide their slowest rays and its walk kernels
+    // hold more warps.  Milliseconds a call (tail kernel alone, render_paths_kernel, wavefront with tail; 1M
+    // triangles, 12 spp, bounce limit 8): 64,000 pixels 3.4, -, 5.0; 99,000 4.1, 5.3, -; 144,000 5.1, 5.5, 6.6;
+    // 256,000 7.3, 5.2, -; on 10,000 triangles 64,000 pixels 0.64, -, 1.2; 144,000 1.1, 1.4, -; 256,000 1.4, 1.7, -.
+    // Large images, 16 spp: 1920x1080 -, 27.0, 30.4; 3840x2160 -, 111.8 (four blocks per SM), 91.8.
+    int64_t lane_count() const { return int64_t(grid_paths) * kPathsBlock; }
+    bool whole() const { return fused && pixels > 2 * lane_count() && pixels <= 40 * lane_count(); }
+    // An image below the tail's length has no wavefront to run first either (1.2 and 0.6 ms for 52,000 pixels of 12
+    // samples on 10,000 triangles).
+    bool tail_alone() const { return (pair_kernel() && pixels < tail_paths) || (fused && pixels <= 2 * lane_count()); }
+    bool pair_kernel() const { return pair_tail && !params.brute && params.debug != PT_DEBUG_BVH && params.debug != PT_DEBUG_INTERSECTIONS; }
     void grids() {
         grid_extend = occupancy_grid((const void *)extend_kernel, block, stack_bytes(block));
         grid_shade = occupancy_grid((const void *)shade_kernel, block);
@@ -680,7 +683,8 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
             r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
             if (!r->small) {                             // what the first call will most likely use
-                if (r->whole(3)) r->lane_buffers();
+                if (r->whole()) r->lane_buffers();
+                else if (r->tail_alone()) r->path_buffers();
                 else r->wavefront_buffers();
             }
         } catch (...) { delete r; throw; }
@@ -713,8 +717,9 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         if (count <= 0 || count > INT32_MAX - r->samples) throw Error(PT_INVALID_ARGUMENT, "invalid accumulated sample count");
         const DeviceScene &scene = r->scene->view;
         cudaStream_t st = r->stream;
-        const bool whole = !r->small && r->whole(count);
+        const bool whole = !r->small && r->whole(), tail_alone = !r->small && !whole && r->tail_alone();
         if (whole) r->lane_buffers();
+        else if (tail_alone) r->path_buffers();
         else if (!r->small) r->wavefront_buffers();
         PT_CUDA(cudaMemsetAsync(r->buf.rays, 0, sizeof(unsigned long long), st));
         PT_CUDA(cudaEventRecord(r->start.get(), st));
@@ -726,15 +731,11 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         } else if (whole) {
             PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
             PT_CUDA(cudaMemsetAsync(r->buf.counters, 0, sizeof(int32_t), st));
-            const bool hand_over = count > 2;
-            const int blocks = std::min(r->grid_paths, (r->pixels + 31) / 32);
-            render_paths_kernel<<<blocks, kPathsBlock, stack_bytes(kPathsBlock), st>>>(scene, r->params, r->buf, r->pixels, count, hand_over);
+            render_paths_kernel<<<r->grid_paths, kPathsBlock, stack_bytes(kPathsBlock), st>>>(scene, r->params, r->buf, r->pixels, count);
             PT_CUDA(cudaGetLastError());
-            if (hand_over) {
-                PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
-                finish_pair_kernel<<<r->grid_finish_pair, r->block, 0, st>>>(scene, r->params, r->buf, 0);
-                PT_CUDA(cudaGetLastError());
-            }
+            PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
+            finish_pair_kernel<<<r->grid_finish_pair, r->block, 0, st>>>(scene, r->params, r->buf, 0);
+            PT_CUDA(cudaGetLastError());
         } else {
             start_samples<<<(r->pixels + 255) / 256, 256, 0, st>>>(r->params, r->buf, r->pixels, count);
             PT_CUDA(cudaGetLastError());
@@ -747,7 +748,7 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         const int64_t max_iterations = int64_t(count) * (int64_t(r->params.max_depth) + 1) + 1;
         int parity = 0;
         int64_t issued = 0, checked = 0;
-        bool done = r->small || whole, tail = false;
+        bool done = r->small || whole, tail = tail_alone;
         while (!done && !tail && issued < max_iterations) {
             extend_kernel<<<r->grid_extend, r->block, stack_bytes(r->block), st>>>(scene, r->params, r->buf, parity, g_query_config.min_active);
             if (issued > 0) PT_CUDA(cudaStreamWaitEvent(st, r->shadowed[parity ^ 1].get(), 0));
@@ -778,7 +779,7 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         if (tail && !done) {
             // the few remaining paths (of the last issued iteration's queue) run to completion
             const RenderParams &q = r->params;
-            if (r->pair_tail && !q.brute && q.debug != PT_DEBUG_BVH && q.debug != PT_DEBUG_INTERSECTIONS) {
+            if (r->pair_kernel()) {
                 PT_CUDA(cudaMemsetAsync(&r->buf.fetch[3], 0, sizeof(unsigned long long), st));
                 finish_pair_kernel<<<r->grid_finish_pair, r->block, 0, st>>>(scene, q, r->buf, parity);
             } else

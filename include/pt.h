@@ -246,8 +246,8 @@ pt_status pt_set_block_shape(pt_renderer *renderer, int width, int height);
  * completion in one fused kernel (two threads per path on four-wide trees: one walks the path's
  * next ray while the other walks its last shadow ray; default max(65536, pixels/4); 0 keeps the
  * wavefront to the end).  Until this is called, shaded renders of scenes of at most 32 primitives, and
- * of images that give every resident GPU thread one to forty pixels, run as one kernel from the first
- * camera ray to the last bounce; calling it asks for the wavefront.  Results do not depend on it. */
+ * of images of two to forty pixels per resident GPU thread, run as one kernel from the first camera ray to
+ * the last bounce, and smaller images in the two-threads-per-path kernel alone; calling it asks for the wavefront.  Results do not depend on it. */
 pt_status pt_renderer_tuning(pt_renderer *renderer, int32_t tail_paths);
 /* Linear FP32 radiance sums (3 floats per pixel, row 0 at the bottom, not divided by spp). */
 pt_status pt_get_sums(const pt_renderer *renderer, float *rgb_sums, size_t floats);
@@ -286,9 +286,9 @@ pt_status pt_batch_get_sums(const pt_batch *batch, int32_t job, float *rgb_sums,
 pt_status pt_batch_stats(const pt_batch *batch, float *kernel_ms, uint64_t *rays, double *job_completion_ms, size_t jobs);
 /* path_capacity: path slots (0 = min(pixels, 2^22)); block: 64, 128 or 256 threads; min_active:
  * traversal refill threshold; tail_paths: live paths below which the fused kernel finishes;
- * use_graph: 1 = the loop runs on the device (one graph launch; or, on four-wide nodes, with one to
- * forty pixels per resident GPU thread and a slot for each such thread, one kernel that walks and
- * shades, which takes no block or refill setting), 0 = host-driven loop. */
+ * use_graph: 1 = the loop runs on the device (one graph launch; or, on four-wide nodes, with up to
+ * two pixels per resident GPU thread and a slot for each pixel the fused kernel alone, and with two to
+ * forty and a slot for each thread one kernel that walks and shades; these take no block or refill setting), 0 = host-driven loop. */
 pt_status pt_batch_tuning(pt_batch *batch, int32_t path_capacity, int32_t block, int32_t min_active, int32_t tail_paths,
                           int32_t use_graph);
 /* Node fetch width of the batch's walks: 1 = four-wide nodes (default), 0 = the two-wide layout.
@@ -365,8 +365,8 @@ typedef struct pt_cached_params {
     float learning_rate;        /* Adam learning rate (1e-2; beta 0.9 / 0.99) */
     uint64_t network_seed;      /* weight initialisation */
     int32_t tail_paths;         /* live paths below which one fused kernel ends the frame's tail
-                                 * (0: max(16384, pixels / 16), and frames of one to some twenty pixels per
-                                 * resident GPU thread run as one kernel instead; the image is the same) */
+                                 * (0: max(16384, pixels / 16), and frames of up to some twenty pixels per
+                                 * resident GPU thread run without the wavefront; the image is the same) */
     int32_t query_specular;     /* 1 (default): paths may also end at metal and glass vertices;
                                  * 0: at diffuse vertices only */
     float weight_average;       /* decay of the weight average queries use (0.99; 0: the live weights) */
