@@ -309,7 +309,10 @@ struct Sync {
 // A whole tile's queries (6656 bytes) come by one bulk copy, issued once the tile before has been
 // encoded, so the encode reads shared memory (13 words a row: no bank conflicts) instead of waiting for 13
 // strided global loads; a partial tile, or queries not 16-byte aligned, are read directly (2^21 queries
-// 133.5 -> 130.7 us: the chain of the layers is what is left).
+// 133.5 -> 130.7 us: the chain of the layers is what is left).  The weights and the first tile come by bulk copies
+// that run beside the TMEM allocation and the first encode, and consecutive tiles go to different CTAs, so a
+// call of few tiles has an SM's issue slots for each (calls back to back, CTA after CTA filled with eight tiles
+// and this: 1,000 queries 14.5 -> 8.4 us, 65,536 15.1 -> 12.5, 211,598 23.8 -> 20.7, 2^21 120.3 -> 115.2).
 // smem: header (Scratch, then the groups' MMA and copy mbarriers from byte 128) | W | (act | queries) x G.
 // One CTA of eight groups per SM: eight tiles in flight (32 warps at 64 registers), all 512
 // TMEM columns, 222 KB of shared memory.
@@ -319,7 +322,7 @@ constexpr int kFwdCtasPerSm = 1;
 constexpr uint32_t kFwdTmemCols = 512;    // power of two >= 64 * kFwdGroups
 constexpr int kFwdQueryBytes = kTile * int(sizeof(pt_cache_query));   // a tile's queries, 6656 bytes
 constexpr size_t kFwdSmem = 256 + kWeightBytes + kFwdGroups * (kActBytes + kFwdQueryBytes);
-static_assert(kFwdQueryBytes % 16 == 0 && kFwdSmem <= 232448, "bulk copies and shared memory");
+static_assert(kFwdQueryBytes % 16 == 0 && kWeightBytes % 16 == 0 && kFwdSmem <= 232448, "bulk copies and shared memory");
 static_assert(64 * kFwdGroups <= kFwdTmemCols && kFwdCtasPerSm * kFwdTmemCols <= 512, "TMEM budget");
 static_assert(128 + 16 * kFwdGroups <= 256 && kFwdGroups < 16, "header and named-barrier budget");
 
@@ -346,17 +349,36 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtasPerSm) forward_kernel(con
     unsigned char *act = w + kWeightBytes + size_t(g) * (kActBytes + kFwdQueryBytes);
     unsigned char *staged = act + kActBytes;                       // the tile's queries
     const float3 ie = make_float3(1.0f / fmaxf(hi.x - lo.x, 1e-30f), 1.0f / fmaxf(hi.y - lo.y, 1e-30f), 1.0f / fmaxf(hi.z - lo.z, 1e-30f));
-    if (threadIdx.x < 2 * kFwdGroups) bar_init(&bars[threadIdx.x]);   // the groups' MMA barriers, then their copy barriers
+    const bool issuer = r == 0;
+    const uint32_t tiles = uint32_t((count + kTile - 1) / kTile);   // < 2^32: 2^39 queries would not fit in memory
+    const uint32_t stride = gridDim.x * kFwdGroups, first = g * gridDim.x + blockIdx.x;
+    // whole tiles of 16-byte aligned queries come by bulk copy, the next one while this one's layers run
+    const uint32_t whole = (reinterpret_cast<uintptr_t>(queries) & 15) ? 0 : uint32_t(count / kTile);
+    uint64_t *copy_bar = &bars[kFwdGroups + g], *weights_bar = &h->bar;
+    uint32_t copy_phase = 0;
+    bool in_flight = false;                       // a copy was issued and not yet waited for
+    auto fetch = [&](uint32_t t) {
+        if (t >= whole) return;
+        if (issuer) bulk_load(staged, queries + size_t(t) * kTile, kFwdQueryBytes, copy_bar);
+        in_flight = true;
+    };
+    // the weights and each group's first tile are on their way before anything else; each issuer sets up the
+    // barriers its own copies and MMAs complete
+    if (issuer) {
+        bar_init(&bars[g]);
+        bar_init(copy_bar);
+        if (g == 0) bar_init(weights_bar);
+        fence_async_smem();
+        if (g == 0) bulk_load(w, weights, kWeightBytes, weights_bar);
+    }
+    if (first < tiles) fetch(first);
     tmem_alloc(h, kFwdTmemCols);
-    load_weights(w, weights);
-    fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tcol = h->tmem + 64u * uint32_t(g);
     const uint32_t lane_col = tcol + ((uint32_t)((r & ~31u)) << 16);   // warp (w % 4) reads lanes 32 (w % 4) ..
     uint64_t *bar = &bars[g];
-    const bool issuer = r == 0;
     uint32_t phase = 0, pending_phase = 0;
     bool ok = true, pending = false;
     auto wait_mma = [&]() {                       // commit this group's MMAs and wait for them (bounded)
@@ -374,20 +396,7 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtasPerSm) forward_kernel(con
         fence_after();
         return all;
     };
-    const uint32_t tiles = uint32_t((count + kTile - 1) / kTile);   // < 2^32: 2^39 queries would not fit in memory
-    const uint32_t stride = gridDim.x * kFwdGroups;
-    // whole tiles of 16-byte aligned queries come by bulk copy, the next one while this one's layers run
-    const uint32_t whole = (reinterpret_cast<uintptr_t>(queries) & 15) ? 0 : uint32_t(count / kTile);
-    uint64_t *copy_bar = &bars[kFwdGroups + g];
-    uint32_t copy_phase = 0;
-    bool in_flight = false;                       // a copy was issued and not yet waited for
-    auto fetch = [&](uint32_t t) {
-        if (t >= whole) return;
-        if (issuer) bulk_load(staged, queries + size_t(t) * kTile, kFwdQueryBytes, copy_bar);
-        in_flight = true;
-    };
-    fetch(blockIdx.x * kFwdGroups + g);
-    for (uint32_t t = blockIdx.x * kFwdGroups + g; t < tiles && ok; t += stride) {
+    for (uint32_t t = first; t < tiles && ok; t += stride) {
         bool here = true;
         if (t < whole) {
             here = bar_wait(copy_bar, copy_phase, attempts);
@@ -400,6 +409,7 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtasPerSm) forward_kernel(con
         } else {
             encode_tile(act, queries, size_t(t) * kTile, count, lo, ie, r);
         }
+        if (t < stride) here = bar_wait(weights_bar, 0, attempts) && here;
         ok = sync_group(here);
         if (!ok) break;
         fetch(t + stride);                        // every thread has read its staged query
@@ -430,6 +440,7 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtasPerSm) forward_kernel(con
     if (!ok && r == 0) atomicExch(status, int(PT_TIMEOUT));
     if (pending) bar_wait(bar, pending_phase, kSpinLimit);   // no MMA of this group may still write TMEM
     if (in_flight) bar_wait(copy_bar, copy_phase, kSpinLimit);   // nor a copy shared memory
+    if (g == 0) bar_wait(weights_bar, 0, kSpinLimit);
     fence_before();
     __syncthreads();
     tmem_free(h->tmem, kFwdTmemCols);
@@ -782,7 +793,7 @@ void cache_bounds(const pt_cache *c, float lo[3], float hi[3]) {
 void cache_forward(pt_cache *c, const pt_cache_query *queries, size_t count, const int32_t *count_dev, float *rgb, cudaStream_t st) {
     size_t tiles = (count + kTile - 1) / kTile;
     if (!tiles) return;
-    int grid = int(std::min<size_t>((tiles + kFwdGroups - 1) / kFwdGroups, size_t(kFwdCtasPerSm) * size_t(c->ctas)));
+    int grid = int(std::min<size_t>(tiles, size_t(kFwdCtasPerSm) * size_t(c->ctas)));
     forward_kernel<<<grid, kFwdThreads, kFwdSmem, st>>>(c->inference(), queries, count, count_dev, lo3(c), hi3(c), rgb,
                                                    c->status.get<int>(), c->attempts);
     PT_CUDA(cudaGetLastError());

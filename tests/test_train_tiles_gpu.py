@@ -31,7 +31,8 @@ def test_gradients_match_oracle_at_tile_edges(n):
     assert again[0] == loss and np.array_equal(again[1], g)
 
 
-@pytest.mark.parametrize("n", [1, 127, 128, 129, 1024, 1025, 148 * 8 * 128, 148 * 8 * 128 * 2 + 77])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1024, 1025, 148 * 128, 148 * 128 + 1, 148 * 7 * 128 + 5, 148 * 8 * 128,
+                               148 * 8 * 128 * 2 + 77])
 def test_forward_at_tile_edges_and_unaligned_queries(n):
     """Whole tiles come by bulk copy, partial tiles and queries off a 16-byte boundary by plain loads: the same bits
     wherever a query lies, nothing written past the last one, and the oracle's values."""
