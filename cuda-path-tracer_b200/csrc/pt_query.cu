@@ -598,6 +598,7 @@ static void query_pageable(pt_scene *scene, const pt_ray *rays, size_t count, in
         if(tmax) w.tmax.reserve(chunk * sizeof(float));
         if(stats) w.stats.reserve(chunk * sizeof(pt_ray_stats));
         StageChunk pinned;
+        DrainOnError drain{w.stream};
         unsigned char *via = pinned.get();
         for(size_t c = next++; c < chunks; c = next++) {
             const size_t b = c * chunk, n = std::min(chunk, count - b);
@@ -685,6 +686,7 @@ pt_status pt_query_rays_compat(const pt_scene *scene, const pt_ray *rays, size_t
             w.rays.reserve(chunk * sizeof(pt_ray));
             w.hits.reserve(chunk * sizeof(pt_trace_result));
             StageChunk pinned;
+            DrainOnError drain{w.stream};
             unsigned char *via = pinned.get();
             for(size_t c = next++; c < chunks; c = next++) {
                 const size_t b = c * chunk, n = std::min(chunk, count - b);

@@ -32,6 +32,13 @@ private:
     void *ptr_ = nullptr;
 };
 
+// A copy under way when an error leaves a worker's loop ends before its chunk goes back to the pool.
+struct DrainOnError {
+    cudaStream_t stream;
+    int entered = std::uncaught_exceptions();
+    ~DrainOnError() { if(std::uncaught_exceptions() > entered) cudaStreamSynchronize(stream); }
+};
+
 bool pageable(const void *host);                  // not pinned, managed or device memory
 // Threads worth starting for this many parts and bytes copied either way: one per 2 MiB (1.5M rays, 66 MB: 8
 // threads 3.6 ms, 4 4.0, 2 5.5; 100,000 full records, 8.4 MB: 4 threads 1.15 ms, 8 1.37, 1 1.55).
