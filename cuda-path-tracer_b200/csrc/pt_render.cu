@@ -598,7 +598,8 @@ struct pt_renderer {
     // there on the wavefront: its queues are long enough to hide their slowest rays and its walk kernels
     // hold more warps.  Milliseconds a call (tail kernel alone, render_paths_kernel, wavefront with tail; 1M
     // triangles, 12 spp, bounce limit 8): 64,000 pixels 3.4, -, 5.0; 99,000 4.1, 5.3, -; 144,000 5.1, 5.5, 6.6;
-    // 256,000 7.3, 5.2, -; on 10,000 triangles 64,000 pixels 0.64, -, 1.2; 144,000 1.1, 1.4, -; 256,000 1.4, 1.7, -.
+    // 187,000 6.4, 5.9, -; 256,000 7.3, 5.2, -; on 10,000 triangles 64,000 pixels 0.64, -, 1.2; 144,000 1.1, 1.4, -;
+    // 187,000 1.3, 1.65, -; 256,000 1.4, 1.7, -.
     // Large images, 16 spp: 1920x1080 -, 27.0, 30.4; 3840x2160 -, 111.8 (four blocks per SM), 91.8.
     int64_t lane_count() const { return int64_t(grid_paths) * kPathsBlock; }
     bool whole() const { return fused && pixels > 2 * lane_count() && pixels <= 40 * lane_count(); }
