@@ -534,7 +534,7 @@ struct pt_batch {
             buf.lane_shadows = reinterpret_cast<ShadowRay *>(at); at += handed * sizeof(ShadowRay);
             buf.claims = reinterpret_cast<int32_t *>(at); at += per_pixel;
             buf.done = reinterpret_cast<int32_t *>(at);
-            PT_CUDA(cudaMemset(buf.claims, 0, per_pixel));
+            PT_CUDA(cudaMemsetAsync(buf.claims, 0, per_pixel, stream));   // on the runs' stream: the default stream may be behind it
         }
         drop_graph();
     }
