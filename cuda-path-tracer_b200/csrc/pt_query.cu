@@ -634,8 +634,10 @@ pt_status pt_query_rays(const pt_scene *cscene, const pt_ray *rays, size_t count
         if(mode != PT_QUERY_CLOSEST && mode != PT_QUERY_ANY) throw Error(PT_INVALID_ARGUMENT, "unknown query mode");
         if(!count) return;
         std::lock_guard<std::mutex> lock(scene->work_mutex);   // the staging buffers are the scene's
-        // (the walk timing of pt_query_profile counts launches in the caller's order: it keeps the single thread)
-        if(count >= kStagedMin && scene->profile_events.empty() && (pageable(rays) || pageable(hits))) {
+        // (the walk timing of pt_query_profile counts launches in the caller's order: it keeps the single thread;
+        // the workers touch the arrays themselves, so a device pointer among them is left to the copies below)
+        if(count >= kStagedMin && scene->profile_events.empty() && (pageable(rays) || pageable(hits)) && on_host(rays) &&
+           on_host(hits) && (!tmax || on_host(tmax)) && (!stats || on_host(stats))) {
             query_pageable(scene, rays, count, mode, tmin, tmax, hits, stats);
             return;
         }
@@ -679,6 +681,7 @@ pt_status pt_query_rays_compat(const pt_scene *scene, const pt_ray *rays, size_t
         // its device buffers: 100,000 rays took 2.6 ms for a kernel of 0.12)
         const size_t chunk = std::min(staged_chunk(count, sizeof(pt_trace_result)), (count + 31) & ~size_t(31));
         const size_t chunks = (count + chunk - 1) / chunk;
+        const bool touch = on_host(rays) && on_host(results);   // otherwise the copies answer for a device pointer
         std::atomic<size_t> next{0};
         run_workers(stage_workers(chunks, count * (sizeof(pt_ray) + sizeof(pt_trace_result))), m->device, [&](int k) {
             auto &w = m->workers[k];
@@ -687,7 +690,7 @@ pt_status pt_query_rays_compat(const pt_scene *scene, const pt_ray *rays, size_t
             w.hits.reserve(chunk * sizeof(pt_trace_result));
             StageChunk pinned;
             DrainOnError drain{w.stream};
-            unsigned char *via = pinned.get();
+            unsigned char *via = touch ? pinned.get() : nullptr;
             for(size_t c = next++; c < chunks; c = next++) {
                 const size_t b = c * chunk, n = std::min(chunk, count - b);
                 if(via) std::memcpy(via, rays + b, n * sizeof(pt_ray));

@@ -37,11 +37,15 @@ StageChunk::~StageChunk() {
     else { cudaFreeHost(ptr_); g_chunks--; }
 }
 
-bool pageable(const void *host) {
+namespace {
+cudaMemoryType memory_type(const void *p) {
     cudaPointerAttributes a{};
-    if(cudaPointerGetAttributes(&a, host) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeUnregistered;
+    if(cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return cudaMemoryTypeDevice; }
+    return a.type;
 }
+} // namespace
+bool pageable(const void *p) { return memory_type(p) == cudaMemoryTypeUnregistered; }
+bool on_host(const void *p) { return memory_type(p) != cudaMemoryTypeDevice; }
 
 int stage_workers(size_t parts, size_t bytes) {
     const size_t cores = std::max(1u, std::thread::hardware_concurrency());

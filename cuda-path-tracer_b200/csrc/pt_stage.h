@@ -39,7 +39,8 @@ struct DrainOnError {
     ~DrainOnError() { if(std::uncaught_exceptions() > entered) cudaStreamSynchronize(stream); }
 };
 
-bool pageable(const void *host);                  // not pinned, managed or device memory
+bool pageable(const void *p);                     // not pinned, managed or device memory
+bool on_host(const void *p);                      // the host can read and write it: not device memory
 // Threads worth starting for this many parts and bytes copied either way: one per 2 MiB (1.5M rays, 66 MB: 8
 // threads 3.6 ms, 4 4.0, 2 5.5; 100,000 full records, 8.4 MB: 4 threads 1.15 ms, 8 1.37, 1 1.55).
 int stage_workers(size_t parts, size_t bytes);
