@@ -586,6 +586,11 @@ static size_t staged_chunk(size_t count, size_t bytes_per_ray) {
     const size_t most = kStageChunk / bytes_per_ray & ~size_t(1023), share = (count / (2 * kStageWorkers) + 1023) & ~size_t(1023);
     return std::min(most, std::max<size_t>(share, 8192));
 }
+// whether two arrays share memory (a null one does not)
+static bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x && y && x < y + b_bytes && y < x + a_bytes;
+}
 static void query_pageable(pt_scene *scene, const pt_ray *rays, size_t count, int mode, float tmin, const float *tmax, pt_hit *hits,
                            pt_ray_stats *stats) {
     const size_t chunk = staged_chunk(count, sizeof(pt_ray) + sizeof(float)), chunks = (count + chunk - 1) / chunk;
@@ -635,9 +640,14 @@ pt_status pt_query_rays(const pt_scene *cscene, const pt_ray *rays, size_t count
         if(!count) return;
         std::lock_guard<std::mutex> lock(scene->work_mutex);   // the staging buffers are the scene's
         // (the walk timing of pt_query_profile counts launches in the caller's order: it keeps the single thread;
-        // the workers touch the arrays themselves, so a device pointer among them is left to the copies below)
+        // the workers touch the arrays themselves and in no order, so a device pointer among them and answers written
+        // over the rays are left to the copies below)
+        auto shared = [&](const void *in, size_t bytes) {
+            return overlap(in, bytes, hits, count * sizeof(pt_hit)) || overlap(in, bytes, stats, count * sizeof(pt_ray_stats));
+        };
         if(count >= kStagedMin && scene->profile_events.empty() && (pageable(rays) || pageable(hits)) && on_host(rays) &&
-           on_host(hits) && (!tmax || on_host(tmax)) && (!stats || on_host(stats))) {
+           on_host(hits) && (!tmax || on_host(tmax)) && (!stats || on_host(stats)) && !shared(rays, count * sizeof(pt_ray)) &&
+           !shared(tmax, count * sizeof(float))) {
             query_pageable(scene, rays, count, mode, tmin, tmax, hits, stats);
             return;
         }
@@ -677,11 +687,22 @@ pt_status pt_query_rays_compat(const pt_scene *scene, const pt_ray *rays, size_t
         if(count > size_t(INT32_MAX)) throw Error(PT_INVALID_ARGUMENT, "too many validation rays");
         pt_scene *m = const_cast<pt_scene *>(scene);
         std::lock_guard<std::mutex> lock(m->work_mutex);
+        // worker threads would write answers over rays not yet read, and cannot read device memory: whole copies then
+        // (which answer for a device pointer)
+        if(!on_host(rays) || !on_host(results) || overlap(rays, count * sizeof(pt_ray), results, count * sizeof(pt_trace_result))) {
+            DeviceBuffer in(count * sizeof(pt_ray)), out(count * sizeof(pt_trace_result));
+            PT_CUDA(cudaMemcpy(in.get(), rays, count * sizeof(pt_ray), cudaMemcpyHostToDevice));
+            compat_kernel<<<grid_for(count, kQueryBlock), kQueryBlock>>>(scene->view, scene->brute_order.get<int32_t>(), scene->leaf_count,
+                                                                         in.get<pt_ray>(), count, brute, out.get<pt_trace_result>());
+            PT_CUDA(cudaGetLastError());
+            PT_CUDA(cudaDeviceSynchronize());
+            PT_CUDA(cudaMemcpy(results, out.get(), count * sizeof(pt_trace_result), cudaMemcpyDeviceToHost));
+            return;
+        }
         // as query_pageable: worker threads, pinned chunks, the scene's workspaces (a call used to allocate and free
         // its device buffers: 100,000 rays took 2.6 ms for a kernel of 0.12)
         const size_t chunk = std::min(staged_chunk(count, sizeof(pt_trace_result)), (count + 31) & ~size_t(31));
         const size_t chunks = (count + chunk - 1) / chunk;
-        const bool touch = on_host(rays) && on_host(results);   // otherwise the copies answer for a device pointer
         std::atomic<size_t> next{0};
         run_workers(stage_workers(chunks, count * (sizeof(pt_ray) + sizeof(pt_trace_result))), m->device, [&](int k) {
             auto &w = m->workers[k];
@@ -690,7 +711,7 @@ pt_status pt_query_rays_compat(const pt_scene *scene, const pt_ray *rays, size_t
             w.hits.reserve(chunk * sizeof(pt_trace_result));
             StageChunk pinned;
             DrainOnError drain{w.stream};
-            unsigned char *via = touch ? pinned.get() : nullptr;
+            unsigned char *via = pinned.get();
             for(size_t c = next++; c < chunks; c = next++) {
                 const size_t b = c * chunk, n = std::min(chunk, count - b);
                 if(via) std::memcpy(via, rays + b, n * sizeof(pt_ray));

@@ -56,3 +56,19 @@ def test_device_pointers_give_the_copies_error(scene, count):
             assert (records if device_rays else on_device.cpu().numpy()).tobytes() == full.tobytes()
     hits, _ = dev.query(rays, tmax=tmax, stats=True)      # the scene is usable afterwards
     assert hits.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("count", [777, STAGED, 2 * STAGED])
+def test_answers_written_over_the_rays(scene, count):
+    """Hits over the rays they answer, and full records over their rays."""
+    cam, dev = scene
+    rays = pt.camera_rays(cam, 160, 100, 3, 0, count)
+    want = dev.query(rays)
+    memory = rays.view(np.uint8).copy()
+    assert query(dev, memory.ctypes.data, count, memory.ctypes.data) == 0
+    assert memory[:count * 16].tobytes() == want.tobytes()
+    full = dev.query_compat(rays).view(np.uint8).tobytes()
+    memory = np.zeros(count * RECORD, np.uint8)
+    memory[:count * 28] = rays.view(np.uint8)
+    assert compat(dev, memory.ctypes.data, count, memory.ctypes.data) == 0
+    assert memory.tobytes() == full
