@@ -701,6 +701,9 @@ pt_status pt_query_rays_compat(const pt_scene *scene, const pt_ray *rays, size_t
         }
         // as query_pageable: worker threads, pinned chunks, the scene's workspaces (a call used to allocate and free
         // its device buffers: 100,000 rays took 2.6 ms for a kernel of 0.12)
+        // Device work queued before the call may still be writing the rays (a pinned array) or reading the results; the
+        // copies on the default stream used to wait for it.
+        PT_CUDA(cudaDeviceSynchronize());
         const size_t chunk = std::min(staged_chunk(count, sizeof(pt_trace_result)), (count + 31) & ~size_t(31));
         const size_t chunks = (count + chunk - 1) / chunk;
         std::atomic<size_t> next{0};

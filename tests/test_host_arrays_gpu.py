@@ -72,3 +72,20 @@ def test_answers_written_over_the_rays(scene, count):
     memory[:count * 28] = rays.view(np.uint8)
     assert compat(dev, memory.ctypes.data, count, memory.ctypes.data) == 0
     assert memory.tobytes() == full
+
+
+@pytest.mark.parametrize("count", [1000, 100_003])
+def test_full_records_of_rays_still_being_copied(scene, count):
+    """Pinned rays that work queued on the default stream is still to write."""
+    import torch
+    cam, dev = scene
+    rays = pt.camera_rays(cam, 160, 100, 3, 0, count)
+    want = dev.query_compat(rays).view(np.uint8).tobytes()
+    on_device = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
+    pinned = torch.zeros(count * 28, dtype=torch.uint8, pin_memory=True)
+    results = np.zeros(count * RECORD, np.uint8)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(40_000_000)                        # about 20 ms
+    pinned.copy_(on_device, non_blocking=True)
+    assert compat(dev, pinned.data_ptr(), count, results.ctypes.data) == 0
+    assert results.tobytes() == want
