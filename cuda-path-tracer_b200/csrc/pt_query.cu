@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kQueryBlock) query_small_kernel(DeviceScene s,
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) {
         const pt_ray r = rays[i];
         HitInfo h;
-        const bool hit = small_walk(s, sh, r, tmin, tmax ? tmax[i] : FLT_MAX, tie, kAny, h);
+        const bool hit = small_walk<true>(s, sh, r, tmin, tmax ? tmax[i] : FLT_MAX, tie, kAny, h);
         int32_t type = PT_BRANCH, id = -1;
         if (hit) hit_ids(s, h.slot, type, id);
         reinterpret_cast<int4 *>(hits)[i] = make_int4(__float_as_int(hit ? h.t : 0.0f), id, type, 0);

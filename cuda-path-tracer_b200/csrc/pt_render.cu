@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene s
                     r.origin = pt_vec3{sr.ox, sr.oy, sr.oz};
                     r.direction = pt_vec3{sr.dx, sr.dy, sr.dz};
                 }
-                hit = small_walk(scene, sh, r, 0.001f, shadow_pass ? sr.tmax : FLT_MAX, kTieLastLeaf, shadow_pass, hi);
+                hit = small_walk<false>(scene, sh, r, 0.001f, shadow_pass ? sr.tmax : FLT_MAX, kTieLastLeaf, shadow_pass, hi);
                 if (shadow_pass && !hit) { s.rr = s.rr + sr.cr; s.rg = s.rg + sr.cg; s.rb = s.rb + sr.cb; }
             }
             __syncwarp();

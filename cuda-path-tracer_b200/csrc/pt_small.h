@@ -51,7 +51,12 @@ __device__ inline void small_load(const DeviceScene &s, SmallScene &sh, float pa
     __syncthreads();
 }
 
-// Closest hit (any = false) or any hit of one ray per lane; true when something was hit.
+// Closest hit (any = false) or any hit of one ray per lane; true when something was hit.  kFar (queries, whose rays
+// may start anywhere): the boxes are widened by the rounding of the slab arithmetic as well, eight units in the
+// last place of the origin's largest coordinate (2^-21), since far from the scene two planes of a box, padded or
+// not, round to the same distance and neighbouring axes to distances in the wrong order.  The primitives' own
+// tests decide, so a box too wide costs time only.
+template <bool kFar>
 __device__ __forceinline__ bool small_walk(const DeviceScene &s, const SmallScene &sh, const pt_ray &r, float tmin, float tmax,
                                            int tie, bool any, HitInfo &hit) {
     hit.slot = -1; hit.t = 0; hit.u = 0; hit.v = 0;
@@ -59,14 +64,27 @@ __device__ __forceinline__ bool small_walk(const DeviceScene &s, const SmallScen
     const f2x oxy = f2x_make(-rb.ox, -rb.oy), ozz = f2x_make(-rb.oz, -rb.oz);   // a - b and a + (-b) round alike
     const f2x ixy = f2x_make(rb.ix, rb.iy), izz = f2x_make(rb.iz, rb.iz);
     const int pattern = (rb.nx ? 1 : 0) | (rb.ny ? 2 : 0) | (rb.nz ? 4 : 0);
+    f2x out_xy = 0, in_xy = 0, out_in_z = 0;             // how much earlier a ray enters and later it leaves (kFar)
+    if constexpr (kFar) {
+        const float pad = fmaxf(fmaxf(fabsf(rb.ox), fabsf(rb.oy)), fabsf(rb.oz)) * 0x1p-21f;
+        auto reach = [&](float inverse) { return fabsf(inverse) <= FLT_MAX ? pad * fabsf(inverse) : 0.0f; };   // 0: parallel to the slab
+        const float x = reach(rb.ix), y = reach(rb.iy), z = reach(rb.iz);
+        out_xy = f2x_make(-x, -y); in_xy = f2x_make(x, y); out_in_z = f2x_make(-z, z);
+    }
     uint32_t passed = 0;
 #pragma unroll 4
     for (int k = 0; k < s.small_count; k++) {
         const ulonglong2 xy = sh.xy[k][pattern];
         float ax, ay, az, bx, by, bz;
-        f2x_split(f2x_mul(f2x_add(xy.x, oxy), ixy), ax, ay);
-        f2x_split(f2x_mul(f2x_add(xy.y, oxy), ixy), bx, by);
-        f2x_split(f2x_mul(f2x_add(sh.z[k][pattern], ozz), izz), az, bz);
+        if constexpr (kFar) {
+            f2x_split(f2x_fma(f2x_add(xy.x, oxy), ixy, out_xy), ax, ay);
+            f2x_split(f2x_fma(f2x_add(xy.y, oxy), ixy, in_xy), bx, by);
+            f2x_split(f2x_fma(f2x_add(sh.z[k][pattern], ozz), izz, out_in_z), az, bz);
+        } else {
+            f2x_split(f2x_mul(f2x_add(xy.x, oxy), ixy), ax, ay);
+            f2x_split(f2x_mul(f2x_add(xy.y, oxy), ixy), bx, by);
+            f2x_split(f2x_mul(f2x_add(sh.z[k][pattern], ozz), izz), az, bz);
+        }
         const float lo = fmaxf(max3(tmin, ax, ay), az), hi = fminf(min3(tmax, bx, by), bz);
         if (hi > lo) passed |= 1u << k;
     }
