@@ -473,6 +473,8 @@ struct pt_batch {
     // tuning (pt_batch_tuning / pt_batch_autotune)
     int32_t capacity = 0, block = 256, min_active = 16, tail_paths = 16384, use_graph = 1;
     int32_t wide = 1;                     // node fetch width: 1 four-wide nodes, 0 the two-wide layout
+    int32_t default_tail = 16384;         // the tail length pt_batch_create chose
+    bool loop = false;                    // a tail length was asked for (or the autotuner is timing the loop): no one-kernel form
     int32_t probe_fault_countdown = 0;   // > 0: that autotune probe run fails on the host (tests)
     int32_t slots = 0;
     BatchBuffers buf{};
@@ -572,6 +574,7 @@ struct pt_batch {
     int64_t lane_count() const { return int64_t(grid_paths()) * kPathsBlock; }
     bool one_kernel() const { return total_pixels > 2 * lane_count() && total_pixels <= 40 * lane_count() && slots >= lane_count(); }
     bool tail_alone() const { return total_pixels <= 2 * lane_count() && slots >= total_pixels; }
+    bool fused() const { return use_graph && wide && !loop; }
     unsigned long long max_iterations() const {
         // every pixel needs at most samples * (depth + 1) extends; slots run pixels back to back
         unsigned long long worst = 0;
@@ -622,8 +625,8 @@ struct pt_batch {
     }
     void run() {
         cudaStream_t st = stream;
-        const bool whole = use_graph && wide && buf.claims && one_kernel();
-        const bool alone = use_graph && wide && tail_alone();
+        const bool whole = fused() && buf.claims && one_kernel();
+        const bool alone = fused() && tail_alone();
         if (!whole && !alone) wavefront_buffers();
         int32_t njobs = int32_t(host_jobs.size());
         std::vector<int32_t> remaining(static_cast<size_t>(njobs));
@@ -850,7 +853,7 @@ pt_status pt_batch_create(const pt_scene_desc *scenes, int32_t scene_count, cons
             f.cursor = sc; f.rays = sc + 1; f.start_ns = sc + 2; f.iterations = sc + 3;
             f.job_remaining = b->job_remaining.get<int32_t>(); f.job_done_ns = b->job_done_ns.get<unsigned long long>();
             f.error = b->error.get<int32_t>();
-            b->tail_paths = int32_t(std::max<int64_t>(16384, offset / 64));
+            b->tail_paths = b->default_tail = int32_t(std::max<int64_t>(16384, offset / 64));
             PT_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
             PT_CUDA(cudaStreamCreateWithFlags(&b->shadow_stream, cudaStreamNonBlocking));
             b->allocate_slots();
@@ -870,6 +873,7 @@ pt_status pt_batch_tuning(pt_batch *b, int32_t path_capacity, int32_t block, int
         if (block != b->block || min_active != b->min_active || tail_paths != b->tail_paths || use_graph != b->use_graph) b->drop_graph();
         b->capacity = path_capacity; b->block = block; b->min_active = min_active; b->tail_paths = tail_paths;
         b->use_graph = use_graph ? 1 : 0;
+        b->loop = tail_paths != 16384 && tail_paths != b->default_tail;
         if (realloc) b->allocate_slots();
     });
 }
@@ -917,9 +921,10 @@ pt_status pt_batch_fail_probe(pt_batch *b, int32_t n) {
     });
 }
 
-// Autotuner: times probe runs (every job at min(probe_samples, its samples)) over path-pool
-// capacity, block size, refill threshold and graph/host loop, then the other node fetch width at
-// the fastest of those, keeps the fastest, and caches it per (log2 triangles, log2 pixels) bucket
+// Autotuner: times probe runs (every job at min(probe_samples, its samples)) of the loop over path-pool
+// capacity, block size, refill threshold and graph/host loop, then, unless a tail length asked for the
+// loop, the one-kernel form that use_graph = 1 stands for at the batch's size, then the other node fetch
+// width at the fastest of those, keeps the fastest, and caches it per (log2 triangles, log2 pixels) bucket
 // in a text file (one "bucket capacity block min_active use_graph node_width ms" line per bucket).
 // With a cached entry for the bucket the sweep is skipped.
 pt_status pt_batch_autotune(pt_batch *b, int32_t probe_samples, const char *cache_path, int32_t *best) {
@@ -949,11 +954,13 @@ pt_status pt_batch_autotune(pt_batch *b, int32_t probe_samples, const char *cach
             struct Restore {
                 pt_batch *b;
                 std::vector<BatchJob> saved;
+                bool loop;
                 ~Restore() {
+                    b->loop = loop;
                     b->host_jobs = saved;
                     try { b->jobs.upload(b->host_jobs); } catch (...) {}
                 }
-            } restore{b, b->host_jobs};
+            } restore{b, b->host_jobs, b->loop};
             if (!b->wide) { b->wide = 1; b->drop_graph(); }   // the sweep runs on four-wide nodes
             for (auto &j : b->host_jobs) j.samples = std::min(j.samples, probe_samples);
             b->jobs.upload(b->host_jobs);
@@ -965,6 +972,7 @@ pt_status pt_batch_autotune(pt_batch *b, int32_t probe_samples, const char *cach
             for (int32_t cap : caps) for (int32_t blk : blocks) for (int32_t act : actives) for (int32_t graph : {1, 0}) {
                 pt_status st = pt_batch_tuning(b, cap, blk, act, b->tail_paths, graph);
                 if (st != PT_OK) continue;
+                b->loop = true;                              // the settings are the loop's
                 try {
                     if (b->probe_fault_countdown > 0 && --b->probe_fault_countdown == 0)
                         throw Error(PT_TIMEOUT, "probe run failed (injected on the host)");
@@ -977,6 +985,12 @@ pt_status pt_batch_autotune(pt_batch *b, int32_t probe_samples, const char *cach
                 if (b->milliseconds < best_ms) { best_ms = b->milliseconds; cfg[0] = cap; cfg[1] = blk; cfg[2] = act; cfg[3] = graph; }
             }
             if (best_ms == 1e30) throw Error(PT_INVALID_ARGUMENT, "every autotune setting failed: " + failure);
+            if (!restore.loop && pt_batch_tuning(b, cfg[0], cfg[1], cfg[2], b->tail_paths, 1) == PT_OK && (b->one_kernel() || b->tail_alone())) {
+                try {
+                    b->run();
+                    if (b->milliseconds < best_ms) { best_ms = b->milliseconds; cfg[3] = 1; }
+                } catch (const Error &e) { if (e.status == PT_CUDA_ERROR) throw; }
+            }
             // node fetch width at the best setting: the four-wide nodes against the two-wide layout
             for (int32_t w : {0, 1}) {
                 if (w == cfg[4]) continue;

@@ -285,10 +285,12 @@ pt_status pt_batch_get_sums(const pt_batch *batch, int32_t job, float *rgb_sums,
 /* Device time of the last run, rays traced, and each job's completion time from the run's start. */
 pt_status pt_batch_stats(const pt_batch *batch, float *kernel_ms, uint64_t *rays, double *job_completion_ms, size_t jobs);
 /* path_capacity: path slots (0 = min(pixels, 2^22)); block: 64, 128 or 256 threads; min_active:
- * traversal refill threshold; tail_paths: live paths below which the fused kernel finishes;
- * use_graph: 1 = the loop runs on the device (one graph launch; or, on four-wide nodes, with up to
- * two pixels per resident GPU thread and a slot for each pixel the fused kernel alone, and with two to
- * forty and a slot for each thread one kernel that walks and shades; these take no block or refill setting), 0 = host-driven loop. */
+ * traversal refill threshold; tail_paths: live paths below which the fused kernel finishes (16384, and
+ * what the batch starts with, max(16384, pixels / 64), leave the form to the batch's size; any other
+ * value asks for the loop); use_graph: 1 = the loop runs on the device (one graph launch; or, on
+ * four-wide nodes, with up to two pixels per resident GPU thread and a slot for each pixel the fused
+ * kernel alone, and with two to forty and a slot for each thread one kernel that walks and shades; these
+ * take no block, refill or tail setting), 0 = host-driven loop. */
 pt_status pt_batch_tuning(pt_batch *batch, int32_t path_capacity, int32_t block, int32_t min_active, int32_t tail_paths,
                           int32_t use_graph);
 /* Node fetch width of the batch's walks: 1 = four-wide nodes (default), 0 = the two-wide layout.
