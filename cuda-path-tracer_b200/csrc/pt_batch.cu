@@ -18,6 +18,7 @@
 #include <string>
 #include <vector>
 #include "pt_api_common.h"
+#include "pt_batch_plan.h"
 #include "pt_device.h"
 #include "pt_paths.h"
 
@@ -63,6 +64,10 @@ struct BatchBuffers {
     ShadowRay *lane_shadows;
     int32_t *claims;                  // per pixel: samples drawn and not yet run (batch_paths; zero between runs)
     int32_t *done;                    // per pixel: samples run by batch_paths
+    const BatchLevel *levels;         // batch_paths' order of samples (pt_batch_plan.h)
+    const int32_t *sorted_jobs;
+    const uint32_t *sorted_first;
+    int32_t level_count;
 };
 
 __device__ inline unsigned long long globaltimer() {
@@ -357,9 +362,8 @@ __global__ void __launch_bounds__(256, 2) batch_finish_pair(DeviceScene scene, B
 }
 
 // The whole batch in one kernel (four-wide trees): pt_paths.h's loop over all jobs' pixels, a sample at
-// a time; a pixel's items past its job's sample count start nothing.  What a sample reads of the pixel's
-// earlier ones (stream, sum, count of samples run) goes past the L1.  The last paths go to
-// batch_finish_pair.
+// a time, in the order of pt_batch_plan.h.  What a sample reads of the pixel's earlier ones (stream, sum,
+// count of samples run) goes past the L1.  The last paths go to batch_finish_pair.
 struct BatchOps {
     const DeviceScene &merged;
     const BatchBuffers &b;
@@ -378,14 +382,13 @@ struct BatchOps {
         b.rng[g] = rng;
     }
     __device__ bool claim(unsigned long long item, int32_t &root) {
-        const unsigned long long pixels = (unsigned long long)b.total_pixels;
-        unsigned long long pass;
-        if ((item | pixels) >> 32) { pass = item / pixels; g = int64_t(item % pixels); }
-        else { pass = uint32_t(item) / uint32_t(pixels); g = uint32_t(item) % uint32_t(pixels); }
-        jid = job_of(b, g);
+        const BatchItem at = batch_item(b.levels, b.level_count, item);
+        const int32_t k = batch_job_at(b.sorted_first, b.job_count, at.place);
+        jid = b.sorted_jobs[k];
         const BatchJob &j = b.jobs[jid];
-        if (pass >= (unsigned long long)j.samples) return false;
-        if (atomicAdd(&b.claims[g], 1) != 0) return false;   // the lane running this pixel will see it
+        g = j.pixel_offset + int64_t(at.place - b.sorted_first[k]);
+        const int32_t taken = at.drawn < 0 ? 1 : j.samples - at.drawn;
+        if (atomicAdd(&b.claims[g], taken) != 0) return false;   // the lane running this pixel will see it
         __threadfence();
         root = j.root;
         first_ray();
@@ -465,7 +468,7 @@ struct pt_batch {
     DeviceScene view{};
     DeviceBuffer nodes4, nodes2, tris, spheres, triangles, sphere_src, materials, textures, pixels, lights, shade_tris, shade_lights, jobs;
     DeviceBuffer sums, rng, paths, hits, shadows, slot_pixel, slot_job, queue0, queue1, shadow_queue, counters, fetch, scalars,
-        job_remaining, job_done_ns, error, lane_records;
+        job_remaining, job_done_ns, error, lane_records, plan;
     std::vector<BatchJob> host_jobs;
     int64_t total_pixels = 0;
     uint64_t total_triangles = 0;
@@ -561,10 +564,25 @@ struct pt_batch {
                                                               size_t(kSharedStack4) * sizeof(int2) * kPathsBlock));
         return device_sm_count() * (per_sm > 0 ? per_sm : 1);
     }
-    int32_t max_samples() const {
-        int32_t most = 0;
-        for (const auto &j : host_jobs) most = std::max(most, j.samples);
-        return most;
+    // batch_paths' order of samples, for the jobs' present sample counts; returns the number of items
+    unsigned long long upload_plan(cudaStream_t st) {
+        std::vector<int32_t> count, samples;
+        for (const auto &j : host_jobs) { count.push_back(j.pixel_count); samples.push_back(j.samples); }
+        const BatchPlan p = batch_plan(count, samples, 2 * lane_count());
+        const size_t n = host_jobs.size(), most = n * (sizeof(BatchLevel) + sizeof(int32_t) + sizeof(uint32_t));
+        plan.reserve(most);
+        std::vector<unsigned char> bytes(most);
+        const size_t at_jobs = n * sizeof(BatchLevel), at_first = at_jobs + n * sizeof(int32_t);
+        std::memcpy(bytes.data(), p.levels.data(), p.levels.size() * sizeof(BatchLevel));
+        std::memcpy(bytes.data() + at_jobs, p.order.data(), n * sizeof(int32_t));
+        std::memcpy(bytes.data() + at_first, p.first.data(), n * sizeof(uint32_t));
+        PT_CUDA(cudaMemcpyAsync(plan.get(), bytes.data(), most, cudaMemcpyHostToDevice, st));
+        const unsigned char *on_device = plan.get<unsigned char>();
+        buf.levels = reinterpret_cast<const BatchLevel *>(on_device);
+        buf.sorted_jobs = reinterpret_cast<const int32_t *>(on_device + at_jobs);
+        buf.sorted_first = reinterpret_cast<const uint32_t *>(on_device + at_first);
+        buf.level_count = int32_t(p.levels.size());
+        return p.items;
     }
     // The renderer's rule (pt_renderer::whole and tail_alone) for graph-form runs of four-wide nodes, where every
     // lane, or every pixel, has a slot.  Six jobs, ms: the graph's loop and the tail kernel
@@ -632,6 +650,7 @@ struct pt_batch {
         std::vector<int32_t> remaining(static_cast<size_t>(njobs));
         for (int32_t k = 0; k < njobs; k++) remaining[size_t(k)] = host_jobs[size_t(k)].pixel_count;
         PT_CUDA(cudaMemcpyAsync(buf.job_remaining, remaining.data(), remaining.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        const unsigned long long items = whole ? upload_plan(st) : 0;
         PT_CUDA(cudaMemsetAsync(buf.job_done_ns, 0, size_t(njobs) * sizeof(unsigned long long), st));
         PT_CUDA(cudaMemsetAsync(buf.rays, 0, sizeof(unsigned long long), st));
         PT_CUDA(cudaMemsetAsync(buf.error, 0, sizeof(int32_t), st));
@@ -640,7 +659,7 @@ struct pt_batch {
         if (whole) {
             const size_t smem = size_t(kSharedStack4) * sizeof(int2) * kPathsBlock;
             batch_paths_start<<<1, 32, 0, st>>>(buf);
-            batch_paths<<<grid_paths(), kPathsBlock, smem, st>>>(view, buf, (unsigned long long)total_pixels * (unsigned long long)max_samples());
+            batch_paths<<<grid_paths(), kPathsBlock, smem, st>>>(view, buf, items);
             PT_CUDA(cudaGetLastError());
             launch_finish(st);
         } else {
