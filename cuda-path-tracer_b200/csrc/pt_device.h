@@ -80,7 +80,8 @@ constexpr int kRayCounters = 64;
 // atomic, so a setter racing with launches on other threads is well defined; a launch reads each
 // field once.
 struct QueryConfig {
-    std::atomic<int> persistent{1}, min_active{24}, blocks_per_sm{0}, wide{1}, speculative{1};
+    static constexpr int kMinActive = 24;
+    std::atomic<int> persistent{1}, min_active{kMinActive}, blocks_per_sm{0}, wide{1}, speculative{1};
     std::atomic<int> order{2};             // 0 never, 1 always, 2 when the walked arrays exceed the L2
 };
 extern QueryConfig g_query_config;

@@ -327,7 +327,9 @@ void launch_query(const pt_scene *sc, const pt_ray *rays, size_t count, int mode
             const size_t pairs = m->profile_events.size() / 2, k = (which ? m->profile_next - 1 : m->profile_next++) % pairs;
             PT_CUDA(cudaEventRecord(m->profile_events[2 * k + size_t(which)], stream));
         };
-        if (s.small_count && wide && g_query_config.speculative && !stats) {
+        // a refill threshold or block count that pt_query_tuning set is the counter form's
+        const bool tuned = g_query_config.min_active != QueryConfig::kMinActive;
+        if (s.small_count && wide && g_query_config.speculative && !stats && !tuned && !g_query_config.blocks_per_sm) {
             auto fn = any ? query_small_kernel<true> : query_small_kernel<false>;
             const int bps = blocks_per_sm(sc->device, 16 + any, (const void *)fn, 0);
             const unsigned grid = unsigned(std::min<size_t>(grid_for(count, kQueryBlock), size_t(device_sm_count()) * size_t(bps > 0 ? bps : 1)));
@@ -360,7 +362,7 @@ void launch_query(const pt_scene *sc, const pt_ray *rays, size_t count, int mode
         unsigned grid = unsigned(std::min<size_t>(want, resident));
         unsigned long long *counter = nullptr;
         int refill = g_query_config.min_active;
-        if (want <= resident && walk == 2) {
+        if (want <= resident && walk == 2 && !tuned) {
             // a batch that the grid holds at once needs no counter: every warp takes its own rays.  A few rays a
             // warp while they leave warps idle: lanes that share a warp wait for each other's steps (random rays
             // on 1M triangles, 64 rays 30.7 us with 32 a warp, 25.6 with 8, 22.2 with 4; 1000 rays on 10,000
