@@ -523,14 +523,11 @@ struct pt_batch {
         const bool one = one_kernel();
         const size_t handed = one ? size_t(lane_count()) : 0;   // batch_paths queues at most a path per lane
         const size_t records = one ? handed : n;
+        drop_graph();
+        buf.paths = nullptr; buf.hits = nullptr;   // set once all is there: the run after a failure allocates again
         paths.resize(records * sizeof(PathState));
         slot_pixel.resize(records * sizeof(int64_t)); slot_job.resize(records * sizeof(int32_t));
         queue0.resize(records * sizeof(int32_t));
-        buf.paths = paths.get<PathState>();
-        buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
-        buf.queue[0] = queue0.get<int32_t>();
-        buf.hits = nullptr;
-        if (!one && !tail_alone()) wavefront_buffers();
         if (one && !buf.claims) {
             const size_t per_pixel = size_t(total_pixels) * sizeof(int32_t);
             lane_records.resize(handed * (sizeof(PathState) + sizeof(ShadowRay)) + 2 * per_pixel);
@@ -541,22 +538,26 @@ struct pt_batch {
             buf.done = reinterpret_cast<int32_t *>(at);
             PT_CUDA(cudaMemsetAsync(buf.claims, 0, per_pixel, stream));   // on the runs' stream: the default stream may be behind it
         }
-        drop_graph();
+        if (!one && !tail_alone()) { wavefront_buffers(); return; }
+        buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
+        buf.queue[0] = queue0.get<int32_t>();
+        buf.paths = paths.get<PathState>();
     }
     // a record per slot for the loop's kernels, allocated with the first run that needs them
     void wavefront_buffers() {
         if (buf.hits) return;
         const size_t n = size_t(std::max(slots, 1));
         drop_graph();
+        buf.paths = nullptr;
         paths.reserve(n * sizeof(PathState)); slot_pixel.reserve(n * sizeof(int64_t)); slot_job.reserve(n * sizeof(int32_t));
         queue0.reserve(n * sizeof(int32_t));
         hits.resize(n * sizeof(PathHit)); shadows.resize(n * sizeof(ShadowRay));
         queue1.resize(n * sizeof(int32_t)); shadow_queue.resize(n * sizeof(int32_t));
-        buf.paths = paths.get<PathState>();
         buf.slot_pixel = slot_pixel.get<int64_t>(); buf.slot_job = slot_job.get<int32_t>();
         buf.queue[0] = queue0.get<int32_t>(); buf.queue[1] = queue1.get<int32_t>();
         buf.shadows = shadows.get<ShadowRay>(); buf.shadow_queue = shadow_queue.get<int32_t>();
         buf.hits = hits.get<PathHit>();
+        buf.paths = paths.get<PathState>();
     }
     int grid_paths() const {
         int per_sm = 0;
@@ -643,6 +644,7 @@ struct pt_batch {
     }
     void run() {
         cudaStream_t st = stream;
+        if (!buf.paths) allocate_slots();
         const bool whole = fused() && buf.claims && one_kernel();
         const bool alone = fused() && tail_alone();
         if (!whole && !alone) wavefront_buffers();

@@ -11,7 +11,9 @@
 namespace ptb {
 
 inline void cuda_check(cudaError_t result, const char *what) {
-    if(result != cudaSuccess) throw Error(PT_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(result));
+    if(result == cudaSuccess) return;
+    cudaGetLastError();   // reported here: the check after the next launch is not to find it again
+    throw Error(PT_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(result));
 }
 #define PT_CUDA(call) ::ptb::cuda_check((call), #call)
 
