@@ -442,6 +442,12 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) batch_paths(De
     if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
 }
 
+__global__ void batch_probe(DeviceScene scene, const BatchJob *jobs, uint32_t *met) {
+    constexpr int blocks = kProbePaths / kProbeBlock;
+    const BatchJob &j = jobs[blockIdx.x / blocks];
+    atomicAdd(&met[blockIdx.x / blocks], probe_path(scene, j.camera, j.root, int32_t(blockIdx.x % blocks * kProbeBlock + threadIdx.x)));
+}
+
 // What batch_paths and the tail after it expect: no slot queued, no pixel left to start.
 __global__ void batch_paths_start(BatchBuffers b) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -478,6 +484,7 @@ struct pt_batch {
     int32_t wide = 1;                     // node fetch width: 1 four-wide nodes, 0 the two-wide layout
     int32_t default_tail = 16384;         // the tail length pt_batch_create chose
     bool loop = false;                    // a tail length was asked for (or the autotuner is timing the loop): no one-kernel form
+    double going_on_pixels = 0, most_going_on = 0;   // pixels of jobs whose paths go on, and their mean limit per lane
     int32_t probe_fault_countdown = 0;   // > 0: that autotune probe run fails on the host (tests)
     int32_t slots = 0;
     BatchBuffers buf{};
@@ -586,12 +593,34 @@ struct pt_batch {
         return p.items;
     }
     // The renderer's rule (pt_renderer::whole and tail_alone) for graph-form runs of four-wide nodes, where every
-    // lane, or every pixel, has a slot.  Six jobs, ms: the graph's loop and the tail kernel
-    // alone 3,900 pixels 0.53 and 0.30, 23,000 1.54 and 0.93, 88,000 4.7 and 2.3; one kernel and the tail kernel alone
-    // 129,000 3.1 and 3.2, 175,000 3.6 and 3.2; the loop and one kernel (four blocks per SM) 534,000 11.9 and 7.0,
-    // 1.2M 32.0 and 25.8, 2.3M 20.6 and 19.5.
+    // lane, or every pixel, has a slot; pt_forms.h has the sizes of batch_paths.  Six jobs, ms: the graph's loop and the
+    // tail kernel alone 3,900 pixels 0.53 and 0.30, 23,000 1.54 and 0.93, 88,000 4.7 and 2.3; one kernel and the tail
+    // kernel alone 129,000 3.1 and 3.2, 175,000 3.6 and 3.2.
     int64_t lane_count() const { return int64_t(grid_paths()) * kPathsBlock; }
-    bool one_kernel() const { return total_pixels > 2 * lane_count() && total_pixels <= 40 * lane_count() && slots >= lane_count(); }
+    bool sized() const { return total_pixels > 2 * lane_count() && total_pixels <= 40 * lane_count(); }
+    bool one_kernel() const {
+        return sized() && slots >= lane_count() &&
+               batch_in_one(double(total_pixels) - going_on_pixels, going_on_pixels, most_going_on,
+                            nodes4.bytes() + tris.bytes() + spheres.bytes(), double(lane_count()));
+    }
+    // Which jobs' paths go on (pt_forms.h); `primitives` per job.
+    void look(const std::vector<size_t> &primitives) {
+        if (!sized()) return;
+        const size_t n = host_jobs.size();
+        DeviceBuffer met(n * sizeof(uint32_t));
+        std::vector<uint32_t> found(n);
+        PT_CUDA(cudaMemsetAsync(met.get(), 0, met.bytes(), stream));
+        batch_probe<<<unsigned(n * (kProbePaths / kProbeBlock)), kProbeBlock, 0, stream>>>(view, jobs.get<BatchJob>(), met.get<uint32_t>());
+        PT_CUDA(cudaGetLastError());
+        PT_CUDA(cudaMemcpyAsync(found.data(), met.get(), met.bytes(), cudaMemcpyDeviceToHost, stream));
+        PT_CUDA(cudaStreamSynchronize(stream));
+        for (size_t k = 0; k < n; k++) {
+            if (!paths_go_on(found[k])) continue;
+            going_on_pixels += host_jobs[k].pixel_count;
+            most_going_on += host_jobs[k].pixel_count * most_pixels_going_on(primitives[k]);
+        }
+        if (going_on_pixels > 0) most_going_on /= going_on_pixels;
+    }
     bool tail_alone() const { return total_pixels <= 2 * lane_count() && slots >= total_pixels; }
     bool fused() const { return use_graph && wide && !loop; }
     unsigned long long max_iterations() const {
@@ -877,6 +906,9 @@ pt_status pt_batch_create(const pt_scene_desc *scenes, int32_t scene_count, cons
             b->tail_paths = b->default_tail = int32_t(std::max<int64_t>(16384, offset / 64));
             PT_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
             PT_CUDA(cudaStreamCreateWithFlags(&b->shadow_stream, cudaStreamNonBlocking));
+            std::vector<size_t> primitives;
+            for (int32_t k = 0; k < job_count; k++) primitives.push_back(scenes[jobs[k].scene].triangle_count + scenes[jobs[k].scene].sphere_count);
+            b->look(primitives);
             b->allocate_slots();
         } catch (...) { delete b; throw; }
         *out = b;

@@ -1047,17 +1047,19 @@ pt_status pt_cached_create(const pt_scene *scene, const pt_camera *camera, int w
             r->grid_frame = occupancy_grid((const void *)frame_kernel, kPathsBlock, size_t(kSharedStack4) * sizeof(int2) * kPathsBlock);
             // A frame that renders every pixel, unless a tail length asks for the wavefront: up to three pixels per resident
             // lane by the tail kernel alone, whose two lanes per path walk extension and shadow rays side by side; up to
-            // twenty, or twenty-eight when the bounces of a frame are many, by frame_kernel; above by the wavefront.
+            // the sizes of pt_forms.h by frame_kernel; above by the wavefront.
             // Tail kernel alone and frame_kernel, ms a frame (1M triangles, bounce limit 12; three pixels per lane are
             // 284,000): 100x80 one sample 0.34 and 0.43, four 0.91 and 1.24; 480x300 0.64 and 0.74, 2.18 and 2.34;
             // 640x400 0.74 and 0.86, 2.54 and 2.67; 960x600 1.16 and 1.10, 4.2 and 3.1; 65,000 triangles 200x120 two
-            // samples 0.15 and 0.28 (wavefront 0.26), 640x400 0.31 and 0.42, 960x600 0.51 and 0.51.  Wavefront and
-            // frame_kernel: 960x600 four 4.8 and 3.0; with four blocks per SM 1920x1080 one 2.1 and 2.3, two 4.07 and
-            // 3.94, four 7.8 and 7.25, four of limit 4 6.5 and 6.6; 2560x1440 11.0 and 12.2.
+            // samples 0.15 and 0.28 (wavefront 0.26), 640x400 0.31 and 0.42, 960x600 0.51 and 0.51.
             const int64_t lanes = int64_t(r->grid_frame) * kPathsBlock, count = int64_t(n);
-            const bool deep = int64_t(p.spf) * p.max_depth >= 24, chosen = p.wide == 2 && cfg.tail_paths == 0;
-            r->alone = chosen && count <= 3 * lanes;
-            r->whole = chosen && !r->alone && count <= (deep ? 28 : 20) * lanes;
+            const bool chosen = p.wide == 2 && cfg.tail_paths == 0;
+            r->alone = chosen && count <= (p.use_cache ? 3 : 2) * lanes;   // as the plain renderer without its cache
+            const bool sized = chosen && !r->alone && count <= 28 * lanes, goes_on = sized && view_goes_on(scene->view, *camera, r->stream);
+            const size_t primitives = scene->triangle_count + scene->sphere_count;
+            const int64_t bounces = int64_t(p.spf) * p.max_depth;
+            r->whole = sized && double(count) <= double(lanes) * (p.use_cache ? most_pixels_cached(goes_on, primitives, scene->walked_bytes(), bounces)
+                                                                              : most_pixels(goes_on, primitives, scene->walked_bytes(), bounces));
             if (r->whole) {
                 const size_t l = size_t(lanes), per_pixel = n * sizeof(int32_t);
                 r->lane_records.resize(l * (sizeof(CachePath) + sizeof(CacheShadow)) + 2 * per_pixel);

@@ -73,6 +73,8 @@ void require_device();
 // Fills the shading records of a scene whose other arrays are on the device (`lights` emitters) and
 // points the view at them.
 void build_shading(DeviceScene &view, size_t lights, DeviceBuffer &shade_tris, DeviceBuffer &shade_lights);
+// Whether the paths of a view of a four-wide scene go on for more than a bounce (pt_forms.h); waits for `stream`.
+bool view_goes_on(const DeviceScene &scene, const pt_camera &camera, cudaStream_t stream);
 int device_sm_count();
 // Ray counters per scene: launches further apart than this many may share one counter, so a scene
 // takes at most this many persistent-kernel launches in flight at once.
@@ -99,6 +101,7 @@ struct pt_scene {
     float light_area = 0;
     int32_t leaf_count = 0;
     size_t triangle_count = 0, sphere_count = 0;
+    size_t walked_bytes() const { return nodes4.bytes() + tris.bytes() + spheres.bytes(); }
     // host-buffer query workspace (reused between calls)
     ptb::DeviceBuffer work_rays[3], work_tmax[3], work_hits[3], work_stats[3];
     cudaStream_t streams[3] = {nullptr, nullptr, nullptr};

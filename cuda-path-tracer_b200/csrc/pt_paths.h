@@ -26,10 +26,36 @@
 // doubled the time a heavy pixel waits for each bounce (12.6 ms in all).
 #pragma once
 
+#include "pt_forms.h"
 #include "pt_wavefront.h"
 
 #ifdef __CUDACC__
 namespace ptb {
+
+constexpr int kProbeBlock = 8;        // few paths to a warp: a probe lasts as long as its slowest warp
+// Camera path `i` of the probe of a view (pt_forms.h): how many surfaces other than lights it meets in two walks,
+// every one of them taken as diffuse.
+__device__ inline uint32_t probe_path(const DeviceScene &scene, const pt_camera &camera, int32_t root, int32_t i) {
+    Pcg rng;
+    rng.seed(1, uint64_t(i));
+    PathState s;
+    camera_path(camera, kProbeSide, kProbeSide, i, rng, s);
+    uint32_t met = 0;
+    for (; met < 2; met++) {
+        const pt_ray r = path_ray(s);
+        HitInfo h;
+        uint32_t boxes = 0, prims = 0;
+        int error = 0;
+        if (!traverse4_rt(scene, r, 0.001f, FLT_MAX, kTieLastLeaf, false, h, boxes, prims, error, root) || error) break;
+        Surface o;
+        surface_hit(scene, r, h, o);
+        if (scene.materials[o.material].type == PT_LIGHT) break;
+        const f3 in = mk(r.direction), d = cosine_direction(dot(o.normal, in) > 0 ? -o.normal : o.normal, rng);
+        s.ox = o.p.x; s.oy = o.p.y; s.oz = o.p.z;
+        s.dx = d.x; s.dy = d.y; s.dz = d.z;
+    }
+    return met;
+}
 
 constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 5;   // 96 registers
 constexpr int kPathsActive = 4;   // lanes of a warp still walking below which the others shade

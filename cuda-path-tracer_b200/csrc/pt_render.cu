@@ -463,6 +463,23 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm) render_paths_k
     if (lane_id() == 0 && rays) atomicAdd(b.rays, rays);
 }
 
+__global__ void probe_kernel(DeviceScene scene, pt_camera camera, uint32_t *met) {
+    atomicAdd(met, probe_path(scene, camera, 0, int32_t(blockIdx.x * blockDim.x + threadIdx.x)));
+}
+void launch_probe(const DeviceScene &scene, const pt_camera &camera, uint32_t *met, cudaStream_t stream) {
+    PT_CUDA(cudaMemsetAsync(met, 0, sizeof(uint32_t), stream));
+    probe_kernel<<<kProbePaths / kProbeBlock, kProbeBlock, 0, stream>>>(scene, camera, met);
+    PT_CUDA(cudaGetLastError());
+}
+bool view_goes_on(const DeviceScene &scene, const pt_camera &camera, cudaStream_t stream) {
+    DeviceBuffer met(sizeof(uint32_t));
+    uint32_t n = 0;
+    launch_probe(scene, camera, met.get<uint32_t>(), stream);
+    PT_CUDA(cudaMemcpyAsync(&n, met.get(), sizeof n, cudaMemcpyDeviceToHost, stream));
+    PT_CUDA(cudaStreamSynchronize(stream));
+    return paths_go_on(n);
+}
+
 // shadow: any-hit of the NEE rays (transport.h:206-214); unoccluded ones add their contribution
 __global__ void __launch_bounds__(256, 4) shadow_kernel(DeviceScene scene, RenderParams p, RenderBuffers b, int parity, int min_active) {
     const int32_t n = b.counters[2 + parity];
@@ -533,6 +550,8 @@ int occupancy_grid(const void *kernel, int block, size_t smem = 0) {
 
 } // namespace ptb
 
+constexpr int kIterationRing = 8;   // == size of pt_renderer::iteration_events
+
 struct pt_renderer {
     const pt_scene *scene = nullptr;
     RenderParams params{};
@@ -549,14 +568,15 @@ struct pt_renderer {
     bool pair_tail = false;             // the tail runs two lanes per path (finish_pair_kernel)
     bool fused = false;                 // four-wide tree and shaded view: the form goes by the image's size (whole, tail_alone)
     bool small = false;                 // the scene fits render_small_kernel and the view is shaded
-    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lanes;
+    bool goes_on = false, looking = false;   // paths of the view looked at last (pt_forms.h); a look is under way
+    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lanes, met;
     RenderBuffers buf{};
     cudaStream_t stream = nullptr;
     cudaStream_t shadow_stream = nullptr;   // shadow kernel k runs beside extend k+1
     Event start, stop;
     Event shaded[2], shadowed[2];           // by iteration parity
-    int32_t *host_counters = nullptr;   // pinned, one slot per in-flight iteration
-    Event iteration_events[8];
+    int32_t *host_counters = nullptr;   // pinned, one slot per in-flight iteration and one for the probe of the view
+    Event iteration_events[8], looked;
     ~pt_renderer() {
         if (host_counters) cudaFreeHost(host_counters);
         if (shadow_stream) cudaStreamDestroy(shadow_stream);
@@ -594,15 +614,34 @@ struct pt_renderer {
     }
     // Which kernels render an image of a four-wide scene in the shaded view, unless pt_renderer_tuning asked
     // for the wavefront.  Up to two pixels per lane of render_paths_kernel: the tail kernel alone, whose two
-    // lanes per path walk extension and shadow rays side by side.  Up to forty: render_paths_kernel.  From
-    // there on the wavefront: its queues are long enough to hide their slowest rays and its walk kernels
-    // hold more warps.  Milliseconds a call (tail kernel alone, render_paths_kernel, wavefront with tail; 1M
+    // lanes per path walk extension and shadow rays side by side.  Above, render_paths_kernel up to the sizes of
+    // pt_forms.h, from there on the wavefront: its queues are long enough to hide their slowest rays and its walk
+    // kernels hold more warps.  Milliseconds a call (tail kernel alone, render_paths_kernel, wavefront with tail; 1M
     // triangles, 12 spp, bounce limit 8): 64,000 pixels 3.4, -, 5.0; 99,000 4.1, 5.3, -; 144,000 5.1, 5.5, 6.6;
     // 187,000 6.4, 5.9, -; 256,000 7.3, 5.2, -; on 10,000 triangles 64,000 pixels 0.64, -, 1.2; 144,000 1.1, 1.4, -;
-    // 187,000 1.3, 1.65, -; 256,000 1.4, 1.7, -.
-    // Large images, 16 spp: 1920x1080 -, 27.0, 30.4; 3840x2160 -, 111.8 (four blocks per SM), 91.8.
+    // 187,000 1.3, 1.65, -; 256,000 1.4, 1.7, 2.7.
     int64_t lane_count() const { return int64_t(grid_paths) * kPathsBlock; }
-    bool whole() const { return fused && pixels > 2 * lane_count() && pixels <= 40 * lane_count(); }
+    bool sized() const { return fused && pixels > 2 * lane_count() && pixels <= 40 * lane_count(); }   // for render_paths_kernel
+    bool whole(int count) const {
+        if (!sized()) return false;
+        return double(pixels) <= most_pixels(goes_on, scene->triangle_count + scene->sphere_count, scene->walked_bytes(),
+                                             int64_t(count) * params.max_depth) * double(lane_count());
+    }
+    // Looks at a view beside whatever comes next; seen() takes the answer once it is there, or waits for it.
+    void look(const pt_camera &camera) {
+        if (!sized()) return;
+        met.reserve(sizeof(uint32_t));
+        launch_probe(scene->view, camera, met.get<uint32_t>(), shadow_stream);
+        PT_CUDA(cudaMemcpyAsync(&host_counters[kIterationRing], met.get(), sizeof(uint32_t), cudaMemcpyDeviceToHost, shadow_stream));
+        PT_CUDA(cudaEventRecord(looked.get(), shadow_stream));
+        looking = true;
+    }
+    void seen(bool wait) {
+        if (!looking || (!wait && cudaEventQuery(looked.get()) != cudaSuccess)) return;
+        PT_CUDA(cudaEventSynchronize(looked.get()));
+        goes_on = paths_go_on(uint32_t(host_counters[kIterationRing]));
+        looking = false;
+    }
     // An image below the tail's length has no wavefront to run first either (1.2 and 0.6 ms for 52,000 pixels of 12
     // samples on 10,000 triangles).
     bool tail_alone() const { return (pair_kernel() && pixels < tail_paths) || (fused && pixels <= 2 * lane_count()); }
@@ -627,7 +666,6 @@ void validate_camera(const pt_camera &c) {
     if (!std::isfinite(c.lens_radius) || c.lens_radius < 0 || !std::isfinite(c.time0) || !std::isfinite(c.time1) || c.time1 < c.time0)
         throw Error(PT_INVALID_ARGUMENT, "invalid camera lens/shutter");
 }
-constexpr int kIterationRing = 8;   // == size of pt_renderer::iteration_events
 } // namespace
 
 extern "C" {
@@ -668,23 +706,29 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             b.sums = r->sums.get<float>(); b.rng = r->rng.get<Pcg>();
             PT_CUDA(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking));
             PT_CUDA(cudaStreamCreateWithFlags(&r->shadow_stream, cudaStreamNonBlocking));
-            PT_CUDA(cudaMallocHost(&r->host_counters, kIterationRing * sizeof(int32_t)));
+            PT_CUDA(cudaMallocHost(&r->host_counters, (kIterationRing + 1) * sizeof(int32_t)));
             r->grids();
             // below 65,536 live paths the fused kernel holds them all at once (measured: config 1 is 3.6 %
             // faster than with a floor of 16,384; larger images are unchanged)
             r->tail_paths = std::max<int32_t>(65536, r->pixels / 4);
+            r->pair_tail = p.wide != 0;
+            r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
+            r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
+            if (!r->small) { r->look(*camera); r->seen(true); }
             // On a tree of a few nodes (tens of primitives) a bounce is mostly shading: the two-wide walk
             // (fewer instructions per visit) and one lane per path in the tail are faster there
             // (config 1, 23 primitives: 8.4 ms per render with the four-wide walk and two lanes per
             // path, 6.8 with one lane, 6.5 with the two-wide walk too); from a few hundred triangles on,
             // two lanes per path win (772 triangles: 3.4 vs 4.1 ms).
             constexpr size_t kSmallTreeNodes = 32;
+            constexpr int kManySamples = 16;             // what the first call is taken to ask for
             if (p.wide && scene->nodes4.bytes() / sizeof(Bvh4QNode) <= kSmallTreeNodes) p.wide = 0;
             r->pair_tail = p.wide != 0;
             r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
             r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
+            if (!r->small) { r->look(*camera); r->seen(true); }
             if (!r->small) {                             // what the first call will most likely use
-                if (r->whole()) r->lane_buffers();
+                if (r->whole(kManySamples)) r->lane_buffers();
                 else if (r->tail_alone()) r->path_buffers();
                 else r->wavefront_buffers();
             }
@@ -706,6 +750,7 @@ pt_status pt_reset(pt_renderer *r, const pt_camera *camera) {
         init_pixels<<<(r->pixels + 255) / 256, 256, 0, r->stream>>>(r->buf.sums, r->buf.rng, r->pixels, r->seed);
         PT_CUDA(cudaGetLastError());
         PT_CUDA(cudaStreamSynchronize(r->stream));
+        if (std::memcmp(camera, &r->params.camera, sizeof *camera)) r->look(*camera);
         r->params.camera = *camera;
         r->samples = 0; r->milliseconds = 0; r->rays = 0;
     });
@@ -718,7 +763,8 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         if (count <= 0 || count > INT32_MAX - r->samples) throw Error(PT_INVALID_ARGUMENT, "invalid accumulated sample count");
         const DeviceScene &scene = r->scene->view;
         cudaStream_t st = r->stream;
-        const bool whole = !r->small && r->whole(), tail_alone = !r->small && !whole && r->tail_alone();
+        r->seen(count >= 4);   // after a reset to another view; a short call takes the form of the view before
+        const bool whole = !r->small && r->whole(count), tail_alone = !r->small && !whole && r->tail_alone();
         if (whole) r->lane_buffers();
         else if (tail_alone) r->path_buffers();
         else if (!r->small) r->wavefront_buffers();

@@ -243,14 +243,16 @@ pt_status pt_reset(pt_renderer *renderer, const pt_camera *camera);
 /* add_samples(count) (src/cuda/cuda_renderer.cu:196-213); blocks until the samples are done. */
 pt_status pt_add_samples(pt_renderer *renderer, int count);
 /* set_block_shape(w, h): accepted shapes 8x8, 16x8, 16x16, 32x8 (src/cuda/cuda_renderer.cu:215-228).
- * Sets the thread-block size of the wavefront kernels to w*h threads. */
+ * Sets the thread-block size of the wavefront kernels and of the kernel that ends a render to w*h threads. */
 pt_status pt_set_block_shape(pt_renderer *renderer, int width, int height);
 /* Live-path count below which add_samples stops the wavefront and runs the remaining paths to
  * completion in one fused kernel (two threads per path on four-wide trees: one walks the path's
  * next ray while the other walks its last shadow ray; default max(65536, pixels/4); 0 keeps the
  * wavefront to the end).  Until this is called, shaded renders of scenes of at most 32 primitives, and
- * of images of two to forty pixels per resident GPU thread, run as one kernel from the first camera ray to
- * the last bounce, and smaller images in the two-threads-per-path kernel alone; calling it asks for the wavefront.  Results do not depend on it. */
+ * images of two to at most forty pixels per resident GPU thread (fewer the larger the scene and the fewer the samples
+ * of a call, and hardly any inside a room, where paths go on: the view is looked at when the renderer is created or
+ * reset to another camera) run as one kernel from the first camera ray to the last bounce, and smaller images in the
+ * two-threads-per-path kernel alone; calling it asks for the wavefront.  Results do not depend on it. */
 pt_status pt_renderer_tuning(pt_renderer *renderer, int32_t tail_paths);
 /* Linear FP32 radiance sums (3 floats per pixel, row 0 at the bottom, not divided by spp). */
 pt_status pt_get_sums(const pt_renderer *renderer, float *rgb_sums, size_t floats);
@@ -292,8 +294,8 @@ pt_status pt_batch_stats(const pt_batch *batch, float *kernel_ms, uint64_t *rays
  * what the batch starts with, max(16384, pixels / 64), leave the form to the batch's size; any other
  * value asks for the loop); use_graph: 1 = the loop runs on the device (one graph launch; or, on
  * four-wide nodes, with up to two pixels per resident GPU thread and a slot for each pixel the fused
- * kernel alone, and with two to forty and a slot for each thread one kernel that walks and shades; these
- * take no block, refill or tail setting), 0 = host-driven loop. */
+ * kernel alone, and with two to at most thirty and a slot for each thread one kernel that walks and shades, unless
+ * most jobs' views are rooms (see pt_renderer_tuning); these take no block, refill or tail setting), 0 = host-driven loop. */
 pt_status pt_batch_tuning(pt_batch *batch, int32_t path_capacity, int32_t block, int32_t min_active, int32_t tail_paths,
                           int32_t use_graph);
 /* Node fetch width of the batch's walks: 1 = four-wide nodes (default), 0 = the two-wide layout.
@@ -370,8 +372,9 @@ typedef struct pt_cached_params {
     float learning_rate;        /* Adam learning rate (1e-2; beta 0.9 / 0.99) */
     uint64_t network_seed;      /* weight initialisation */
     int32_t tail_paths;         /* live paths below which one fused kernel ends the frame's tail
-                                 * (0: max(16384, pixels / 16), and frames of up to some twenty pixels per
-                                 * resident GPU thread run without the wavefront; the image is the same) */
+                                 * (0: max(16384, pixels / 16), and frames of up to three, open views of up
+                                 * to ten to twenty-eight pixels per resident GPU thread run without the
+                                 * wavefront; the image is the same) */
     int32_t query_specular;     /* 1 (default): paths may also end at metal and glass vertices;
                                  * 0: at diffuse vertices only */
     float weight_average;       /* decay of the weight average queries use (0.99; 0: the live weights) */

@@ -1,0 +1,115 @@
+"""Which kernels render an image of ordinary size: the one that walks and shades where most paths end early, the
+wavefront where they go on (csrc/pt_forms.h).  Inside a room the former took up to 1.7 times as long as the latter.
+
+Told by memory: the wavefront's records, some 70 bytes a pixel, are allocated by the first call that needs them."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import ptb200 as pt
+
+pytestmark = pytest.mark.gpu
+WIDTH, HEIGHT = 1280, 720            # 921,600 pixels
+RECORDS = 40 << 20
+
+
+def free() -> int:
+    import torch
+    return torch.cuda.mem_get_info()[0]
+
+
+def room(width=WIDTH, height=HEIGHT):
+    """The Cornell box, every triangle split into sixteen."""
+    flat, cam = pt.cornell_box(width, height)
+    t = flat.triangles
+    for _ in range(2):
+        a, b, c = t["v0"], t["v1"], t["v2"]
+        ab, bc, ca = (a + b) / 2, (b + c) / 2, (c + a) / 2
+        parts = []
+        for corners in ((a, ab, ca), (ab, b, bc), (ca, bc, c), (ab, bc, ca)):
+            q = t.copy()
+            q["v0"], q["v1"], q["v2"] = corners
+            parts.append(q)
+        t = np.concatenate(parts)
+    return pt.FlatScene(t, flat.spheres, None, flat.materials, flat.textures, flat.pixels).build_bvh(), cam
+
+
+def spheres(width=WIDTH, height=HEIGHT):
+    return pt.procedural_scene(width, height, sphere_count=4, segments=24, rings=13, seed=2)
+
+
+@pytest.mark.parametrize("view,loop", [(room, True), (spheres, False)], ids=["room", "open"])
+def test_renderer_form(view, loop):
+    flat, cam = view()
+    r = pt.CudaRenderer(flat, cam, WIDTH, HEIGHT, 3, max_depth=6)
+    r.add_samples(2)
+    want, before = r.sums().tobytes(), free()
+    r.set_tail_paths(WIDTH * HEIGHT // 4)
+    r.reset(cam)
+    r.add_samples(2)
+    assert (before - free() < RECORDS) == loop
+    assert r.sums().tobytes() == want
+
+
+@pytest.mark.parametrize("view,loop", [(room, True), (spheres, False)], ids=["room", "open"])
+def test_batch_form(view, loop):
+    flat, cam = view()
+    b = pt.Batch([flat], [dict(scene=0, camera=cam, width=WIDTH, height=HEIGHT, samples=2, max_depth=6, seed=3)])
+    b.run()
+    want, before = b.sums(0).tobytes(), free()
+    b.tuning(tail_paths=20000)
+    b.run()
+    assert (before - free() < RECORDS) == loop
+    assert b.sums(0).tobytes() == want
+
+
+@pytest.mark.parametrize("view,loop", [(room, True), (spheres, False)], ids=["room", "open"])
+def test_cached_form(view, loop):
+    flat, cam = view()
+    r = pt.CachedRenderer(flat, cam, WIDTH, HEIGHT, seed=3, max_depth=6, samples_per_frame=2)
+    r.frames(1)
+    before = free()
+    r.train(1)                       # training-only frames run in the wavefront
+    assert (before - free() < RECORDS) == loop
+
+
+def test_reset_looks_at_the_new_view():
+    flat, inside = room()
+    away = pt.make_camera((40, 0.5, 0.5), (60, 0.5, 0.5), (0, 1, 0), 40.0, WIDTH / HEIGHT)
+    r = pt.CudaRenderer(flat, away, WIDTH, HEIGHT, 3, max_depth=6)
+    r.add_samples(2)
+    before = free()
+    r.reset(inside)
+    r.add_samples(4)                 # a call of few samples would not wait for the look
+    assert before - free() >= RECORDS
+    want = pt.CudaRenderer(flat, inside, WIDTH, HEIGHT, 3, max_depth=6)
+    want.add_samples(4)
+    assert r.sums().tobytes() == want.sums().tobytes()
+    r.reset(away)
+    r.add_samples(1)
+    r.reset(inside)
+    r.add_samples(1)
+    r.add_samples(3)
+    assert r.sums().tobytes() == want.sums().tobytes()
+
+
+def test_batch_of_rooms_and_open_views():
+    """Two rooms of 20,000 pixels among 600,000 of an open scene, and against a lone renderer each."""
+    a, cam_a = room(200, 100)
+    b, cam_b = spheres(1000, 600)
+    jobs = [dict(scene=0, camera=cam_a, width=200, height=100, samples=3, max_depth=6, seed=1),
+            dict(scene=1, camera=cam_b, width=1000, height=600, samples=1, max_depth=4, seed=2),
+            dict(scene=0, camera=cam_a, width=200, height=100, samples=2, max_depth=9, seed=3)]
+    batch = pt.Batch([a, b], jobs)
+    batch.run()
+    before = free()
+    for k, j in enumerate(jobs):
+        r = pt.CudaRenderer((a, b)[j["scene"]], j["camera"], j["width"], j["height"], j["seed"], direct_light=True, max_depth=j["max_depth"])
+        r.add_samples(j["samples"])
+        assert batch.sums(k).tobytes() == r.sums().tobytes()
+        r.close()
+    before = free()
+    batch.tuning(tail_paths=20000)
+    batch.run()
+    assert before - free() >= RECORDS // 2
