@@ -568,8 +568,9 @@ struct pt_renderer {
     bool pair_tail = false;             // the tail runs two lanes per path (finish_pair_kernel)
     bool fused = false;                 // four-wide tree and shaded view: the form goes by the image's size (whole, tail_alone)
     bool small = false;                 // the scene fits render_small_kernel and the view is shaded
+    bool tiny = false;                  // a tree of a few nodes
     bool goes_on = false, looking = false;   // paths of the view looked at last (pt_forms.h); a look is under way
-    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, claims, lanes, met;
+    DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, lanes, met;
     RenderBuffers buf{};
     cudaStream_t stream = nullptr;
     cudaStream_t shadow_stream = nullptr;   // shadow kernel k runs beside extend k+1
@@ -642,6 +643,7 @@ struct pt_renderer {
         goes_on = paths_go_on(uint32_t(host_counters[kIterationRing]));
         looking = false;
     }
+    void narrow() { params.wide = 0; pair_tail = false; fused = false; }
     // An image below the tail's length has no wavefront to run first either (1.2 and 0.6 ms for 52,000 pixels of 12
     // samples on 10,000 triangles).
     bool tail_alone() const { return (pair_kernel() && pixels < tail_paths) || (fused && pixels <= 2 * lane_count()); }
@@ -715,18 +717,15 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
             r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
             if (!r->small) { r->look(*camera); r->seen(true); }
-            // On a tree of a few nodes (tens of primitives) a bounce is mostly shading: the two-wide walk
-            // (fewer instructions per visit) and one lane per path in the tail are faster there
-            // (config 1, 23 primitives: 8.4 ms per render with the four-wide walk and two lanes per
-            // path, 6.8 with one lane, 6.5 with the two-wide walk too); from a few hundred triangles on,
-            // two lanes per path win (772 triangles: 3.4 vs 4.1 ms).
+            // On a tree of a few nodes (tens of primitives) the wavefront's bounce is mostly shading: with an explicit
+            // tail length, and in the debug views, the two-wide walk (fewer instructions per visit) and one lane per path
+            // in the tail (64 triangles, 1920x1080, one sample, all of it in the tail: 0.62 ms and 1.6 with two lanes).  Not so
+            // what runs otherwise (two-wide wavefront and now, 16 spp, ms; 64 triangles 64x40 0.81 and 0.30, 960x600
+            // 3.2 and 1.55, 3000x1688 13.8 and 13.6; 80 in a room 320x200 8.4 and 5.4, 960x600 40 and 28).
             constexpr size_t kSmallTreeNodes = 32;
             constexpr int kManySamples = 16;             // what the first call is taken to ask for
-            if (p.wide && scene->nodes4.bytes() / sizeof(Bvh4QNode) <= kSmallTreeNodes) p.wide = 0;
-            r->pair_tail = p.wide != 0;
-            r->fused = p.wide == 2 && !p.brute && p.debug == PT_DEBUG_SHADED;
-            r->small = scene->view.small_count > 0 && !p.brute && p.debug == PT_DEBUG_SHADED;
-            if (!r->small) { r->look(*camera); r->seen(true); }
+            r->tiny = scene->nodes4.bytes() / sizeof(Bvh4QNode) <= kSmallTreeNodes;
+            if (r->tiny && (r->small || !r->fused)) r->narrow();
             if (!r->small) {                             // what the first call will most likely use
                 if (r->whole(kManySamples)) r->lane_buffers();
                 else if (r->tail_alone()) r->path_buffers();
@@ -862,6 +861,7 @@ pt_status pt_renderer_tuning(pt_renderer *r, int32_t tail_paths) {
         if (!r || tail_paths < 0) throw Error(PT_INVALID_ARGUMENT, "invalid renderer tuning");
         r->tail_paths = tail_paths;
         r->small = r->fused = false;   // an explicit wavefront / tail split asks for the general kernels
+        if (r->tiny) r->narrow();
     });
 }
 

@@ -113,3 +113,44 @@ def test_batch_of_rooms_and_open_views():
     batch.tuning(tail_paths=20000)
     batch.run()
     assert before - free() >= RECORDS // 2
+
+
+@pytest.mark.parametrize("segments,rings", [(5, 5), (6, 6), (8, 8), (10, 10)])
+@pytest.mark.parametrize("width,height", [(64, 40), (640, 400), (1280, 720)])
+def test_trees_of_a_few_nodes(segments, rings, width, height):
+    """Scenes of 33 to some 190 triangles: the forms of larger scenes, and the wavefront's own when asked for."""
+    flat, cam = pt.procedural_scene(width, height, sphere_count=1, segments=segments, rings=rings, seed=4)
+    r = pt.CudaRenderer(flat, cam, width, height, 3, max_depth=6)
+    r.add_samples(3)
+    want, rays, before = r.sums().tobytes(), r.rays_traced(), free()
+    r.set_tail_paths(500)
+    r.reset(cam)
+    r.add_samples(3)
+    assert r.sums().tobytes() == want and r.rays_traced() == rays
+    if width == WIDTH:
+        assert before - free() >= RECORDS
+    brute = pt.CudaRenderer(flat, cam, width, height, 3, max_depth=6, brute=True)
+    brute.add_samples(3)
+    assert brute.rays_traced() == rays and brute.sums().tobytes() == want
+
+
+def test_small_room():
+    """80 triangles in a room: the two-lane kernel alone for a small image, the two-wide wavefront for a large one."""
+    flat, cam = pt.cornell_box(320, 200)
+    t = flat.triangles
+    parts = [t.copy() for _ in range(4)]
+    mid = (t["v0"] + t["v1"] + t["v2"]) / np.float32(3)
+    flat = pt.FlatScene(np.concatenate(parts), flat.spheres, None, flat.materials, flat.textures, flat.pixels)
+    for k, (a, b) in enumerate((("v0", "v1"), ("v1", "v2"), ("v2", "v0"))):      # three parts around the centroid
+        part = flat.triangles[k * len(t):(k + 1) * len(t)]
+        part["v0"], part["v1"], part["v2"] = t[a], t[b], mid
+    flat = pt.FlatScene(flat.triangles[:3 * len(t)], flat.spheres, None, flat.materials, flat.textures, flat.pixels).build_bvh()
+    for width, height in ((320, 200), (900, 560)):
+        _, cam = pt.cornell_box(width, height)
+        r = pt.CudaRenderer(flat, cam, width, height, 3, max_depth=6)
+        r.add_samples(2)
+        want = r.sums().tobytes()
+        r.set_tail_paths(500)
+        r.reset(cam)
+        r.add_samples(2)
+        assert r.sums().tobytes() == want
