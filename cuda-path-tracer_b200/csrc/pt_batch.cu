@@ -189,7 +189,7 @@ __global__ void batch_shade(DeviceScene scene, BatchBuffers b, int parity) {
             DeviceScene js = job_scene(scene, j);
             Pcg rng = b.rng[g];
             ShadowRay sr;
-            live = shade_path(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), slot, s, h, make_uint2(0, 0),
+            live = shade_path<false>(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), slot, s, h, make_uint2(0, 0),
                               rng, sr, shadow);
             b.rng[g] = rng;
             if (shadow) b.shadows[slot] = sr;
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(256, 2) batch_finish_pair(DeviceScene scene, B
                 PathHit h;
                 h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = (hit && !error) ? hi.slot : (error ? -2 : -1);
                 bool shadow = false;
-                live = shade_path(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), slot, s, h, make_uint2(0, 0),
+                live = shade_path<true>(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), slot, s, h, make_uint2(0, 0),
                                   rng, sr, shadow);
                 pending = shadow;
             }
@@ -409,7 +409,7 @@ struct BatchOps {
         PathState s = b.lane_paths[lane];
         Pcg rng = b.rng[g];
         ShadowRay sr;
-        n.live = shade_path(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), int32_t(lane), s, h, make_uint2(0, 0),
+        n.live = shade_path<true>(js, job_ctx(j, b.mis), b.sums + 3 * g, int32_t(g - j.pixel_offset), int32_t(lane), s, h, make_uint2(0, 0),
                             rng, sr, n.shadow);
         b.rng[g] = rng;
         if (n.live) b.lane_paths[lane] = s;

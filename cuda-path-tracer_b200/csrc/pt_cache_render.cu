@@ -230,6 +230,7 @@ struct ShadeOut {
 };
 
 // One bounce of path i given its closest hit (see the file comment).
+template <bool kWhole>
 __device__ inline void shade(const DeviceScene &scene, const Params &p, const Buffers &b, int32_t i, CachePath &s,
                              const PathHit &h, Pcg &rng, ShadeOut &o) {
     f3 R = mk(s.rr, s.rg, s.rb), T = mk(s.tr, s.tg, s.tb), U = mk(s.ur, s.ug, s.ub), S = mk(s.sr, s.sg, s.sb);
@@ -251,7 +252,7 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
         const bool suffix = s.vertices >= 0;
         if (mat.type == PT_LIGHT) {
             float weight = s.prev_pdf > 0 ? mis_weight(s.prev_pdf, hit_light_pdf(scene, mk(s.ox, s.oy, s.oz), rec)) : 1;
-            f3 e = weight * surface_texture(scene, mat.texture_id, rec);
+            f3 e = weight * surface_texture<kWhole>(scene, mat.texture_id, rec);
             R = R + T * e;
             if (suffix) S = S + U * e;
             o.finished = true;
@@ -263,7 +264,7 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
             // glass ones (roughness = fuzz, 0 for glass; albedo 1 for glass).
             const bool cacheable = diffuse || (p.query_specular && (mat.type == PT_METAL || mat.type == PT_GLASS));
             const f3 albedo = mat.type == PT_GLASS ? mk(1, 1, 1)
-                            : mat.type == PT_METAL ? mk(mat.albedo) : surface_texture(scene, mat.texture_id, rec);
+                            : mat.type == PT_METAL ? mk(mat.albedo) : surface_texture<kWhole>(scene, mat.texture_id, rec);
             bool stop = false;
             if (cacheable && p.use_cache) {
                 const bool at_query = !suffix && s.depth >= 1 && s.spread * s.spread > p.spread_c * s.a0;
@@ -308,7 +309,7 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
                         float cosl = fmaxf(0, dot(normal, direction));
                         float pdf = light_direction_pdf(scene.light_area, pos, light.point, light.normal);
                         if (cosl > 0 && pdf > 0) {
-                            f3 emission = light_emission(scene, light);
+                            f3 emission = light_emission<kWhole>(scene, light);
                             float bsdf_pdf = cosl / float(M_PI);
                             f3 local = albedo * emission * (bsdf_pdf * mis_weight(pdf, bsdf_pdf) / pdf);
                             f3 c = T * local, cs = U * local;
@@ -333,7 +334,7 @@ __device__ inline void shade(const DeviceScene &scene, const Params &p, const Bu
                 s.prev_pdf = 0;
                 s.bounce_pdf = 0;                   // a delta lobe adds no spread
                 f3 attenuation, dir;
-                if (!trace_scatter(scene, mat, d, rec, rng, attenuation, dir)) o.finished = true;
+                if (!trace_scatter<kWhole>(scene, mat, d, rec, rng, attenuation, dir)) o.finished = true;
                 else {
                     T = T * attenuation;
                     U = U * attenuation;
@@ -400,7 +401,7 @@ __global__ void shade_kernel(DeviceScene scene, Params p, Buffers b, int parity)
             s = b.paths[i];
             PathHit h = b.hits[i];
             rng = b.rng[i];
-            shade(scene, p, b, i, s, h, rng, o);
+            shade<false>(scene, p, b, i, s, h, rng, o);
             if (o.shadow) b.shadows[i] = o.sr;
         }
         const int32_t q = append(o.query, &b.counters[3]);
@@ -438,7 +439,7 @@ __global__ void finish_kernel(DeviceScene scene, Params p, Buffers b, int parity
             PathHit h;
             h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = (hit && !error) ? hi.slot : (error ? -2 : -1);
             ShadeOut o;
-            shade(scene, p, b, i, s, h, rng, o);
+            shade<false>(scene, p, b, i, s, h, rng, o);
             if (o.shadow) {
                 rays++;
                 const CacheShadow &sr = o.sr;
@@ -533,7 +534,7 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
                 PathHit h;
                 h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = (hit && !error) ? hi.slot : (error ? -2 : -1);
                 ShadeOut o;
-                shade(scene, p, b, i, s, h, rng, o);
+                shade<true>(scene, p, b, i, s, h, rng, o);
                 if (o.shadow) { sr = o.sr; pending = true; }
                 if (o.finished) {
                     const int32_t qi = o.query ? atomicAdd(&b.counters[3], 1) : -1;
@@ -603,7 +604,7 @@ struct FrameOps {
         CachePath s = b.lane_paths[lane];
         Pcg rng = b.rng[i];
         ShadeOut o;
-        nrc::shade(scene, p, b, i, s, h, rng, o);
+        nrc::shade<true>(scene, p, b, i, s, h, rng, o);
         if (o.finished) {
             const int32_t q = o.query ? atomicAdd(&b.counters[3], 1) : -1;
             retire(p, b, i, s, rng, o, q);                   // one sample left: starts no other

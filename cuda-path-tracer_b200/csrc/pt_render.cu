@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256, 4) shade_kernel(DeviceScene scene, Render
             uint2 st = (p.debug == PT_DEBUG_BVH || p.debug == PT_DEBUG_INTERSECTIONS) ? b.stats[i] : make_uint2(0, 0);
             Pcg rng = b.rng[i];
             ShadowRay sr;
-            live = shade_path(scene, shade_ctx(p), b.sums + 3 * size_t(i), i, i, s, h, st, rng, sr, shadow);
+            live = shade_path<false>(scene, shade_ctx(p), b.sums + 3 * size_t(i), i, i, s, h, st, rng, sr, shadow);
             b.paths[i] = s;
             b.rng[i] = rng;
             if (shadow) b.shadows[i] = sr;
@@ -207,7 +207,7 @@ __global__ void finish_kernel(DeviceScene scene, RenderParams p, RenderBuffers b
             h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = (hit && !error) ? hi.slot : (error ? -2 : -1);
             ShadowRay sr;
             bool shadow = false;
-            bool live = shade_path(scene, shade_ctx(p), b.sums + 3 * size_t(i), i, i, s, h, make_uint2(boxes, prims), rng, sr, shadow);
+            bool live = shade_path<false>(scene, shade_ctx(p), b.sums + 3 * size_t(i), i, i, s, h, make_uint2(boxes, prims), rng, sr, shadow);
             if (shadow) {
                 rays++;
                 pt_ray q;
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(256, 2) finish_pair_kernel(DeviceScene scene, 
                 PathHit h;
                 h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = (hit && !error) ? hi.slot : (error ? -2 : -1);
                 bool shadow = false;
-                live = shade_path(scene, shade_ctx(p), b.sums + 3 * size_t(i), i, i, s, h, make_uint2(boxes, prims), rng, sr, shadow);
+                live = shade_path<true>(scene, shade_ctx(p), b.sums + 3 * size_t(i), i, i, s, h, make_uint2(boxes, prims), rng, sr, shadow);
                 pending = shadow;
             }
         }
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kSmallBlock) render_small_kernel(DeviceScene s
         if (live) {
             PathHit h;
             h.t = hi.t; h.u = hi.u; h.v = hi.v; h.slot = hit ? hi.slot : -1;
-            live = shade_path(scene, ctx, b.sums + 3 * size_t(i), i, i, s, h, make_uint2(0, 0), rng, sr, pending);
+            live = shade_path<true>(scene, ctx, b.sums + 3 * size_t(i), i, i, s, h, make_uint2(0, 0), rng, sr, pending);
         }
         __syncwarp();
     }
@@ -438,7 +438,7 @@ struct RenderOps {
         PathState s = b.lane_paths[lane];
         Pcg rng = b.rng[i];
         ShadowRay sr;
-        n.live = shade_path(scene, ctx, b.sums + 3 * size_t(i), i, i, s, h, make_uint2(0, 0), rng, sr, n.shadow);
+        n.live = shade_path<true>(scene, ctx, b.sums + 3 * size_t(i), i, i, s, h, make_uint2(0, 0), rng, sr, n.shadow);
         b.rng[i] = rng;
         if (n.live) b.lane_paths[lane] = s;
         if (n.shadow) b.lane_shadows[lane] = sr;

@@ -97,9 +97,12 @@ __device__ inline void surface_hit(const DeviceScene &s, const pt_ray &r, const 
     }
 }
 
-// Texture coordinates of a hit, and the texture there (out of line: textures other than constant
-// colours are the rarer case, and the code is long).
-static __device__ __noinline__ f3 surface_texel(const DeviceScene &s, int32_t id, int32_t slot, float u, float v, f3 normal) {
+// Texture coordinates of a hit, and the texture there.  Rarer code like this (textures other than constant colours, glass, the
+// debug views) is long: kernels that carry paths through all their bounces keep it out of line (kWhole), the others
+// inline, since a kernel that calls anything keeps registers for it (shade_kernel with the calls and without: a
+// room of 1,280 triangles at 960x600, 16 spp, 36.1 and 34.2 ms; 64 triangles at 1920x1080 7.11 and 6.69; the Cornell box
+// in render_small_kernel, 960x600, 11.5 and 11.9).
+static __device__ __forceinline__ f3 surface_texel_inline(const DeviceScene &s, int32_t id, int32_t slot, float u, float v, f3 normal) {
     if (slot < s.tri_slots) {
         const pt_triangle &face = s.triangles[s.tris[slot].id];
         f3 uv = (1 - u - v) * mk(face.uv0) + u * mk(face.uv1) + v * mk(face.uv2);
@@ -109,10 +112,14 @@ static __device__ __noinline__ f3 surface_texel(const DeviceScene &s, int32_t id
     }
     return trace_texture(s, id, u, v);
 }
-__device__ inline f3 surface_texture(const DeviceScene &s, int32_t id, const Surface &o) {
+static __device__ __noinline__ f3 surface_texel(const DeviceScene &s, int32_t id, int32_t slot, float u, float v, f3 normal) {
+    return surface_texel_inline(s, id, slot, u, v, normal);
+}
+template <bool kWhole> __device__ inline f3 surface_texture(const DeviceScene &s, int32_t id, const Surface &o) {
     const pt_texture &tex = s.textures[id];
     if (tex.type == PT_TEX_CONSTANT) return mk(tex.color);
-    return surface_texel(s, id, o.slot, o.u, o.v, o.normal);
+    if constexpr (kWhole) return surface_texel(s, id, o.slot, o.u, o.v, o.normal);
+    else return surface_texel_inline(s, id, o.slot, o.u, o.v, o.normal);
 }
 
 // A sampled emitter point; `u`, `v` are the two uniform draws it came from.
@@ -148,7 +155,7 @@ __device__ inline LightSample sample_light(const DeviceScene &scene, Pcg &random
 }
 
 // The emitter's texture at the sampled point.
-static __device__ __noinline__ f3 light_texel(const DeviceScene &s, int32_t id, int32_t index, float u, float v, f3 normal) {
+static __device__ __forceinline__ f3 light_texel_inline(const DeviceScene &s, int32_t id, int32_t index, float u, float v, f3 normal) {
     const pt_light &light = s.lights[index];
     if (light.type == PT_TRIANGLE) {
         const pt_triangle &t = s.triangles[light.primitive];
@@ -160,11 +167,15 @@ static __device__ __noinline__ f3 light_texel(const DeviceScene &s, int32_t id, 
     }
     return trace_texture(s, id, u, v);
 }
-__device__ inline f3 light_emission(const DeviceScene &s, const LightSample &l) {
+static __device__ __noinline__ f3 light_texel(const DeviceScene &s, int32_t id, int32_t index, float u, float v, f3 normal) {
+    return light_texel_inline(s, id, index, u, v, normal);
+}
+template <bool kWhole> __device__ inline f3 light_emission(const DeviceScene &s, const LightSample &l) {
     const int32_t id = s.materials[l.material].texture_id;
     const pt_texture &tex = s.textures[id];
     if (tex.type == PT_TEX_CONSTANT) return mk(tex.color);
-    return light_texel(s, id, l.index, l.u, l.v, l.normal);
+    if constexpr (kWhole) return light_texel(s, id, l.index, l.u, l.v, l.normal);
+    else return light_texel_inline(s, id, l.index, l.u, l.v, l.normal);
 }
 
 // light_direction_pdf (light_sampling.h:56-65)
@@ -189,18 +200,22 @@ __device__ inline float hit_light_pdf(const DeviceScene &scene, f3 from, const S
     return light_direction_pdf(scene.light_area, from, hit.p, normal);
 }
 
-// Schlick's pow(1 - cosine, 5) in double, as the reference's C++ promotes it; out of line, since the
-// code is long and only glass needs it
-static __device__ __noinline__ double schlick_pow(float cosine) { return pow(1 - cosine, 5); }
+// Schlick's pow(1 - cosine, 5) in double, as the reference's C++ promotes it
+static __device__ __noinline__ double schlick_pow_call(float cosine) { return pow(1 - cosine, 5); }
+template <bool kWhole> __device__ inline double schlick_pow(float cosine) {
+    if constexpr (kWhole) return schlick_pow_call(cosine);
+    else return pow(1 - cosine, 5);
+}
 
 // trace_scatter (transport.h:115-155)
+template <bool kWhole>
 __device__ inline bool trace_scatter(const DeviceScene &scene, const pt_material &mat, f3 in_dir,
                                      const Surface &rec, Pcg &random, f3 &attenuation, f3 &out_dir) {
     f3 p = rec.p, n = rec.normal;
     if (mat.type == PT_DIFFUSE) {
         f3 target = p + n + sample_ball(random);
         out_dir = target - p;
-        attenuation = surface_texture(scene, mat.texture_id, rec);
+        attenuation = surface_texture<kWhole>(scene, mat.texture_id, rec);
         return true;
     }
     if (mat.type == PT_METAL) {
@@ -229,7 +244,7 @@ __device__ inline bool trace_scatter(const DeviceScene &scene, const pt_material
             refracted = ratio * (uv - outward * dt) - outward * sqrt(discriminant);
             float r0 = (1 - mat.ref_idx) / (1 + mat.ref_idx);
             r0 *= r0;
-            probability = r0 + (1 - r0) * schlick_pow(cosine);
+            probability = r0 + (1 - r0) * schlick_pow<kWhole>(cosine);
         }
         if (random.uniform() < probability) out_dir = reflected;
         else out_dir = refracted;

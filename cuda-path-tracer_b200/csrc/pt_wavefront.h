@@ -70,13 +70,16 @@ __device__ inline pt_ray path_ray(const PathState &s) {
     return r;
 }
 
-// The normals, triangle-id and material-id views' colour of a hit (out of line, off the shaded path).
-static __device__ __noinline__ f3 debug_color(const DeviceScene &scene, int debug, const pt_ray &r, const HitInfo &hi) {
+// The normals, triangle-id and material-id views' colour of a hit.
+static __device__ __forceinline__ f3 debug_color_inline(const DeviceScene &scene, int debug, const pt_ray &r, const HitInfo &hi) {
     pt_flat_hit rec;
     finalize_hit(scene, r, hi, rec);
     if (debug == PT_DEBUG_NORMALS) return 0.5f * (mk(rec.normal) + mk(1, 1, 1));
     if (debug == PT_DEBUG_TRIANGLE) return rec.primitive_type == PT_TRIANGLE ? id_color(rec.primitive_id) : mk(0.3f, 0.3f, 0.3f);
     return id_color(rec.material_id);
+}
+static __device__ __noinline__ f3 debug_color(const DeviceScene &scene, int debug, const pt_ray &r, const HitInfo &hi) {
+    return debug_color_inline(scene, debug, r, hi);
 }
 
 // The rest of one trace_color iteration for the path in `slot`, rendering `pixel` (its index
@@ -84,6 +87,7 @@ static __device__ __noinline__ f3 debug_color(const DeviceScene &scene, int debu
 // hit: emission with its MIS weight, next-event estimation (which may emit a shadow ray),
 // cosine or material scatter; when the sample ends, its radiance is added to the pixel sum and
 // the pixel's next camera ray starts.  Returns whether the path is still live.
+template <bool kWhole>
 __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, float *sum, int32_t pixel, int32_t slot,
                                   PathState &s, const PathHit &h, const uint2 &stats, Pcg &rng, ShadowRay &sr, bool &shadow) {
     shadow = false;
@@ -101,7 +105,8 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
         pt_ray r = path_ray(s);
         HitInfo hi; hi.t = h.t; hi.u = h.u; hi.v = h.v; hi.slot = h.slot;
         if (p.debug != PT_DEBUG_SHADED) {
-            radiance = debug_color(scene, p.debug, r, hi);
+            if constexpr (kWhole) radiance = debug_color(scene, p.debug, r, hi);
+            else radiance = debug_color_inline(scene, p.debug, r, hi);
             finished = true;
         } else {
             Surface rec;
@@ -111,12 +116,12 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
             f3 pos = rec.p, normal = rec.normal;
             if (mat.type == PT_LIGHT) {
                 float weight = s.prev_pdf > 0 ? mis_weight(s.prev_pdf, hit_light_pdf(scene, mk(s.ox, s.oy, s.oz), rec)) : 1;
-                radiance = radiance + weight * throughput * surface_texture(scene, mat.texture_id, rec);
+                radiance = radiance + weight * throughput * surface_texture<kWhole>(scene, mat.texture_id, rec);
                 finished = true;
             } else if (s.depth == p.max_depth) {
                 finished = true;
             } else if (p.mis && mat.type == PT_DIFFUSE) {
-                f3 attenuation = surface_texture(scene, mat.texture_id, rec);
+                f3 attenuation = surface_texture<kWhole>(scene, mat.texture_id, rec);
                 if (scene.light_count) {
                     LightSample light = sample_light(scene, rng);
                     f3 delta = light.point - pos;
@@ -126,7 +131,7 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
                         float cosine = fmaxf(0, dot(normal, direction));
                         float pdf = light_direction_pdf(scene.light_area, pos, light.point, light.normal);
                         if (cosine > 0 && pdf > 0) {
-                            f3 emission = light_emission(scene, light);
+                            f3 emission = light_emission<kWhole>(scene, light);
                             float bsdf_pdf = cosine / float(M_PI);
                             f3 c = throughput * attenuation * emission * (bsdf_pdf * mis_weight(pdf, bsdf_pdf) / pdf);
                             sr.ox = pos.x; sr.oy = pos.y; sr.oz = pos.z; sr.tmax = distance - 0.001f;
@@ -145,7 +150,7 @@ __device__ inline bool shade_path(const DeviceScene &scene, const ShadeCtx &p, f
             } else {
                 s.prev_pdf = 0;
                 f3 attenuation, dir;
-                if (!trace_scatter(scene, mat, in_dir, rec, rng, attenuation, dir)) finished = true;
+                if (!trace_scatter<kWhole>(scene, mat, in_dir, rec, rng, attenuation, dir)) finished = true;
                 else {
                     throughput = throughput * attenuation;
                     s.ox = pos.x; s.oy = pos.y; s.oz = pos.z;
