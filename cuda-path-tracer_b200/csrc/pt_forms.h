@@ -62,13 +62,14 @@ inline bool batch_in_one(double open_pixels, double going_on_pixels, double most
            (going_on_pixels <= 0 || going_on <= (most_going_on > 1 ? most_going_on : 1) + open / 3);
 }
 
-// The cached renderer's paths end at their first query (without its cache it is the plain renderer), so rooms gain for longer (1080p is 22 pixels per lane; samples x
-// limit 48; wavefront over kernel): 1,280 triangles 0.98 at 6.1, 0.70 at 22; 20,480 1.36, 0.84; 327,680 2.25, 1.33.
+// The cached renderer's paths end at their first query (without its cache it is the plain renderer), so rooms gain for
+// longer (pixels per lane, samples x limit 48; wavefront over kernel): 1,280 triangles 0.98 at 6.1, 0.70 at 22; 20,480 1.36, 0.84; 327,680 2.25, 1.33.
 // Open views: 20 pixels per lane, 28 when the bounces of a frame are many (65,000 triangles at 15 and 22: 1.27 and
 // 1.10; 1M 1.33 and 1.15; of one sample 1.13 and 1.04 at 15, none measured above); half of that past the L2 (2.6M, one
 // sample 1.03 at 6.1 and 0.90 at 15, four 1.11 at 9.7 and 0.94 at 15).
 inline double most_pixels_cached(bool go_on, size_t primitives, size_t walked_bytes, int64_t bounces) {
-    const double most = (bounces >= 24 ? 28 : 20) / (walked_bytes <= (size_t(100) << 20) ? 1.0 : 2.0), room = 1.1 * std::pow(double(primitives), 0.25);
+    const double most = (bounces >= 24 ? 28 : 20) / (walked_bytes <= (size_t(100) << 20) ? 1.0 : 2.0);
+    const double room = 1.1 * std::pow(double(primitives), 0.25);
     return go_on && room < most ? room : most;
 }
 

@@ -38,7 +38,7 @@ constexpr int kOutMatBytes = kOutPad * kWidth * 2;         // 2 KB
 constexpr int kWeightBytes = kHidden * kMatBytes + kOutMatBytes;   // 43008
 constexpr int kActBytes = kTile * kWidth * 2;              // 16 KB per 128 x 64 tile
 constexpr int kOutActBytes = kTile * kOutPad * 2;          // 4 KB per 128 x 16 tile
-constexpr int kPad = 2048;                                 // guard after every operand buffer
+constexpr int kPad = 2048;                                 // after train_kernel's last operand: mma_tn reads past its end
 constexpr int kMasterFloats = kHidden * kWidth * kWidth + kWidth * kOut;   // 20672
 constexpr long long kSpinLimit = 1ll << 22;   // mbarrier try_wait attempts before a wait gives up
 
@@ -226,7 +226,6 @@ __device__ inline void tmem_free(uint32_t base, uint32_t cols) {
     if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(base), "r"(cols) : "memory");
 }
 
-// Copies the canonical BF16 weights (global) into shared memory.
 // X (128 x 64, rows = queries) into the core-matrix layout; rows past `count` are zero.
 // `r` is the calling thread's row of the tile; kPart as encode's.
 template <int kPart = 0>

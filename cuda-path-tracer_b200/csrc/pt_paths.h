@@ -17,13 +17,17 @@
 // and a heavy pixel runs without a break from the first pass on.
 //
 // What it measured (kernel time, 1M triangles, bounce limit 8, 16 spp; wavefront and pair tail before):
-// 960x600 15.1 -> 9.4 ms, 480x300 8.4 -> 7.0, 1920x1080 30.4 -> 27.0; 65,000 triangles at 960x600 5.4 -> 2.8.
+// 960x600 15.1 -> 9.5 ms, 1920x1080 30.4 -> 27.1; 65,000 triangles at 960x600 5.4 -> 2.9.  Where it loses, inside rooms
+// and on large images, pt_forms.h says.
 // Lanes that shade together cost one pass through 60 KB of shading code whether 8 or 28 of them do, so
-// a warp waits until fewer than kPathsActive still walk (the 960x600 call: 24 13.0 ms, 16 12.3, 8 11.35, 5
-// 10.9, 2 11.5).  Five blocks of 128 per SM, since records became the lanes' own and stay in L1: with four
-// 1920x1080 takes 29.2 ms (480x300 6.8), with six 960x600 10 % more.  Shading 32 at a time from rings of 64
-// paths per warp filled the lanes better (8.2 ms until the items ran out, records in the pixels' slots) but
-// doubled the time a heavy pixel waits for each bounce (12.6 ms in all).
+// a warp waits until fewer than kPathsActive still walk (time with 2, 5, 8 and 16 over that with 4: 1M triangles
+// 960x600 1.01, 1.00, 1.04, 1.12, 1920x1080 1.07, 0.99, 0.99, 1.05; 65,000 at 960x600 0.95, 1.04, 1.09, 1.12; six-job
+// batch 0.98, 1.01, 1.04, 1.06).  Five blocks of 128 per SM, since records became the lanes' own and stay in L1, although
+// 96 registers then spill (bytes stored and loaded per thread: render_paths_kernel 56 and 52, batch_paths 100 and 92,
+// frame_kernel 190 and 196): with four, which spill 48 in frame_kernel alone, 1920x1080 takes 10 % longer, the batch 5,
+// 960x600 2, and 640x400 13 % less; with six 960x600 takes 7 % longer, 640x400 17, the batch 8.  Shading 32 at a time
+// from rings of 64 paths per warp filled the lanes better (8.2 ms until the items ran out, records in the pixels' slots)
+// but doubled the time a heavy pixel waits for each bounce (12.6 ms in all).
 #pragma once
 
 #include "pt_forms.h"
@@ -57,7 +61,7 @@ __device__ inline uint32_t probe_path(const DeviceScene &scene, const pt_camera 
     return met;
 }
 
-constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 5;   // 96 registers
+constexpr int kPathsBlock = 128, kPathsBlocksPerSm = 5;   // 96 registers, with spills (see above)
 constexpr int kPathsActive = 4;   // lanes of a warp still walking below which the others shade
 
 // The lane's next ray: path and shadow records begin with origin and (shadow) tmax, then the direction.

@@ -579,7 +579,9 @@ pt_status pt_query_rays_brute_device(const pt_scene *scene, const pt_ray *rays, 
 // Host buffers, at least one of them pageable: worker threads take chunks of rays, each moving its
 // chunk through pinned memory, the walk and back on a stream of its own (pt_stage.h), so the copies
 // between the caller's memory and the pinned chunks, which are most of the time, run side by side.
-// 1.5M rays of the 1M-triangle scene with a freshly allocated answer: 5.9 -> 3.5 ms, 4M rays 25 -> 6.
+// 1.5M rays of the 1M-triangle scene with a freshly allocated answer: 5.9 -> 3.5 ms, 4M rays 25 -> 6.  A chunk is too
+// short to be ordered (kOrderMin): past the L2 that shows behind the copies only in part (8.4M rays on 2.6M triangles
+// into memory used before 39.9 -> 13.9 ms; on 1M, which nothing orders, 33.9 -> 10.3).
 static_assert(kStageWorkers == sizeof(pt_scene::workers) / sizeof(pt_scene::workers[0]), "a workspace per worker");
 // Rays from which the threads are worth starting (1M rays 3.5 ms in one thread, 2.6 in eight; 400,000 1.45
 // and 1.45; 100,000 0.5 and 0.75).

@@ -93,8 +93,9 @@ PT_HD __forceinline__ bool accept_hit(const DeviceScene &s, int32_t slot, float 
 // is the float above the closest distance (an accepted t is below tmax, so nextafterf(t, tmax) is
 // next_up(t)).  The limit changes only here, so it is kept instead of being recomputed before each
 // test, and the tie key is formed only when two distances are equal (2^25 rays on the 1M-triangle
-// scene: 7.00 -> 6.39 ms; 2^22 incoherent ones: 2.02 -> 1.85).  Returns true when a hit was accepted.  `any` selects any-hit (the first hit is the answer) or closest-hit (ties by key) at run
-// time; the template below fixes it at compile time.
+// scene: 7.00 -> 6.39 ms; 2^22 incoherent ones: 2.02 -> 1.85).  Returns true when a hit was accepted.
+// `any` selects any-hit (the first hit is the answer) or closest-hit (ties by key) at run time; the
+// template below fixes it at compile time.
 PT_HD __forceinline__ bool test_leaf_rt(const DeviceScene &s, int32_t slot, const pt_ray &r, float dl, float tmin,
                                         float &limit, int tie, bool any, HitInfo &hit, uint32_t &prims) {
     float t, u = 0, v = 0;
