@@ -569,7 +569,8 @@ struct pt_renderer {
     bool fused = false;                 // four-wide tree and shaded view: the form goes by the image's size (whole, tail_alone)
     bool small = false;                 // the scene fits render_small_kernel and the view is shaded
     bool tiny = false;                  // a tree of a few nodes
-    bool goes_on = false, looking = false;   // paths of the view looked at last (pt_forms.h); a look is under way
+    bool goes_on = false;               // paths of the view looked at last (pt_forms.h)
+    bool moved = false, looking = false;   // a reset brought another view; a look at it is under way
     DeviceBuffer paths, hits, stats, shadows, queue0, queue1, shadow_queue, counters, fetch, ray_total, error, sums, rng, rgba, lanes, met;
     RenderBuffers buf{};
     cudaStream_t stream = nullptr;
@@ -579,6 +580,7 @@ struct pt_renderer {
     int32_t *host_counters = nullptr;   // pinned, one slot per in-flight iteration and one for the probe of the view
     Event iteration_events[8], looked;
     ~pt_renderer() {
+        if (looking) cudaEventSynchronize(looked.get());
         if (host_counters) cudaFreeHost(host_counters);
         if (shadow_stream) cudaStreamDestroy(shadow_stream);
         if (stream) cudaStreamDestroy(stream);
@@ -628,7 +630,7 @@ struct pt_renderer {
         return double(pixels) <= most_pixels(goes_on, scene->triangle_count + scene->sphere_count, scene->walked_bytes(),
                                              int64_t(count) * params.max_depth) * double(lane_count());
     }
-    // Looks at a view beside whatever comes next; seen() takes the answer once it is there, or waits for it.
+    // Looks at a view, beside the call that follows; seen() takes the answer once it is there, or waits for it.
     void look(const pt_camera &camera) {
         if (!sized()) return;
         met.reserve(sizeof(uint32_t));
@@ -749,7 +751,7 @@ pt_status pt_reset(pt_renderer *r, const pt_camera *camera) {
         init_pixels<<<(r->pixels + 255) / 256, 256, 0, r->stream>>>(r->buf.sums, r->buf.rng, r->pixels, r->seed);
         PT_CUDA(cudaGetLastError());
         PT_CUDA(cudaStreamSynchronize(r->stream));
-        if (std::memcmp(camera, &r->params.camera, sizeof *camera)) r->look(*camera);
+        if (std::memcmp(camera, &r->params.camera, sizeof *camera)) r->moved = true;
         r->params.camera = *camera;
         r->samples = 0; r->milliseconds = 0; r->rays = 0;
     });
@@ -762,7 +764,10 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         if (count <= 0 || count > INT32_MAX - r->samples) throw Error(PT_INVALID_ARGUMENT, "invalid accumulated sample count");
         const DeviceScene &scene = r->scene->view;
         cudaStream_t st = r->stream;
-        r->seen(count >= 4);   // after a reset to another view; a short call takes the form of the view before
+        // after a reset to another view a short call takes the form of the view before, and looks at its own beside itself
+        // (0.05 ms in a room of 1,280 triangles, 0.2 on 1M)
+        if (r->moved) { r->look(r->params.camera); r->moved = false; }
+        r->seen(count >= 4);
         const bool whole = !r->small && r->whole(count), tail_alone = !r->small && !whole && r->tail_alone();
         if (whole) r->lane_buffers();
         else if (tail_alone) r->path_buffers();
@@ -840,6 +845,7 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         }
         PT_CUDA(cudaEventRecord(r->stop.get(), st));
         PT_CUDA(cudaEventSynchronize(r->stop.get()));
+        r->seen(true);
         int32_t error = 0;
         unsigned long long total = 0;
         PT_CUDA(cudaMemcpy(&error, r->buf.error, sizeof error, cudaMemcpyDeviceToHost));

@@ -250,8 +250,8 @@ pt_status pt_set_block_shape(pt_renderer *renderer, int width, int height);
  * next ray while the other walks its last shadow ray; default max(65536, pixels/4); 0 keeps the
  * wavefront to the end).  Until this is called, shaded renders of scenes of at most 32 primitives, and
  * images of two to at most forty pixels per resident GPU thread (fewer the larger the scene and the fewer the samples
- * of a call, and hardly any inside a room, where paths go on: the view is looked at when the renderer is created or
- * reset to another camera) run as one kernel from the first camera ray to the last bounce, and smaller images in the
+ * of a call, and hardly any inside a room, where paths go on: the view is looked at when the renderer is created and
+ * by the first call after a reset to another camera) run as one kernel from the first camera ray to the last bounce, and smaller images in the
  * two-threads-per-path kernel alone; calling it asks for the wavefront.  Results do not depend on it. */
 pt_status pt_renderer_tuning(pt_renderer *renderer, int32_t tail_paths);
 /* Linear FP32 radiance sums (3 floats per pixel, row 0 at the bottom, not divided by spp). */
