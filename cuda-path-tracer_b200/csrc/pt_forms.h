@@ -48,6 +48,15 @@ inline double most_pixels_open(size_t walked_bytes, int64_t bounces) {
     return bounces < 8 ? 12 : bounces < 32 ? 25 : bounces < 128 ? 32 : 40;
 }
 
+// Up to how many pixels per lane an image runs in the tail kernel alone, whose two lanes per path walk extension and
+// shadow rays side by side.  Where walks are short a call of several samples gains by it for longer (tail kernel alone
+// over the kernel of pt_paths.h, 4 and 16 spp at 2.0, 2.7 and 4.1 pixels per lane: 400 triangles 0.81 0.69, 0.88 0.72, 1.08
+// 0.83; 10,000 0.88 0.84, 0.97 0.86, 1.03 1.02; 65,000 0.89 0.86, 0.89 0.89, 1.16 1.19; 200,000 0.97 0.94, 1.07 1.00, 1.26
+// 1.20; 1M 1.15 1.11, 1.35 1.37, 1.56 1.71; of one sample 1.02 to 1.27 at 2.0 on all but 200,000 triangles).
+inline double most_pixels_alone(bool go_on, size_t walked_bytes, int64_t samples) {
+    return !go_on && walked_bytes <= (size_t(8) << 20) && samples >= 4 ? 3 : 2;
+}
+
 // Most pixels per lane of an image.
 inline double most_pixels(bool go_on, size_t primitives, size_t walked_bytes, int64_t bounces) {
     return go_on ? most_pixels_going_on(primitives) : most_pixels_open(walked_bytes, bounces);

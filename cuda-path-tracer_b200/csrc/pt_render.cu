@@ -616,17 +616,17 @@ struct pt_renderer {
         buf.queue[1] = queue1.get<int32_t>(); buf.shadow_queue = shadow_queue.get<int32_t>();
     }
     // Which kernels render an image of a four-wide scene in the shaded view, unless pt_renderer_tuning asked
-    // for the wavefront.  Up to two pixels per lane of render_paths_kernel: the tail kernel alone, whose two
-    // lanes per path walk extension and shadow rays side by side.  Above, render_paths_kernel up to the sizes of
-    // pt_forms.h, from there on the wavefront: its queues are long enough to hide their slowest rays and its walk
-    // kernels hold more warps.  Milliseconds a call (tail kernel alone, render_paths_kernel, wavefront with tail; 1M
-    // triangles, 12 spp, bounce limit 8): 64,000 pixels 3.4, -, 5.0; 99,000 4.1, 5.3, -; 144,000 5.1, 5.5, 6.6;
-    // 187,000 6.4, 5.9, -; 256,000 7.3, 5.2, -; on 10,000 triangles 64,000 pixels 0.64, -, 1.2; 144,000 1.1, 1.4, -;
-    // 187,000 1.3, 1.65, -; 256,000 1.4, 1.7, 2.7.
+    // for the wavefront.  Small images: the tail kernel alone (12 spp, bounce limit 8, ms, with a wavefront before it and
+    // without: 64,000 pixels of 1M triangles 5.0 and 3.4, of 10,000 1.2 and 0.64).  Above, render_paths_kernel up to
+    // the sizes of pt_forms.h, from there on the wavefront: its queues are long enough to hide their slowest rays and
+    // its walk kernels hold more warps.
     int64_t lane_count() const { return int64_t(grid_paths) * kPathsBlock; }
     bool sized() const { return fused && pixels > 2 * lane_count() && pixels <= 40 * lane_count(); }   // for render_paths_kernel
+    bool alone(int count) const {
+        return fused && double(pixels) <= most_pixels_alone(goes_on, scene->walked_bytes(), count) * double(lane_count());
+    }
     bool whole(int count) const {
-        if (!sized()) return false;
+        if (!sized() || alone(count)) return false;
         return double(pixels) <= most_pixels(goes_on, scene->triangle_count + scene->sphere_count, scene->walked_bytes(),
                                              int64_t(count) * params.max_depth) * double(lane_count());
     }
@@ -648,7 +648,7 @@ struct pt_renderer {
     void narrow() { params.wide = 0; pair_tail = false; fused = false; }
     // An image below the tail's length has no wavefront to run first either (1.2 and 0.6 ms for 52,000 pixels of 12
     // samples on 10,000 triangles).
-    bool tail_alone() const { return (pair_kernel() && pixels < tail_paths) || (fused && pixels <= 2 * lane_count()); }
+    bool tail_alone(int count) const { return (pair_kernel() && pixels < tail_paths) || alone(count); }
     bool pair_kernel() const { return pair_tail && !params.brute && params.debug != PT_DEBUG_BVH && params.debug != PT_DEBUG_INTERSECTIONS; }
     void grids() {
         grid_extend = occupancy_grid((const void *)extend_kernel, block, stack_bytes(block));
@@ -730,7 +730,7 @@ pt_status pt_renderer_create(const pt_scene *scene, const pt_camera *camera, int
             if (r->tiny && (r->small || !r->fused)) r->narrow();
             if (!r->small) {                             // what the first call will most likely use
                 if (r->whole(kManySamples)) r->lane_buffers();
-                else if (r->tail_alone()) r->path_buffers();
+                else if (r->tail_alone(kManySamples)) r->path_buffers();
                 else r->wavefront_buffers();
             }
         } catch (...) { delete r; throw; }
@@ -768,7 +768,7 @@ pt_status pt_add_samples(pt_renderer *r, int count) {
         // (0.05 ms in a room of 1,280 triangles, 0.2 on 1M)
         if (r->moved) { r->look(r->params.camera); r->moved = false; }
         r->seen(count >= 4);
-        const bool whole = !r->small && r->whole(count), tail_alone = !r->small && !whole && r->tail_alone();
+        const bool whole = !r->small && r->whole(count), tail_alone = !r->small && !whole && r->tail_alone(count);
         if (whole) r->lane_buffers();
         else if (tail_alone) r->path_buffers();
         else if (!r->small) r->wavefront_buffers();

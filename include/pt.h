@@ -249,7 +249,7 @@ pt_status pt_set_block_shape(pt_renderer *renderer, int width, int height);
  * completion in one fused kernel (two threads per path on four-wide trees: one walks the path's
  * next ray while the other walks its last shadow ray; default max(65536, pixels/4); 0 keeps the
  * wavefront to the end).  Until this is called, shaded renders of scenes of at most 32 primitives, and
- * images of two to at most forty pixels per resident GPU thread (fewer the larger the scene and the fewer the samples
+ * images of two or three to at most forty pixels per resident GPU thread (fewer the larger the scene and the fewer the samples
  * of a call, and hardly any inside a room, where paths go on: the view is looked at when the renderer is created and
  * by the first call after a reset to another camera) run as one kernel from the first camera ray to the last bounce, and smaller images in the
  * two-threads-per-path kernel alone; calling it asks for the wavefront.  Results do not depend on it. */

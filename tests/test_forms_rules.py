@@ -20,6 +20,7 @@ int main() {
         if (kind == 'o') printf("%g\n", most_pixels_open(size_t(a), int64_t(b)));
         if (kind == 'c') printf("%g\n", most_pixels_cached(a != 0, size_t(b), size_t(c), int64_t(d)));
         if (kind == 'b') printf("%d\n", int(batch_in_one(a, b, c, size_t(d), 1.0)));
+        if (kind == 'a') printf("%g\n", most_pixels_alone(a != 0, size_t(b), int64_t(c)));
         if (kind == 'p') printf("%d\n", int(paths_go_on(uint32_t(a))));
     }
 }
@@ -72,3 +73,12 @@ def test_batches(rule):
     assert rule("b", 29, 0, 0, light) == 1 and rule("b", 31, 0, 0, light) == 0
     assert rule("b", 21, 0, 0, heavy) == 1 and rule("b", 23, 0, 0, heavy) == 0
     assert rule("b", 5.2, 0, 0, 170e6) == 1 and rule("b", 10.6, 0, 0, 170e6) == 0
+
+
+def test_tail_kernel_alone(rule):
+    light, heavy = 6e6, 14e6
+    assert 2.7 < rule("a", 0, light, 4) < 4.1 and rule("a", 0, light, 1) <= 2
+    assert rule("a", 0, heavy, 16) <= 2.7 and rule("a", 1, light, 16) <= 2.7
+    for size in (0, light, heavy, 1e12):                                                 # the other form takes over above it
+        for samples in (1, 4, 16, 1e6):
+            assert rule("a", 0, size, samples) <= rule("o", size, samples)

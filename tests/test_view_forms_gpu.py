@@ -154,3 +154,20 @@ def test_small_room():
         r.reset(cam)
         r.add_samples(2)
         assert r.sums().tobytes() == want
+
+
+@pytest.mark.parametrize("samples", [3, 4])
+def test_open_view_of_few_pixels_and_samples(samples):
+    """256,000 pixels of an open scene: the tail kernel alone from four samples, one call or split."""
+    flat, cam = spheres(640, 400)
+    r = pt.CudaRenderer(flat, cam, 640, 400, 3, max_depth=6)
+    r.add_samples(samples)
+    want, rays = r.sums().tobytes(), r.rays_traced()
+    r.reset(cam)
+    r.add_samples(1)
+    r.add_samples(samples - 1)
+    assert r.sums().tobytes() == want and r.rays_traced() == rays
+    r.set_tail_paths(500)
+    r.reset(cam)
+    r.add_samples(samples)
+    assert r.sums().tobytes() == want
